@@ -25,10 +25,9 @@
 #include "deform.h"
 
 // Resident blocks of 128 an SM the walks and the shading are compiled for (their register budgets: 64 a thread each).
-// Measured on the city frame: the extend walk 3 % faster than at 6 blocks (72 registers, no spills), 2.6 % faster
-// than at 7 (70, no spills; both of its loops compiled in) and 6 % faster than at 9 (56); the split shadow walk (trace_binary_split) 5 % faster at 8 than at 7 (67 registers), 3 % faster
-// than at 9 and 9 % faster than at 10; the shading, latency-bound, 2.5 % faster at 8 blocks than at 6 (80
-// registers), its spills notwithstanding, and no faster at 10 (48).
+// Measured on the city frame: the walks 1.3 % slower at 7 blocks (70 registers) and 2 % slower at 9 (56, with spills);
+// the shading, latency-bound, 2.5 % faster at 8 blocks than at 6 (80 registers), its spills notwithstanding, and no
+// faster at 10 (48).
 #ifndef TRT_BLOCKS_EXTEND
 #define TRT_BLOCKS_EXTEND 8
 #endif
@@ -37,12 +36,6 @@
 #endif
 #ifndef TRT_BLOCKS_SHADE
 #define TRT_BLOCKS_SHADE 8
-#endif
-// The closest-hit walk's loop (see trace_binary_split): 0 single, 1 split, 2 split past the camera's rays (the
-// default: measured on the city, split everywhere the extend walk is 4.6 % slower, split past depth 0 2 % faster; the
-// camera's coherent rays keep the single loop).
-#ifndef TRT_SPLIT_CLOSEST
-#define TRT_SPLIT_CLOSEST 2
 #endif
 #include "sky.h"
 #include "unet.h"
@@ -233,12 +226,10 @@ __global__ void k_raygen(const Job* __restrict__ jobs, uint32_t n_jobs, PathBufs
     Q.q[0][at] = p;
 }
 
-// SPLIT: the binary walk with its loop split (trace_binary_split), which the shadow walks use.
-template <bool COUNT, bool WIDE, bool SPLIT = false>
+template <bool COUNT, bool WIDE>
 __device__ __forceinline__ Hit walk(const Walk& wk, const Sections& X, V3 o, V3 d, float tmax, uint32_t mode,
                                     WalkCount* wc, bool* guard) {
     if (WIDE) return trace_wide<COUNT>(wk.S, wk.W, X, o, d, tmax, mode, wc, guard);
-    if (SPLIT) return trace_binary_split<COUNT>(wk.S, X, wk.top, wk.n_units, o, d, tmax, mode, wc, guard);
     return trace_binary<COUNT>(wk.S, X, wk.top, wk.n_units, o, d, tmax, mode, wc, guard);
 }
 
@@ -258,9 +249,7 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend(const Job* __
             Sections X(J.P);
             float4 o = B.o[p], d = B.d[p];
             bool guard = false;
-            Hit h = (TRT_SPLIT_CLOSEST == 1 || (TRT_SPLIT_CLOSEST == 2 && depth > 0))
-                        ? walk<COUNT, WIDE, true>(J.wk, X, xyz(o), xyz(d), INF, TRACE_CLOSEST, &wc, &guard)
-                        : walk<COUNT, WIDE, false>(J.wk, X, xyz(o), xyz(d), INF, TRACE_CLOSEST, &wc, &guard);
+            Hit h = walk<COUNT, WIDE>(J.wk, X, xyz(o), xyz(d), INF, TRACE_CLOSEST, &wc, &guard);
             if (guard) guard_trips++;
             Q.hit_a[p] = make_float4(h.t, h.u, h.v, bf(h.tri));
             Q.hit_b[p] = make_uint2(h.inst, h.part);
@@ -300,7 +289,7 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADOW) k_shadow(const Job* __
             Sections X(J.P);
             float4 o = Q.so[i], d = Q.sd[i];
             bool guard = false;
-            Hit h = walk<COUNT, WIDE, true>(J.wk, X, xyz(o), xyz(d), o.w, bu(d.w), &wc, &guard);
+            Hit h = walk<COUNT, WIDE>(J.wk, X, xyz(o), xyz(d), o.w, bu(d.w), &wc, &guard);
             if (guard) guard_trips++;
             if (h.tri == MISS) atomicOr(&B.vis[sp >> 3], 1u << (sp & 7u));
         }
@@ -729,10 +718,8 @@ __global__ void k_trace(Params P, Walk wk, const trt_ray* rays, uint64_t n, trt_
     if (i < n) {
         trt_ray r = rays[i];
         bool guard = false;
-        // (closest-hit rays through the single loop, any-hit rays through the split one: the pass's own walks)
         const V3 o{r.o[0], r.o[1], r.o[2]}, d{r.d[0], r.d[1], r.d[2]};
-        Hit h = r.mode == TRACE_CLOSEST ? walk<COUNT, WIDE>(wk, X, o, d, r.tmax, r.mode, &wc, &guard)
-                                        : walk<COUNT, WIDE, true>(wk, X, o, d, r.tmax, r.mode, &wc, &guard);
+        Hit h = walk<COUNT, WIDE>(wk, X, o, d, r.tmax, r.mode, &wc, &guard);
         hits[i] = trt_hit{h.t, h.tri, h.u, h.v, h.inst, h.part};
     }
     if (COUNT) {

@@ -1,20 +1,12 @@
 // Software traversal over the reference's own two-level binary trees (renderer/shaders/trace_units.wgsl:44-135):
 // the top tree over the units' world boxes, each unit's mesh tree in its model space, one loop over both levels.
-// It is the pass's walk (faster on B200 than the wide-BVH walk of wide_bvh.cuh, which TRT_RENDER_WIDE selects), in
-// two forms with the same nodes, tests and results a ray: trace_binary's single loop, and trace_binary_split's loop
-// split into interior nodes and leaves.
+// It is the pass's walk (faster on B200 than the wide-BVH walk of wide_bvh.cuh, which TRT_RENDER_WIDE selects).
 #pragma once
 #include "device_common.cuh"
 
 namespace trt {
 
 struct Hit { float t; uint32_t tri; float u, v; uint32_t inst, part; };
-
-struct Node { V3 bmin; uint32_t left_or_first; V3 bmax; uint32_t count; };
-__device__ __forceinline__ Node node_at(const DScene& S, uint32_t i) {
-    uint4 a = __ldg(S.nodes + 2ull * i), b = __ldg(S.nodes + 2ull * i + 1);
-    return {{bf(a.x), bf(a.y), bf(a.z)}, a.w, {bf(b.x), bf(b.y), bf(b.z)}, b.w};
-}
 
 // Three-input minimum and maximum (one instruction each on sm_100; exact, like two fminf / fmaxf).
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -28,15 +20,14 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return r;
 }
 
-// pathtrace.wgsl:732-739 ray_aabb (min and max are exact, so grouping them three at a time rounds nothing)
-__device__ __forceinline__ float ray_aabb(V3 o, V3 inv_d, V3 bmin, V3 bmax, float tmax) {
-    V3 t0 = (bmin - o) * inv_d;
-    V3 t1 = (bmax - o) * inv_d;
-    V3 tmin_v = vmin(t0, t1);
-    V3 tmax_v = vmax(t0, t1);
-    float tn = max3f(tmin_v.x, tmin_v.y, fmaxf(tmin_v.z, 0.0f));
-    float tf = min3f(tmax_v.x, tmax_v.y, fminf(tmax_v.z, tmax));
-    return tn <= tf ? tn : INF;
+// pathtrace.wgsl:732-739 ray_aabb over a node record's two halves, as a predicate and the entry distance (min and max are
+// exact, so grouping them three at a time rounds nothing).
+__device__ __forceinline__ bool box_hit(V3 o, V3 inv_d, const uint4& a, const uint4& b, float tmax, float& tn) {
+    const float x0 = (bf(a.x) - o.x) * inv_d.x, y0 = (bf(a.y) - o.y) * inv_d.y, z0 = (bf(a.z) - o.z) * inv_d.z;
+    const float x1 = (bf(b.x) - o.x) * inv_d.x, y1 = (bf(b.y) - o.y) * inv_d.y, z1 = (bf(b.z) - o.z) * inv_d.z;
+    tn = max3f(fminf(x0, x1), fminf(y0, y1), fmaxf(fminf(z0, z1), 0.0f));
+    const float tf = min3f(fmaxf(x0, x1), fmaxf(y0, y1), fminf(fmaxf(z0, z1), tmax));
+    return tn <= tf;
 }
 
 // pathtrace.wgsl:742-761 intersect_tri (Moller-Trumbore on the leaf's v0, e1, e2), t = INF for none.
@@ -75,165 +66,121 @@ struct WalkCount { uint32_t nodes, tris, units; };
 constexpr uint32_t WALK_GUARD = 1u << 20;
 
 // trace_units.wgsl:44-135, with a 64-entry stack of its own. Returns the hit (tri MISS for none).
+//
+// The loop is split in two (Aila and Laine's "while-while"): interior nodes in an inner loop until a leaf, then the
+// leaf (a unit's record, or a mesh's triangles). What bounds it is issue, above all of the half-rate integer and
+// min / max pipe, at 8-10 of 32 lanes a warp instruction: ncu on a 512 x 512 town, depth 1, had 65-69 % of issue slots
+// and 52-57 % of that pipe busy, DRAM and L2 below 10 %, and neither fewer loads a step, nor prefetching the stacked
+// nodes, nor packed two-lane arithmetic moved the time. So the step is short: a child's link and count come with its
+// box (the node is not read again when the walk descends into it), the box tests answer with predicates, a pair's four
+// loads share one address, indices are checked in 32 bits, and a stack entry is a node's index, read again when it is
+// popped (keeping the links on the stack took five more instructions a step than the two loads at a pop). Warp
+// instructions of that depth: 82.2 -> 75.1 M closest, 139.6 -> 125.4 M shadow; the city frame (720p, 1 spp, depth 4)
+// 4.89 -> 4.49 ms, the town (512 x 512, 16 spp) 18.34 -> 16.90 ms. With the loop unsplit (each node a round of one
+// loop) the walks of the camera's rays are no faster (4.56 ms); 7 or 9 blocks an SM instead of 8: 4.55 and 4.60 ms.
 template <bool COUNT>
-__device__ Hit trace_binary(const DScene& S, const Sections& X, uint32_t top, uint32_t n_units, V3 o, V3 d, float tmax,
-                            uint32_t mode, WalkCount* wc, bool* guard) {
+__device__ __forceinline__ Hit trace_binary(const DScene& S, const Sections& X, uint32_t top, uint32_t n_units, V3 o, V3 d,
+                                            float tmax, uint32_t mode, WalkCount* wc, bool* guard) {
     Hit hit{tmax, MISS, 0.0f, 0.0f, NO_INST, 0u};
     if (n_units == 0) return hit;
     if (top >= S.n_nodes) { *guard = true; return hit; }
     V3 inv_d = safe_inv(d);
-    Node whole = node_at(S, top);
-    if (COUNT) wc->nodes++;
-    if (ray_aabb(o, inv_d, whole.bmin, whole.bmax, hit.t) == INF) return hit;
-    uint32_t stack[64];
-    uint32_t sp = 0, node = top, rec = NO_INST;
-    V3 ro = o, rd = d, rinv = inv_d;
-    uint32_t off = top, first = 0, base = 0;
-    for (uint32_t iter = 0;; ++iter) {
-        // (Every index a walk follows is checked: a bad tree ends the walk with the guard set, never a fault.)
-        if (iter >= WALK_GUARD || node >= S.n_nodes) { *guard = true; break; }
-        Node n = node_at(S, node);
+    // The buffers' ends in 32 bits, as the indices are: the last node (a pair of children starts before it), the
+    // triangles, the tables.
+    const uint32_t last_node = (uint32_t)min((unsigned long long)S.n_nodes - 1ull, 0xffffffffull);
+    const uint32_t tris_end = (uint32_t)min((unsigned long long)S.n_tris, 0xffffffffull);
+    const uint32_t tables_end = (uint32_t)min((unsigned long long)S.n_table_vec4, 0xffffffffull);
+    // The node the walk is at: `count` 0, an interior node, `at` its left child's index; else a leaf, `at` the first
+    // of its `count` items.
+    uint32_t at, count;
+    {
+        const uint4* q = S.nodes + 2ull * top;
+        const uint4 a = __ldg(q), b = __ldg(q + 1);
+        float t;
         if (COUNT) wc->nodes++;
-        if (n.count == 0) {
-            uint32_t l = off + n.left_or_first, r = l + 1;
-            if (r >= S.n_nodes) { *guard = true; break; }
-            Node nl = node_at(S, l), nr = node_at(S, r);
-            if (COUNT) wc->nodes += 2;
-            float tl = ray_aabb(ro, rinv, nl.bmin, nl.bmax, hit.t);
-            float tr = ray_aabb(ro, rinv, nr.bmin, nr.bmax, hit.t);
-            if (tl != INF || tr != INF) {
-                uint32_t nearn = l, farn = r;
-                if (tr < tl) { nearn = r; farn = l; float tmp = tl; tl = tr; tr = tmp; }
-                node = nearn;
-                if (tr != INF && sp < 64) stack[sp++] = farn;
-                continue;
-            }
-        } else if (rec == NO_INST) {
-            uint32_t b = X.t_instances + n.left_or_first * 10u;
-            if ((uint64_t)b + 10u > S.n_table_vec4) { *guard = true; break; }
-            float4 n1 = tab(S, b + 4);
-            uint32_t ubits = bu(n1.w);
-            if (COUNT) wc->units++;
-            if (mode != TRACE_SHADOW || (ubits & UNIT_SHADOW) != 0) {
-                float4 m0 = tab(S, b), m1 = tab(S, b + 1), m2 = tab(S, b + 2), n0 = tab(S, b + 3), n2 = tab(S, b + 5);
-                uint4 info = tabu(S, b + 6);
-                rec = n.left_or_first;
-                ro = o - V3{m0.w, m1.w, m2.w};
-                if ((ubits & UNIT_SHIFTED) == 0) {
-                    ro = proc_dir(n0, n1, n2, ro);
-                    rd = proc_dir(n0, n1, n2, d);
-                    rinv = safe_inv(rd);
-                }
-                off = bu(n0.w);
-                first = info.x;
-                base = sp;
-                node = off;
-                continue;
-            }
-        } else {
-            for (uint32_t k = 0; k < n.count; ++k) {
-                uint32_t ti = first + n.left_or_first + k;
-                if (ti >= S.n_tris) { *guard = true; return hit; }
-                if (COUNT) wc->tris++;
-                float3 x = intersect_tri(S, ro, rd, ti, hit.t);
-                if (x.x < hit.t) {
-                    uint32_t part = bu(__ldg(S.leaves + 3ull * ti).w);
-                    hit = Hit{x.x, ti, x.y, x.z, rec, part};
-                    if (mode != TRACE_CLOSEST) return hit;
-                }
-            }
-        }
-        if (rec != NO_INST && sp == base) {
+        if (!box_hit(o, inv_d, a, b, hit.t, t)) return hit;
+        if (COUNT) wc->nodes++;
+        count = b.w;
+        at = count == 0 ? a.w + top : a.w;
+    }
+    uint32_t stack[64];
+    uint32_t sp = 0, rec = NO_INST;
+    constexpr uint32_t NO_BASE = 0xffffffffu;  // (base outside a unit: no height of the stack)
+    uint32_t off = top, first = 0, base = NO_BASE;
+    V3 ro = o, rd = d, rinv = inv_d;
+    // Out of a unit whose subtree is done, then the next node (false: the walk is over).
+    auto pop = [&]() -> bool {
+        if (sp == base) {
             rec = NO_INST;
+            base = NO_BASE;
             ro = o; rd = d; rinv = inv_d;
             off = top;
         }
-        if (sp == 0) break;
-        sp--;
-        node = stack[sp];
-    }
-    return hit;
-}
-
-// The same walk with its loop split in two (Aila and Laine's "while-while"): interior nodes in an inner loop until a
-// leaf, then the leaf. A ray's nodes, tests, pops and result are trace_binary's; only the lanes of a warp fall into
-// step differently. Measured on B200 (the city frame): the shadow walks 6 % faster with it (2.49 -> 2.33 ms a
-// frame, compiled for 8 blocks an SM); the closest-hit walk 4.6 % slower with it on every depth but 2 % faster on
-// the depths past the camera's rays, so the shadow walks and the closest-hit walks past depth 0 use this one.
-template <bool COUNT>
-__device__ Hit trace_binary_split(const DScene& S, const Sections& X, uint32_t top, uint32_t n_units, V3 o, V3 d, float tmax,
-                            uint32_t mode, WalkCount* wc, bool* guard) {
-    Hit hit{tmax, MISS, 0.0f, 0.0f, NO_INST, 0u};
-    if (n_units == 0) return hit;
-    if (top >= S.n_nodes) { *guard = true; return hit; }
-    V3 inv_d = safe_inv(d);
-    Node whole = node_at(S, top);
-    if (COUNT) wc->nodes++;
-    if (ray_aabb(o, inv_d, whole.bmin, whole.bmax, hit.t) == INF) return hit;
-    uint32_t stack[64];
-    uint32_t sp = 0, node = top, rec = NO_INST;
-    V3 ro = o, rd = d, rinv = inv_d;
-    uint32_t off = top, first = 0, base = 0;
+        if (sp == 0) return false;
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * stack[--sp]);
+        if (COUNT) wc->nodes++;
+        at = __ldg(q + 3);
+        count = __ldg(q + 7);
+        if (count == 0) at += off;
+        return true;
+    };
     uint32_t iter = 0;
-    // The pop after a node that leads nowhere: out of a unit whose subtree is done, then the next node (false: the walk
-    // is over).
-#define TRT_WALK_POP()                        \
-    (((rec != NO_INST && sp == base)          \
-          ? (rec = NO_INST, ro = o, rd = d, rinv = inv_d, off = top, 0) \
-          : 0),                               \
-     sp == 0 ? false : (node = stack[--sp], true))
     for (;;) {
-        // Interior nodes first, until a leaf (a unit's record or a mesh's triangles); the nodes, tests and pops are
-        // the single loop's, in the same order.
-        Node n;
-        for (;; ++iter) {
-            // (Every index a walk follows is checked: a bad tree ends the walk with the guard set, never a fault.)
-            if (iter >= WALK_GUARD || node >= S.n_nodes) { *guard = true; return hit; }
-            n = node_at(S, node);
-            if (COUNT) wc->nodes++;
-            if (n.count != 0) break;
-            uint32_t l = off + n.left_or_first, r = l + 1;
-            if (r >= S.n_nodes) { *guard = true; return hit; }
-            Node nl = node_at(S, l), nr = node_at(S, r);
+        // (Every index a walk follows is checked: a bad tree ends the walk with the guard set, never a fault.)
+        bool over = false;
+        while (count == 0) {
+            if (iter++ >= WALK_GUARD || at >= last_node) { *guard = true; return hit; }
+            const uint4* q = S.nodes + 2ull * at;
+            const uint4 l0 = __ldg(q), l1 = __ldg(q + 1), r0 = __ldg(q + 2), r1 = __ldg(q + 3);
             if (COUNT) wc->nodes += 2;
-            float tl = ray_aabb(ro, rinv, nl.bmin, nl.bmax, hit.t);
-            float tr = ray_aabb(ro, rinv, nr.bmin, nr.bmax, hit.t);
-            if (tl != INF || tr != INF) {
-                uint32_t nearn = l, farn = r;
-                if (tr < tl) { nearn = r; farn = l; float tmp = tl; tl = tr; tr = tmp; }
-                node = nearn;
-                if (tr != INF && sp < 64) stack[sp++] = farn;
-                continue;
+            float tl, tr;
+            const bool hl = box_hit(ro, rinv, l0, l1, hit.t, tl), hr = box_hit(ro, rinv, r0, r1, hit.t, tr);
+            if (hl || hr) {
+                const bool swap = hr && (!hl || tr < tl);
+                const uint32_t link = swap ? r0.w : l0.w;
+                count = swap ? r1.w : l1.w;
+                if (COUNT) wc->nodes++;
+                if (hl && hr && sp < 64) stack[sp++] = swap ? at : at + 1u;
+                at = count == 0 ? link + off : link;
+            } else if (!pop()) {
+                over = true;
+                break;
             }
-            if (!TRT_WALK_POP()) return hit;
         }
-        ++iter;
+        if (over) break;
+        if (iter++ >= WALK_GUARD) { *guard = true; return hit; }
         if (rec == NO_INST) {
-            uint32_t b = X.t_instances + n.left_or_first * 10u;
-            if ((uint64_t)b + 10u > S.n_table_vec4) { *guard = true; return hit; }
-            float4 n1 = tab(S, b + 4);
+            uint32_t b = X.t_instances + at * 10u;
+            if (tables_end < 10u || b > tables_end - 10u) { *guard = true; return hit; }
+            const uint4* u = S.tables + b;
+            const float4* uf = reinterpret_cast<const float4*>(u);
+            const float4 n1 = __ldg(uf + 4);
             uint32_t ubits = bu(n1.w);
             if (COUNT) wc->units++;
             if (mode != TRACE_SHADOW || (ubits & UNIT_SHADOW) != 0) {
-                float4 m0 = tab(S, b), m1 = tab(S, b + 1), m2 = tab(S, b + 2), n0 = tab(S, b + 3), n2 = tab(S, b + 5);
-                uint4 info = tabu(S, b + 6);
-                rec = n.left_or_first;
-                ro = o - V3{m0.w, m1.w, m2.w};
+                const float4 n0 = __ldg(uf + 3), n2 = __ldg(uf + 5);
+                rec = at;
+                ro = o - V3{__ldg(&uf[0].w), __ldg(&uf[1].w), __ldg(&uf[2].w)};
+                first = __ldg(&u[6].x);
                 if ((ubits & UNIT_SHIFTED) == 0) {
                     ro = proc_dir(n0, n1, n2, ro);
                     rd = proc_dir(n0, n1, n2, d);
                     rinv = safe_inv(rd);
                 }
                 off = bu(n0.w);
-                first = info.x;
                 base = sp;
-                node = off;
+                if (off > last_node) { *guard = true; return hit; }
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * off);
+                at = __ldg(q + 3);
+                count = __ldg(q + 7);
+                if (COUNT) wc->nodes++;
+                if (count == 0) at += off;
                 continue;
             }
         } else {
-            for (uint32_t k = 0; k < n.count; ++k) {
-                uint32_t ti = first + n.left_or_first + k;
-                if (ti >= S.n_tris) { *guard = true; return hit; }
+            for (uint32_t k = 0; k < count; ++k) {
+                uint32_t ti = first + at + k;
+                if (ti >= tris_end) { *guard = true; return hit; }
                 if (COUNT) wc->tris++;
                 float3 x = intersect_tri(S, ro, rd, ti, hit.t);
                 if (x.x < hit.t) {
@@ -243,9 +190,8 @@ __device__ Hit trace_binary_split(const DScene& S, const Sections& X, uint32_t t
                 }
             }
         }
-        if (!TRT_WALK_POP()) break;
+        if (!pop()) break;
     }
-#undef TRT_WALK_POP
     return hit;
 }
 
