@@ -82,11 +82,13 @@ typedef struct { float t; uint32_t tri; float u; float v; uint32_t inst; uint32_
 #define TRT_RENDER_COUNT      2u /* also count node visits, triangle tests and unit entries (a slower walk) */
 #define TRT_RENDER_WIDE       4u /* walk the 8-wide quantised BVH instead of the reference's binary trees */
 /* Coherence sorts on the device, per depth; the image does not depend on them, bit for bit. trt_render sorts hits by
- * material before shading when the scene has more than TRT_SORT_HITS_MIN_MATERIALS materials (measured: the city's
- * 4,201 and the crowd's 217 gain 3-10 %, the Cornell box's 4 loses 14 %), unless this flag is given; a server sorts
- * every step's hits unless its options' flags hold it: */
+ * instance and section (so by material) before shading when the scene has more than TRT_SORT_HITS_MIN_MATERIALS
+ * materials (measured: the city's 4,201 and the crowd's 217 gain 3-10 %, the Cornell box's 4 loses 14 %) and the wave
+ * at least TRT_SORT_HITS_MIN_PATHS paths, unless this flag is given; a server sorts the hits of every step of that size
+ * unless its options' flags hold it: */
 #define TRT_RENDER_UNSORTED_HITS 16u
 #define TRT_SORT_HITS_MIN_MATERIALS 32u
+#define TRT_SORT_HITS_MIN_PATHS 393216u
 /* Optional, measured slower on the city scene: secondary rays by (queue chunk, direction octant) before the
  * closest-hit walk, shadow rays by (position chunk, direction octant) in each light class before the shadow walk. */
 #define TRT_RENDER_SORT_RAYS      8u

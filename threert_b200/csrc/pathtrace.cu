@@ -532,9 +532,11 @@ __global__ void k_resolve(const Job* __restrict__ jobs, const Job one, PathBufs 
 // it, since a path's state, hit and random numbers belong to the path, not to its queue position.
 //   SORT_RAYS: the extend queue by (queue chunk, direction octant): a warp's rays start near one another (the chunk)
 //     and point the same way, so they walk the same nodes in the same order.
-//   SORT_HITS (on unless TRT_RENDER_UNSORTED_HITS): the shade queue by material, misses first: a warp then reads one
-//     material record and takes one set of branches, and the next depth's queue, appended in this order, starts its
-//     rays from one mesh.
+//   SORT_HITS (on unless TRT_RENDER_UNSORTED_HITS, in waves of TRT_SORT_HITS_MIN_PATHS): the shade queue by instance
+//     and section, misses first: a warp then reads one material record and takes one set of branches, and the next
+//     depth's queue, appended in this order, starts its rays from one mesh. The key is made of the hit record alone:
+//     the material row it stands for lay behind three dependent loads (the job, the instance, its row), which bounded
+//     the count (latency; 720p city frame 36 us a launch of 460,800 items under ncu). The frame 4.36 -> 4.32 ms.
 //   SORT_SHADOWS: the shadow rays by (position chunk, direction octant) in each light class.
 constexpr uint32_t SORT_BINS = 4096u, SORT_THREADS = 256u, SORT_PER_THREAD = 8u;
 constexpr uint32_t SORT_ITEMS = SORT_THREADS * SORT_PER_THREAD;
@@ -558,25 +560,17 @@ __device__ __forceinline__ uint32_t sort_item(const Queues& Q, const uint32_t* i
     return KIND == SORT_SHADOWS ? shadow_slot(Q, j, n0, n1) : in[j];
 }
 template <uint32_t KIND>
-__device__ __forceinline__ uint32_t sort_key(const Job* jobs, const PathBufs& B, const Queues& Q, uint32_t j,
-                                             uint32_t item, uint32_t shift) {
+__device__ __forceinline__ uint32_t sort_key(const PathBufs& B, const Queues& Q, uint32_t j, uint32_t item,
+                                             uint32_t shift) {
     if (KIND == SORT_RAYS) return ((j >> shift) << 3) | octant(B.d[item]);
     if (KIND == SORT_SHADOWS) return ((j >> shift) << 3) | octant(Q.sd[item]);
-    if (bu(Q.hit_a[item].w) == MISS) return 0u;
-    const Job& J = jobs[B.job[item]];
-    const DScene& S = J.wk.S;
-    Sections X(J.P);
-    uint2 hb = Q.hit_b[item];
-    uint32_t mat = 0;
-    if (hb.x != NO_INST) {
-        uint32_t rows = tabu(S, X.t_instances + hb.x * 10u + 6u).w;
-        mat = __ldg(S.words + X.w_rows + (rows + hb.y) * 4u) & ROW_MATERIAL;
-    }
-    return 1u + mat % (SORT_BINS - 1u);
+    const uint32_t tri = bu(Q.hit_a[item].w);
+    const uint2 hb = Q.hit_b[item];
+    return tri == MISS ? 0u : 1u + (hb.x + hb.y) % (SORT_BINS - 1u);
 }
 
 template <uint32_t KIND>
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_count(const Job* __restrict__ jobs, PathBufs B, Queues Q,
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_count(PathBufs B, Queues Q,
                                                             const uint32_t* __restrict__ in, uint32_t depth,
                                                             uint32_t shift) {
     __shared__ uint32_t h[SORT_BINS];
@@ -593,7 +587,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_count(const Job* __restri
 #pragma unroll
         for (uint32_t k = 0; k < SORT_PER_THREAD; ++k) {
             uint32_t j = base + k * SORT_THREADS + tid;
-            key[k] = j < n ? sort_key<KIND>(jobs, B, Q, j, sort_item<KIND>(Q, in, j, n0, n1), shift) & (SORT_BINS - 1u) : 0u;
+            key[k] = j < n ? sort_key<KIND>(B, Q, j, sort_item<KIND>(Q, in, j, n0, n1), shift) & (SORT_BINS - 1u) : 0u;
         }
 #pragma unroll
         for (uint32_t k = 0; k < SORT_PER_THREAD; ++k) {
@@ -1005,7 +999,7 @@ uint32_t chunk_shift(uint32_t cap) {
 template <uint32_t KIND>
 void launch_sort(trt_scene* s, Wave& W, const uint32_t* in, uint32_t* out, uint32_t depth, uint32_t cap, cudaStream_t st) {
     uint32_t shift = chunk_shift(cap);
-    k_sort_count<KIND><<<(cap + SORT_ITEMS - 1u) / SORT_ITEMS, SORT_THREADS, 0, st>>>(W.jobs, W.B, W.Q, in, depth, shift);
+    k_sort_count<KIND><<<(cap + SORT_ITEMS - 1u) / SORT_ITEMS, SORT_THREADS, 0, st>>>(W.B, W.Q, in, depth, shift);
     k_sort_scatter<KIND><<<(cap + 255u) / 256u, 256, 0, st>>>(W.Q, in, out, depth);
     s->launches += 2;
 }
@@ -1121,7 +1115,11 @@ int render_waves(trt_scene* s, const Params& P, uint32_t first_sample, uint32_t 
     uint32_t last = P.w[P_COUNTS + 2];
     // the material table's records (18 vec4 each) between its first row and the lights' first row
     const uint32_t n_materials = (P.w[P_TABLE_FIRST + 2] - P.w[P_TABLE_FIRST + 1]) / 18u;
-    const bool sort_hits = (flags & TRT_RENDER_UNSORTED_HITS) == 0 && n_materials > TRT_SORT_HITS_MIN_MATERIALS;
+    // (A small wave's sort is two launches of latency a depth, more than the shading it saves: a 512 x 512 town's wave
+    // of 262,144 paths 1.59 ms sorted, 1.52 unsorted; a 640 x 360 city's of 230,400 1.71 and 1.67; even at 410,000; the
+    // town at 524,288 2.59 and 2.59, the city at 518,400 2.84 and 2.95, at 921,600 4.32 and 4.50.)
+    const bool sort_hits = (flags & TRT_RENDER_UNSORTED_HITS) == 0 && n_materials > TRT_SORT_HITS_MIN_MATERIALS &&
+                           (uint64_t)n_idx * K >= TRT_SORT_HITS_MIN_PATHS;
     const uint32_t flags_eff = (flags & ~TRT_RENDER_UNSORTED_HITS) | (sort_hits ? 0u : TRT_RENDER_UNSORTED_HITS);
     const int blk = 128;
     int g_ext = grid_for((const void*)k_extend<COUNT, WIDE, false>, blk, c->sm_count);

@@ -141,7 +141,7 @@ void serve_enqueue(trt_server* s, uint32_t last, uint32_t size, cudaStream_t st)
     uint32_t grid = (size + blk - 1) / blk;
     cudaMemsetAsync(W.Q.cnt, 0, 4ull * (MAX_DEPTH * CNT_STRIDE + CNT_STRIDE), st);
     k_raygen<<<grid, blk, 0, st>>>(tj, 0u, W.B, W.Q, size, head);
-    bool sort_hits = (s->opt.flags & TRT_RENDER_UNSORTED_HITS) == 0;
+    bool sort_hits = (s->opt.flags & TRT_RENDER_UNSORTED_HITS) == 0 && size >= TRT_SORT_HITS_MIN_PATHS;
     // Each depth's shadow walk runs on the second stream beside the next depth's closest-hit walk, as trt_render
     // runs them: both read what the depth's shading wrote and write apart (visibility bits; hit records), and the
     // depth's resolve waits for the shadow walk (the join) before the next depth's hit sort rewrites its order.
@@ -152,7 +152,7 @@ void serve_enqueue(trt_server* s, uint32_t last, uint32_t size, cudaStream_t st)
         uint32_t* shade_q = raw;
         if (sort_hits) {
             shade_q = W.Q.qx;
-            k_sort_count<SORT_HITS><<<(size + SORT_ITEMS - 1u) / SORT_ITEMS, SORT_THREADS, 0, st>>>(tj, W.B, W.Q, raw,
+            k_sort_count<SORT_HITS><<<(size + SORT_ITEMS - 1u) / SORT_ITEMS, SORT_THREADS, 0, st>>>(W.B, W.Q, raw,
                                                                                                   depth, 0u);
             k_sort_scatter<SORT_HITS><<<(size + 255u) / 256u, 256, 0, st>>>(W.Q, raw, shade_q, depth);
         }
