@@ -1,11 +1,12 @@
-"""The ways a render's waves run give one image, bit for bit: hits shaded in the order they came or sorted. A path's
-random numbers, state and sums are its own, so the tolerance is none."""
+"""The ways a render's waves run give one image, bit for bit: hits shaded in the order they came or sorted, and small
+waves in one launch (a block's paths start to end) or as the wavefront's launches. A path's random numbers, state and
+sums are its own in each, so the tolerance is none."""
 import numpy as np
 import pytest
 
 from threert_b200 import _native as N
-from threert_b200 import prep
-from util import small_city, small_crowd
+from threert_b200 import prep, scenes
+from util import scaled_units_scene, small_city, small_crowd
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +32,41 @@ def test_sorted_hits_shade_the_same_image(gpu, make, w, h, spp):
     P = prep.prepare(make())
     S = gpu.upload(P)
     same(S, sized(P, w, h), spp, 0, N.TRT_RENDER_UNSORTED_HITS)
+
+
+# One pixel, ragged tiles, a path a block and the most paths of one round of blocks (94,720 on 148 SMs: 256 x 368 tiles
+# of one sample, 128 x 92 of eight), and one tile row past it; a sort flag keeps the wavefront.
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (1, 1, 37), (7, 5, 3), (33, 31, 1), (64, 64, 1), (250, 370, 1),
+                                     (256, 370, 1), (256, 372, 1), (127, 92, 8)])
+@pytest.mark.parametrize("make", [lambda: scenes.cornell(16, 16), small_city, scaled_units_scene])
+def test_small_waves_render_the_wavefronts_image(gpu, make, w, h, spp):
+    P = prep.prepare(make())
+    S = gpu.upload(P)
+    same(S, sized(P, w, h), spp, N.TRT_RENDER_DEPTH, N.TRT_RENDER_DEPTH | N.TRT_RENDER_SORT_RAYS)
+
+
+@pytest.mark.parametrize("bounces", [0, 1, 12])
+def test_small_waves_of_few_and_many_vertices(gpu, bounces):
+    P = prep.prepare(scenes.cornell(16, 16))
+    S = gpu.upload(P)
+    same(S, sized(P, 40, 24, max_bounces=bounces), 5, 0, N.TRT_RENDER_SORT_RAYS)
+
+
+def test_small_waves_resume_and_accumulate(gpu):
+    P = prep.prepare(small_city())
+    S = gpu.upload(P)
+    p = sized(P, 50, 30)
+    whole, _ = S.render_raw(p, 6)
+    S.render_raw(p, 2)
+    got, _ = S.render_raw(p, 4, first_sample=2, flags=N.TRT_RENDER_ACCUMULATE)
+    assert np.array_equal(whole.view(np.uint32), got.view(np.uint32))
+
+
+def test_a_scene_of_four_suns_and_one_of_no_lights(gpu):
+    """Every shadow slot of a vertex in use, and none."""
+    d = small_city()
+    d.lights = [prep.DirLight(direction=(0.3 * k - 0.5, -1.0, 0.2 * k), intensity=3000.0 * (k + 1)) for k in range(4)]
+    for desc in (d, prep.SceneDescription(d.meshes[:2], d.materials[:2], d.instances[:2], d.camera, preset=d.preset)):
+        P = prep.prepare(desc)
+        S = gpu.upload(P)
+        same(S, sized(P, 61, 43), 3, 0, N.TRT_RENDER_SORT_RAYS)

@@ -189,6 +189,26 @@ __device__ void camera_ray(const Params& P, uint32_t gx, uint32_t gy, const floa
     }
 }
 
+// A path's state at its camera ray.
+__device__ __forceinline__ void start_path(const Job& J, const PathBufs& B, uint32_t p, uint32_t gx, uint32_t gy) {
+    const Params& P = J.P;
+    uint32_t sample = J.first_sample + (p - J.slot_first) / J.n_idx;
+    Rng R{sample, pixel_seed(gx, gy, P.w[P_SIZE + 3]), 0u};
+    float cam[4];
+    R.rng4(R.dim(D_CAMERA), cam);
+    V3 o, d;
+    camera_ray(P, gx, gy, cam, o, d);
+    B.o[p] = f4(o, 0.0f);
+    B.d[p] = f4(d, bf(F_SPECULAR_BOUNCE | F_STRAIGHT));
+    B.thr[p] = f4(v3(1.0f), bf(gy * P.w[P_SIZE] + gx));
+    B.rad[p] = f4(v3(0.0f), bf(sample));
+    B.alb[p] = f4(v3(0.0f), 0.0f);
+    B.nrm[p] = f4(v3(0.0f), 0.0f);
+    B.mis_x[p] = f4(v3(0.0f), 0.0f);
+    B.mis_n[p] = f4(v3(0.0f), 0.0f);
+    B.nee_thr[p] = f4(v3(0.0f), bf(0u));
+}
+
 __global__ void k_raygen(const Job* __restrict__ jobs, uint32_t n_jobs, PathBufs B, Queues Q, uint32_t n_slots,
                          const StepHead* __restrict__ head) {
     if (head) n_jobs = head->n_jobs;
@@ -204,25 +224,8 @@ __global__ void k_raygen(const Job* __restrict__ jobs, uint32_t n_jobs, PathBufs
     }
     uint32_t at = warp_append(&Q.cnt[0], valid);
     if (!valid) return;
-    const Job& J = jobs[j];
-    const Params& P = J.P;
-    uint32_t w = P.w[P_SIZE];
     B.job[p] = j;
-    uint32_t sample = J.first_sample + (p - J.slot_first) / J.n_idx;
-    Rng R{sample, pixel_seed(gx, gy, P.w[P_SIZE + 3]), 0u};
-    float cam[4];
-    R.rng4(R.dim(D_CAMERA), cam);
-    V3 o, d;
-    camera_ray(P, gx, gy, cam, o, d);
-    B.o[p] = f4(o, 0.0f);
-    B.d[p] = f4(d, bf(F_SPECULAR_BOUNCE | F_STRAIGHT));
-    B.thr[p] = f4(v3(1.0f), bf(gy * w + gx));
-    B.rad[p] = f4(v3(0.0f), bf(sample));
-    B.alb[p] = f4(v3(0.0f), 0.0f);
-    B.nrm[p] = f4(v3(0.0f), 0.0f);
-    B.mis_x[p] = f4(v3(0.0f), 0.0f);
-    B.mis_n[p] = f4(v3(0.0f), 0.0f);
-    B.nee_thr[p] = f4(v3(0.0f), bf(0u));
+    start_path(jobs[j], B, p, gx, gy);
     Q.q[0][at] = p;
 }
 
@@ -312,7 +315,179 @@ __device__ __forceinline__ void push_shadow(const Queues& Q, uint32_t* cnt, uint
     Q.sp[at] = (p << 3) | slot;
 }
 
-// One path vertex: pathtrace.wgsl:4176-4477 from the hit on (the trace itself is k_extend's).
+// One path vertex: pathtrace.wgsl:4176-4477 from the hit on (the trace itself is k_extend's). `sink` takes the vertex's
+// shadow rays; whether the path goes on.
+template <class Sink>
+__device__ __forceinline__ bool shade_vertex(const Job& J, const PathBufs& B, uint32_t p, uint32_t depth, const Hit& hit,
+                                             Sink&& sink) {
+    const Params& P = J.P;
+    const DScene& S = J.wk.S;
+    Sections X(P);
+    float4 o4 = B.o[p], d4 = B.d[p], thr4 = B.thr[p], rad4 = B.rad[p];
+    V3 o = xyz(o4), d = xyz(d4), thr = xyz(thr4), radiance = xyz(rad4);
+    float last_pdf = o4.w;
+    uint32_t flags = bu(d4.w);
+    uint32_t pix = bu(thr4.w), sample = bu(rad4.w);
+    uint32_t w = P.w[P_SIZE];
+    Rng R{sample, pixel_seed(pix % w, pix / w, P.w[P_SIZE + 3]), depth};
+    float clamp_v = pf(P, P_MISC);
+    uint32_t last = P.w[P_COUNTS + 2];
+    bool straight = (flags & F_STRAIGHT) != 0;
+    uint32_t nee_mask = 0, vis = 0;
+    bool live = false;
+    if (hit.tri == MISS) {
+        V3 c = thr * sky_mis(S, X, P, d, depth > 0u ? last_pdf : 0.0f);
+        if (depth > 1u && !straight) {
+            float lum = luminance(c);
+            if (lum > clamp_v) c = c * (clamp_v / lum);
+        }
+        radiance = radiance + c;
+        flags |= F_DONE;
+    } else {
+        Surface s = surface(S, X, o, d, hit);
+        if (depth == 0u) {
+            V3 albedo = s.card ? s.emissive / fmaxf(fmaxf(s.emissive.x, fmaxf(s.emissive.y, s.emissive.z)), 1e-6f) : s.base;
+            B.alb[p] = f4(albedo, hit.t);  // (w: the first hit's distance, for TRT_RENDER_DEPTH)
+            B.nrm[p] = f4(s.n, 0.0f);
+        }
+        if (any_gt0(s.emissive) && (s.front || !s.card)) {
+            float wgt = 1.0f;
+            if (depth > 0u && (flags & F_SPECULAR_BOUNCE) == 0u)
+                wgt = emit_mis(S, X, P, hit, d, last_pdf, xyz(B.mis_x[p]), xyz(B.mis_n[p]));
+            V3 c = thr * s.emissive * wgt;
+            if (depth > 1u && !straight) {
+                float lum = luminance(c);
+                if (lum > clamp_v) c = c * (clamp_v / lum);
+            }
+            radiance = radiance + c;
+        }
+        if (s.card || depth == last) {
+            flags |= F_DONE;
+        } else {
+            V3 v = -d;
+            float nov = fmaxf(dot(s.n, v), 1e-4f);
+            Lobes lb = lobes(S, X, P, s, nov);
+            // direct_light (pathtrace.wgsl:2444-2546): each light's sample and its contribution if unoccluded.
+            V3 oo = offset_origin(s.p, s.ng);
+            uint32_t nd = min(P.w[P_COUNTS2], MAX_DIR_LIGHTS);
+            for (uint32_t li = 0; li < nd; ++li) {
+                uint32_t b = X.t_lights + li * 5u;
+                float4 dir = tab(S, b + 1);
+                float cos_max = dir.w;
+                V3 to_light = -xyz(dir);
+                float u[2];
+                R.rng2(rng_sub(R.dim(D_SUN), li), u);
+                float cos_t = 1.0f - u[0] * (1.0f - cos_max);
+                float sin_t = sqrtf(fmaxf(0.0f, 1.0f - cos_t * cos_t));
+                float phi = 2.0f * PI * u[1];
+                Mat3 tb = basis(to_light);
+                V3 l = mul(tb, V3{sin_t * cosf(phi), sin_t * sinf(phi), cos_t});
+                V3 color = xyz(tab(S, b + 2));
+                if (all_le0(color)) continue;
+                V3 f = eval_bsdf_k(s, lb, v, l, tab(S, b + 4).y);
+                if (any_gt0(f)) {
+                    float pdf_l = 1.0f / (2.0f * PI * (1.0f - cos_max));
+                    float wgt = light_mis(pdf_l, s, lb, v, l);
+                    B.nee[li * B.n + p] = f4(color * f * wgt * 1.0f, 0.0f);
+                    nee_mask |= 1u << li;
+                    if (tab(S, b + 3).w >= 0.5f) sink.shadow(CLASS_SUN, li, oo, l, INF, TRACE_SHADOW);
+                    else vis |= 1u << li;
+                }
+            }
+            V3 ne = s.n;
+            B.mis_x[p] = f4(oo, 0.0f);
+            B.mis_n[p] = f4(ne, 0.0f);
+            if (emitters_on(S, X, P)) {
+                // The candidates pathtrace.wgsl:2513 resamples: the tree's count at camera hits (one deeper),
+                // 6 / 3 without a tree where the camera sees the point, 2 with light LOD; else one CDF draw.
+                bool lt_on = pf(P, P_LTREE + 3) > 0.5f;
+                bool seen_directly = depth == 0u || (depth == 1u && (flags & F_MIRROR) != 0u);
+                uint32_t m = 0;
+                if (lt_on) m = depth == 0u ? (uint32_t)pf(P, P_LTREE + 3) : 1u;
+                else if (seen_directly) m = depth == 0u ? EMIT_RIS_M : EMIT_RIS_M / 2u;
+                else if (pf(P, P_LIGHT_LOD + 3) > 0.0f) m = 2u;
+                ES es = m > 0u ? sample_emitter_ris(S, X, P, R, oo, ne, m, s, lb, v, R.dim(D_EMIT))
+                               : sample_emitter(S, X, P, R, oo, ne, R.dim(D_EMIT));
+                if (es.pdf_w > 0.0f) {
+                    V3 f = eval_bsdf_k(s, lb, v, es.l, 1.0f);
+                    if (any_gt0(f)) {
+                        float wgt = light_mis(es.pdf_w, s, lb, v, es.l) * 1.0f;
+                        B.nee[SLOT_EMIT * B.n + p] = f4(es.le * f * wgt * es.w, 0.0f);
+                        nee_mask |= 1u << SLOT_EMIT;
+                        sink.shadow(CLASS_EMIT, SLOT_EMIT, oo, es.l, es.dist * 0.999f, TRACE_ANY);
+                    }
+                }
+            }
+            bool env_sampled = P.w[P_COUNTS2 + 1] != 0u && (pf(P, P_ENV) > 0.5f || luminance(pv(P, P_SKY)) > 0.0f);
+            if (env_sampled) {
+                V3 l = sample_env(S, P, R, R.dim(D_ENV));
+                V3 f = eval_bsdf_k(s, lb, v, l, 1.0f);
+                if (any_gt0(f)) {
+                    float pdf_e = env_pdf(S, P, l);
+                    if (pdf_e > 0.0f) {
+                        B.nee[SLOT_ENV * B.n + p] = f4(env_radiance(S, P, l) * f * light_mis(pdf_e, s, lb, v, l) / pdf_e * 1.0f, 0.0f);
+                        nee_mask |= 1u << SLOT_ENV;
+                        sink.shadow(CLASS_ENV, SLOT_ENV, oo, l, INF, TRACE_SHADOW);
+                    }
+                }
+            }
+            bool clamp_dl = depth > 0u && !straight;
+            B.nee_thr[p] = f4(thr, bf(nee_mask | (clamp_dl ? 0x100u : 0u)));
+            // sample_bsdf (pathtrace.wgsl:1848-1887, no coat, no glass)
+            Mat3 tbn = basis(s.n);
+            float r4[4];
+            R.rng4(R.dim(D_BSDF), r4);
+            bool sampled_spec = r4[1] < lb.p_spec;
+            V3 l;
+            if (sampled_spec) {
+                V3 hv = sample_vndf(v, tbn, s.roughness * s.roughness, r4[2], r4[3]);
+                l = reflect(-v, hv);
+            } else {
+                float rr = sqrtf(r4[2]);
+                float phi = 2.0f * PI * r4[3];
+                l = mul(tbn, V3{rr * cosf(phi), rr * sinf(phi), sqrtf(fmaxf(0.0f, 1.0f - rr * rr))});
+            }
+            float pdf = pdf_bsdf(s, lb, v, l);
+            V3 wgt = eval_bsdf_k(s, lb, v, l, 1.0f) / fmaxf(pdf, 1e-20f);
+            if (pdf <= 0.0f || all_le0(wgt)) {
+                flags |= F_DONE;
+            } else {
+                thr = thr * wgt;
+                bool mirror = (depth == 0u || (flags & F_MIRROR) != 0u) && s.roughness < MIRROR_ROUGHNESS && sampled_spec;
+                flags &= ~(F_SPECULAR_BOUNCE | F_STRAIGHT | F_MIRROR);
+                if (mirror) flags |= F_MIRROR;
+                if (depth >= P.w[P_COUNTS + 3]) {
+                    float q = fminf(fmaxf(thr.x, fmaxf(thr.y, thr.z)), 0.95f);
+                    if (R.rng1(R.dim(D_RR)) > q) flags |= F_DONE;
+                    else thr = thr / q;
+                }
+                if ((flags & F_DONE) == 0u) {
+                    o = offset_origin(s.p, dot(l, s.ng) < 0.0f ? -s.ng : s.ng);
+                    d = l;
+                    last_pdf = pdf;
+                    live = true;
+                }
+            }
+        }
+    }
+    B.vis[p] = vis;
+    if (nee_mask == 0u) B.nee_thr[p] = f4(v3(0.0f), bf(0u));
+    B.o[p] = f4(o, last_pdf);
+    B.d[p] = f4(d, bf(flags));
+    B.thr[p] = f4(thr, bf(pix));
+    B.rad[p] = f4(radiance, bf(sample));
+    return live;
+}
+
+struct QueueSink {
+    const Queues& Q;
+    uint32_t* cnt;
+    uint32_t p;
+    __device__ __forceinline__ void shadow(uint32_t cls, uint32_t slot, V3 o, V3 l, float tmax, uint32_t mode) const {
+        push_shadow(Q, cnt, cls, p, slot, o, l, tmax, mode);
+    }
+};
+
 template <bool MULTI>
 __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADE) k_shade(const Job* __restrict__ jobs, const Job one, PathBufs B, Queues Q,
                                                   uint32_t depth, const uint32_t* __restrict__ queue,
@@ -324,165 +499,10 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADE) k_shade(const Job* __re
     uint32_t p = 0;
     if (i < n) {
         p = queue[i];
-        const Job& J = MULTI ? jobs[B.job[p]] : one;
-        const Params& P = J.P;
-        const DScene& S = J.wk.S;
-        Sections X(P);
-        float4 o4 = B.o[p], d4 = B.d[p], thr4 = B.thr[p], rad4 = B.rad[p];
-        V3 o = xyz(o4), d = xyz(d4), thr = xyz(thr4), radiance = xyz(rad4);
-        float last_pdf = o4.w;
-        uint32_t flags = bu(d4.w);
-        uint32_t pix = bu(thr4.w), sample = bu(rad4.w);
-        uint32_t w = P.w[P_SIZE];
-        Rng R{sample, pixel_seed(pix % w, pix / w, P.w[P_SIZE + 3]), depth};
-        float clamp_v = pf(P, P_MISC);
-        uint32_t last = P.w[P_COUNTS + 2];
-        bool straight = (flags & F_STRAIGHT) != 0;
         float4 ha = Q.hit_a[p];
         uint2 hb = Q.hit_b[p];
-        Hit hit{ha.x, bu(ha.w), ha.y, ha.z, hb.x, hb.y};
-        uint32_t nee_mask = 0, vis = 0;
-        if (hit.tri == MISS) {
-            V3 c = thr * sky_mis(S, X, P, d, depth > 0u ? last_pdf : 0.0f);
-            if (depth > 1u && !straight) {
-                float lum = luminance(c);
-                if (lum > clamp_v) c = c * (clamp_v / lum);
-            }
-            radiance = radiance + c;
-            flags |= F_DONE;
-        } else {
-            Surface s = surface(S, X, o, d, hit);
-            if (depth == 0u) {
-                V3 albedo = s.card ? s.emissive / fmaxf(fmaxf(s.emissive.x, fmaxf(s.emissive.y, s.emissive.z)), 1e-6f) : s.base;
-                B.alb[p] = f4(albedo, hit.t);  // (w: the first hit's distance, for TRT_RENDER_DEPTH)
-                B.nrm[p] = f4(s.n, 0.0f);
-            }
-            if (any_gt0(s.emissive) && (s.front || !s.card)) {
-                float wgt = 1.0f;
-                if (depth > 0u && (flags & F_SPECULAR_BOUNCE) == 0u)
-                    wgt = emit_mis(S, X, P, hit, d, last_pdf, xyz(B.mis_x[p]), xyz(B.mis_n[p]));
-                V3 c = thr * s.emissive * wgt;
-                if (depth > 1u && !straight) {
-                    float lum = luminance(c);
-                    if (lum > clamp_v) c = c * (clamp_v / lum);
-                }
-                radiance = radiance + c;
-            }
-            if (s.card || depth == last) {
-                flags |= F_DONE;
-            } else {
-                V3 v = -d;
-                float nov = fmaxf(dot(s.n, v), 1e-4f);
-                Lobes lb = lobes(S, X, P, s, nov);
-                // direct_light (pathtrace.wgsl:2444-2546): each light's sample and its contribution if unoccluded.
-                V3 oo = offset_origin(s.p, s.ng);
-                uint32_t nd = min(P.w[P_COUNTS2], MAX_DIR_LIGHTS);
-                for (uint32_t li = 0; li < nd; ++li) {
-                    uint32_t b = X.t_lights + li * 5u;
-                    float4 dir = tab(S, b + 1);
-                    float cos_max = dir.w;
-                    V3 to_light = -xyz(dir);
-                    float u[2];
-                    R.rng2(rng_sub(R.dim(D_SUN), li), u);
-                    float cos_t = 1.0f - u[0] * (1.0f - cos_max);
-                    float sin_t = sqrtf(fmaxf(0.0f, 1.0f - cos_t * cos_t));
-                    float phi = 2.0f * PI * u[1];
-                    Mat3 tb = basis(to_light);
-                    V3 l = mul(tb, V3{sin_t * cosf(phi), sin_t * sinf(phi), cos_t});
-                    V3 color = xyz(tab(S, b + 2));
-                    if (all_le0(color)) continue;
-                    V3 f = eval_bsdf_k(s, lb, v, l, tab(S, b + 4).y);
-                    if (any_gt0(f)) {
-                        float pdf_l = 1.0f / (2.0f * PI * (1.0f - cos_max));
-                        float wgt = light_mis(pdf_l, s, lb, v, l);
-                        B.nee[li * B.n + p] = f4(color * f * wgt * 1.0f, 0.0f);
-                        nee_mask |= 1u << li;
-                        if (tab(S, b + 3).w >= 0.5f) push_shadow(Q, cnt, CLASS_SUN, p, li, oo, l, INF, TRACE_SHADOW);
-                        else vis |= 1u << li;
-                    }
-                }
-                V3 ne = s.n;
-                B.mis_x[p] = f4(oo, 0.0f);
-                B.mis_n[p] = f4(ne, 0.0f);
-                if (emitters_on(S, X, P)) {
-                    // The candidates pathtrace.wgsl:2513 resamples: the tree's count at camera hits (one deeper),
-                    // 6 / 3 without a tree where the camera sees the point, 2 with light LOD; else one CDF draw.
-                    bool lt_on = pf(P, P_LTREE + 3) > 0.5f;
-                    bool seen_directly = depth == 0u || (depth == 1u && (flags & F_MIRROR) != 0u);
-                    uint32_t m = 0;
-                    if (lt_on) m = depth == 0u ? (uint32_t)pf(P, P_LTREE + 3) : 1u;
-                    else if (seen_directly) m = depth == 0u ? EMIT_RIS_M : EMIT_RIS_M / 2u;
-                    else if (pf(P, P_LIGHT_LOD + 3) > 0.0f) m = 2u;
-                    ES es = m > 0u ? sample_emitter_ris(S, X, P, R, oo, ne, m, s, lb, v, R.dim(D_EMIT))
-                                   : sample_emitter(S, X, P, R, oo, ne, R.dim(D_EMIT));
-                    if (es.pdf_w > 0.0f) {
-                        V3 f = eval_bsdf_k(s, lb, v, es.l, 1.0f);
-                        if (any_gt0(f)) {
-                            float wgt = light_mis(es.pdf_w, s, lb, v, es.l) * 1.0f;
-                            B.nee[SLOT_EMIT * B.n + p] = f4(es.le * f * wgt * es.w, 0.0f);
-                            nee_mask |= 1u << SLOT_EMIT;
-                            push_shadow(Q, cnt, CLASS_EMIT, p, SLOT_EMIT, oo, es.l, es.dist * 0.999f, TRACE_ANY);
-                        }
-                    }
-                }
-                bool env_sampled = P.w[P_COUNTS2 + 1] != 0u && (pf(P, P_ENV) > 0.5f || luminance(pv(P, P_SKY)) > 0.0f);
-                if (env_sampled) {
-                    V3 l = sample_env(S, P, R, R.dim(D_ENV));
-                    V3 f = eval_bsdf_k(s, lb, v, l, 1.0f);
-                    if (any_gt0(f)) {
-                        float pdf_e = env_pdf(S, P, l);
-                        if (pdf_e > 0.0f) {
-                            B.nee[SLOT_ENV * B.n + p] = f4(env_radiance(S, P, l) * f * light_mis(pdf_e, s, lb, v, l) / pdf_e * 1.0f, 0.0f);
-                            nee_mask |= 1u << SLOT_ENV;
-                            push_shadow(Q, cnt, CLASS_ENV, p, SLOT_ENV, oo, l, INF, TRACE_SHADOW);
-                        }
-                    }
-                }
-                bool clamp_dl = depth > 0u && !straight;
-                B.nee_thr[p] = f4(thr, bf(nee_mask | (clamp_dl ? 0x100u : 0u)));
-                // sample_bsdf (pathtrace.wgsl:1848-1887, no coat, no glass)
-                Mat3 tbn = basis(s.n);
-                float r4[4];
-                R.rng4(R.dim(D_BSDF), r4);
-                bool sampled_spec = r4[1] < lb.p_spec;
-                V3 l;
-                if (sampled_spec) {
-                    V3 hv = sample_vndf(v, tbn, s.roughness * s.roughness, r4[2], r4[3]);
-                    l = reflect(-v, hv);
-                } else {
-                    float rr = sqrtf(r4[2]);
-                    float phi = 2.0f * PI * r4[3];
-                    l = mul(tbn, V3{rr * cosf(phi), rr * sinf(phi), sqrtf(fmaxf(0.0f, 1.0f - rr * rr))});
-                }
-                float pdf = pdf_bsdf(s, lb, v, l);
-                V3 wgt = eval_bsdf_k(s, lb, v, l, 1.0f) / fmaxf(pdf, 1e-20f);
-                if (pdf <= 0.0f || all_le0(wgt)) {
-                    flags |= F_DONE;
-                } else {
-                    thr = thr * wgt;
-                    bool mirror = (depth == 0u || (flags & F_MIRROR) != 0u) && s.roughness < MIRROR_ROUGHNESS && sampled_spec;
-                    flags &= ~(F_SPECULAR_BOUNCE | F_STRAIGHT | F_MIRROR);
-                    if (mirror) flags |= F_MIRROR;
-                    if (depth >= P.w[P_COUNTS + 3]) {
-                        float q = fminf(fmaxf(thr.x, fmaxf(thr.y, thr.z)), 0.95f);
-                        if (R.rng1(R.dim(D_RR)) > q) flags |= F_DONE;
-                        else thr = thr / q;
-                    }
-                    if ((flags & F_DONE) == 0u) {
-                        o = offset_origin(s.p, dot(l, s.ng) < 0.0f ? -s.ng : s.ng);
-                        d = l;
-                        last_pdf = pdf;
-                        live = true;
-                    }
-                }
-            }
-        }
-        B.vis[p] = vis;
-        if (nee_mask == 0u) B.nee_thr[p] = f4(v3(0.0f), bf(0u));
-        B.o[p] = f4(o, last_pdf);
-        B.d[p] = f4(d, bf(flags));
-        B.thr[p] = f4(thr, bf(pix));
-        B.rad[p] = f4(radiance, bf(sample));
+        live = shade_vertex(MULTI ? jobs[B.job[p]] : one, B, p, depth, Hit{ha.x, bu(ha.w), ha.y, ha.z, hb.x, hb.y},
+                            QueueSink{Q, cnt, p});
     }
     uint32_t at = warp_append(&Q.cnt[(depth + 1u) * CNT_STRIDE], live);
     if (live && depth + 1u < MAX_DEPTH) next[at] = p;
@@ -490,20 +510,13 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADE) k_shade(const Job* __re
 
 // The vertex's direct light from its visible slots (pathtrace.wgsl:4398-4403), and a finished path's last fixes
 // (4494-4497).
-template <bool MULTI>
-__global__ void k_resolve(const Job* __restrict__ jobs, const Job one, PathBufs B, Queues Q, uint32_t depth,
-                          const uint32_t* __restrict__ queue) {
-    uint32_t n = Q.cnt[depth * CNT_STRIDE];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t p = queue[i];
-    float clamp_v = pf(MULTI ? jobs[B.job[p]].P : one.P, P_MISC);
+__device__ __forceinline__ void resolve_vertex(const PathBufs& B, uint32_t p, float clamp_v, uint32_t vis) {
     float4 nt = B.nee_thr[p];
     uint32_t m = bu(nt.w);
     float4 rad4 = B.rad[p];
     V3 radiance = xyz(rad4);
     if (m & 0xffu) {
-        uint32_t vis = B.vis[p] & m;
+        vis &= m;
         V3 sum = v3(0.0f);
         for (uint32_t k = 0; k < N_SLOTS; ++k)
             if (vis & (1u << k)) sum = sum + xyz(B.nee[k * B.n + p]);
@@ -522,6 +535,145 @@ __global__ void k_resolve(const Job* __restrict__ jobs, const Job one, PathBufs 
         if (non_finite3(xyz(nn))) B.nrm[p] = f4(V3{0.0f, 1.0f, 0.0f}, 0.0f);
     }
     B.rad[p] = f4(radiance, rad4.w);
+}
+template <bool MULTI>
+__global__ void k_resolve(const Job* __restrict__ jobs, const Job one, PathBufs B, Queues Q, uint32_t depth,
+                          const uint32_t* __restrict__ queue) {
+    uint32_t n = Q.cnt[depth * CNT_STRIDE];
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t p = queue[i];
+    resolve_vertex(B, p, pf(MULTI ? jobs[B.job[p]].P : one.P, P_MISC), B.vis[p]);
+}
+
+// ---- small waves: every vertex of a block's paths in one launch ----
+//
+// A wave that does not fill the GPU is bound by latency: each depth's walks, shading and resolve are launches that wait
+// for their slowest ray (a 64 x 64 Cornell box: 30 launches, 350 us, of which a depth's closest-hit walk is 27 us with
+// its median warp done in 18). Here a block takes its paths from the camera to the end, with barriers among its four
+// warps only: a depth's rays (the paths' own, and the last vertices' shadow rays) are listed in shared memory and its
+// warps take them from the list, in chunks that spread few rays over all four; then each path's thread resolves the
+// last vertex and shades the next. The paths, the queues' places for their rays and the arithmetic are the wavefront's,
+// so the image is too, bit for bit. A path's three or four rays a vertex walk side by side (one after another in a
+// lane, without the list, the same waves took 1.2-1.5 times as long).
+// Per wave, launched as a wavefront and so (us): Cornell box 32 x 32 350 / 124, 64 x 64 351 / 152, 256 x 256 411 / 234;
+// a town (45,000 triangles) 32 x 32 674 / 225, 128 x 128 782 / 389, 256 x 256 863 / 640 (774 unsorted); past what the
+// GPU holds at once the wavefront's fuller warps win: 384 x 384 1,080 unsorted / 1,279. So it takes the waves whose
+// paths all fit on the GPU in one round of blocks (94,720 on 148 SMs).
+// Five blocks an SM (96 registers, nothing spilled): 640 us for that town's 256 x 256; 4 blocks 679, 6 668, 8 701.
+#ifndef TRT_BLOCKS_PATHS
+#define TRT_BLOCKS_PATHS 5
+#endif
+// A vertex's shadow rays, kept by path: each slot's direction and distance in that slot's place of the shadow queue.
+struct PathSink {
+    const Queues& Q;
+    uint32_t p, n;
+    uint32_t& pending;
+    __device__ __forceinline__ void shadow(uint32_t, uint32_t slot, V3, V3 l, float tmax, uint32_t) const {
+        Q.sd[place(Q, slot, p, n)] = f4(l, tmax);
+        pending |= 1u << slot;
+    }
+    // (a sun's slot: the n paths' places of that sun; the others: their class's region)
+    static __device__ __forceinline__ uint32_t place(const Queues& Q, uint32_t slot, uint32_t p, uint32_t n) {
+        return slot < MAX_DIR_LIGHTS ? slot * n + p : Q.class_base[slot - SLOT_EMIT + CLASS_EMIT] + p;
+    }
+};
+constexpr uint32_t PATHS_BLOCK = 128u;
+// per_block: paths a block takes at once (at most its threads); paths: the wave's, for the totals.
+__global__ void __launch_bounds__(PATHS_BLOCK, TRT_BLOCKS_PATHS) k_paths(const Job one, PathBufs B, Queues Q, uint32_t n,
+                                                                        uint32_t per_block, uint32_t paths) {
+    constexpr uint32_t CLOSEST = 7u;  // the path's own ray, beside the slots of its vertex's shadow rays
+    __shared__ uint32_t s_ray[PATHS_BLOCK * (N_SLOTS + 1u)];  // a depth's rays: path << 3 | slot
+    __shared__ Hit s_hit[PATHS_BLOCK];
+    __shared__ uint32_t s_vis[PATHS_BLOCK];
+    __shared__ uint32_t s_count[2], s_next;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    const Params& P = one.P;
+    const Sections X(P);
+    unsigned long long guard_trips = 0, closest = 0, shadows = 0;
+    for (uint32_t first = blockIdx.x * per_block; first < n; first += gridDim.x * per_block) {
+        const uint32_t p = first + tid;
+        uint32_t gx = 0, gy = 0, pending = 0;
+        bool live = tid < per_block && p < n &&
+                    slot_pixel(p % one.n_idx + one.pix_first, P.w[P_SIZE], P.w[P_SIZE + 1], gx, gy);
+        bool shaded = false;
+        if (live) start_path(one, B, p, gx, gy);
+        for (uint32_t depth = 0;; ++depth) {
+            // The depth's rays into the list: the paths' own first, then the last vertices' shadow rays.
+            if (tid < 2u) s_count[tid] = 0u;
+            if (tid == 2u) s_next = 0u;
+            __syncthreads();
+            const uint32_t own = __ballot_sync(0xffffffffu, live), mine = __popc(pending);
+            uint32_t incl = mine;
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            uint32_t at0 = 0, at1 = 0;
+            if (lane == 31u) {
+                at0 = atomicAdd(&s_count[0], (uint32_t)__popc(own));
+                at1 = atomicAdd(&s_count[1], incl);
+            }
+            at0 = __shfl_sync(0xffffffffu, at0, 31) + __popc(own & ((1u << lane) - 1u));
+            at1 = __shfl_sync(0xffffffffu, at1, 31) + incl - mine;
+            if (live) s_ray[at0] = (tid << 3) | CLOSEST;
+            __syncthreads();
+            const uint32_t n_own = s_count[0], n_rays = n_own + s_count[1];
+            for (uint32_t m = pending; m != 0u; m &= m - 1u) s_ray[n_own + at1++] = (tid << 3) | (__ffs(m) - 1);
+            __syncthreads();
+            if (n_rays == 0u) break;
+            const uint32_t chunk = min(32u, (n_rays + PATHS_BLOCK / 32u - 1u) / (PATHS_BLOCK / 32u));
+            for (;;) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&s_next, chunk);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (at >= n_rays) break;
+                at += lane;
+                if (lane < chunk && at < n_rays) {
+                    const uint32_t id = s_ray[at], q = id >> 3, slot = id & 7u, pq = first + q;
+                    float4 o, d;
+                    float tmax = INF;
+                    uint32_t mode = TRACE_CLOSEST;
+                    if (slot == CLOSEST) {
+                        o = B.o[pq];
+                        d = B.d[pq];
+                    } else {
+                        o = B.mis_x[pq];  // (the vertex's offset point, where its shadow rays start)
+                        d = Q.sd[PathSink::place(Q, slot, pq, n)];
+                        tmax = d.w;
+                        mode = slot == SLOT_EMIT ? TRACE_ANY : TRACE_SHADOW;
+                    }
+                    bool guard = false;
+                    WalkCount wc{0, 0, 0};
+                    const Hit h = trace_binary<false>(one.wk.S, X, one.wk.top, one.wk.n_units, xyz(o), xyz(d), tmax, mode, &wc, &guard);
+                    if (guard) guard_trips++;
+                    if (slot == CLOSEST) {
+                        s_hit[q] = h;
+                        closest++;
+                    } else {
+                        if (h.tri == MISS) atomicOr(&s_vis[q], 1u << slot);
+                        shadows++;
+                    }
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            if (shaded) resolve_vertex(B, p, pf(P, P_MISC), s_vis[tid]);
+            shaded = live;
+            pending = 0u;
+            if (live) {
+                const Hit hit = s_hit[tid];
+                live = shade_vertex(one, B, p, depth, hit, PathSink{Q, p, n, pending});
+                s_vis[tid] = B.vis[p];
+            }
+        }
+        __syncthreads();
+    }
+    warp_add64(&Q.totals[T_GUARD], guard_trips);
+    warp_add64(&Q.totals[T_CLOSEST], closest);
+    warp_add64(&Q.totals[T_SHADOW], shadows);
+    if (blockIdx.x == 0 && tid == 0) atomicAdd(&Q.totals[T_PATHS], (unsigned long long)paths);
 }
 
 // ---- coherence sorts ----
@@ -1125,10 +1277,25 @@ int render_waves(trt_scene* s, const Params& P, uint32_t first_sample, uint32_t 
     int g_ext = grid_for((const void*)k_extend<COUNT, WIDE, false>, blk, c->sm_count);
     int g_sha = grid_for((const void*)k_shadow<COUNT, WIDE, false>, blk, c->sm_count);
     std::vector<uint32_t> host_cnt(MAX_DEPTH * CNT_STRIDE + CNT_STRIDE, 0);
+    // A wave that the GPU holds in one round of blocks takes k_paths (the counted, the wide and the profiled walks and the
+    // optional sorts are the wavefront's).
+    const uint32_t path_blocks = (uint32_t)grid_for((const void*)k_paths, (int)PATHS_BLOCK, c->sm_count);
+    const bool small = !COUNT && !WIDE && !s->profiling && (uint64_t)n_idx * K <= (uint64_t)path_blocks * PATHS_BLOCK &&
+                       (flags & (TRT_RENDER_SORT_RAYS | TRT_RENDER_SORT_SHADOWS)) == 0;
     for (uint32_t s0 = 0; s0 < spp; s0 += K) {
         uint32_t k = std::min(K, spp - s0);
         const uint32_t depth_flag = (flags & TRT_RENDER_DEPTH) ? 1u : 0u;
         Job job_a{P, wk, s->accum, 0u, n_idx_a, k, first_sample + s0, 0u, depth_flag, 0u};
+        if (small) {
+            const uint32_t n = n_idx * k;
+            const uint32_t per_block = (n + path_blocks - 1u) / path_blocks;
+            const uint32_t grid = (n + per_block - 1u) / per_block;
+            k_put_job<<<1, 128, 0, st>>>(job_a, s->wave.jobs, 0u);
+            k_paths<<<grid, PATHS_BLOCK, 0, st>>>(job_a, s->wave.B, s->wave.Q, n, per_block, w * h * k);
+            k_accumulate<<<dim3((n_idx + blk - 1) / blk, 1), blk, 0, st>>>(s->wave.jobs, s->wave.B);
+            s->launches += 3;
+            continue;
+        }
         TRT_CUDA(c, cudaMemcpyAsync(s->wave.Q.cnt, host_cnt.data(), host_cnt.size() * 4, cudaMemcpyHostToDevice, st));
         if (halves) {
             // The second half on its own stream pair, after what the main stream holds so far; joined at the end.
