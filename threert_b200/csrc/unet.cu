@@ -70,13 +70,11 @@ constexpr uint32_t TS = 5;                  // pipeline stages (82 KB of shared 
 constexpr uint32_t A_STAGE = 128u * 32u * 2u, B_STAGE = 128u * 32u * 2u;
 constexpr uint32_t CONV_SMEM = TS * (A_STAGE + B_STAGE) + 256u + 1024u;  // + room to align the stages to 1 KB
 // The halo variant (a row tile of 128 pixels read once with its halo, the taps as shifted descriptors): a stage is a
-// 32-channel block as four planes of 8 channels x 3 rows x 130 pixels (16 bytes a pixel, each plane padded to a
-// multiple of 128 bytes), the weights resident.
+// 32-channel block's 3 rows x 130 pixels, 64 bytes a pixel in the 64-byte swizzle, padded to a multiple of 1 KB.
 constexpr uint32_t HALO_W = 130u, HALO_ROWS = 3u;
-constexpr uint32_t HALO_PLANE = (HALO_ROWS * HALO_W * 16u + 127u) / 128u * 128u;  // 6,272 bytes
-constexpr uint32_t HALO_STAGE = 4u * HALO_PLANE, HALO_TS = 3u;
-constexpr uint32_t HALO_W_OFF = (HALO_TS * HALO_STAGE + 1023u) / 1024u * 1024u;  // the resident weights, 1 KB aligned
-constexpr uint32_t HALO_A_ALIGNED = (HALO_STAGE + 1023u) / 1024u * 1024u;  // a streaming stage's weights start here
+constexpr uint32_t HALO_BYTES = HALO_ROWS * HALO_W * 64u, HALO_STAGE = (HALO_BYTES + 1023u) / 1024u * 1024u;
+constexpr uint32_t HALO_TS = 3u;
+constexpr uint32_t HALO_W_OFF = HALO_TS * HALO_STAGE;                            // the resident weights
 constexpr uint32_t SMEM_MAX = 227u * 1024u;                                      // dynamic shared memory a CTA
 // The halo variant's shared memory: the stages, then every (32-channel block, tap) weight box of the output tile
 // (nt rows of 64 bytes each), then the barriers.
@@ -144,13 +142,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int c
 __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr, uint32_t sbo) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) |
            (1ull << 46) | (4ull << 61);
-}
-// The canonical K-major shared-memory matrix without swizzle: core matrices of 8 rows x 16 bytes, rows 16 bytes
-// apart, `sbo` bytes between core matrices along M / N and `lbo` bytes between the two along K (8 elements each);
-// descriptor version 1, layout type 0. The start may be any 16-byte boundary.
-__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 // kind::f16 instruction descriptor: f32 accumulator, bf16 A and B, both K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc(uint32_t M, uint32_t N) {
@@ -228,16 +219,19 @@ __device__ __forceinline__ void conv_store16(const Conv& a, uint64_t p, uint32_t
 
 // HALO: tiles of 128 x 1 pixels, the weights resident (every 32-channel block of one output tile) or, where they do
 // not fit, streamed with the activations (a stage then also holds its block's nine weight boxes), and a stage is one
-// block of the tile's activations with their halo (four TMA boxes of 8 channels x 130 pixels x 3 rows, no swizzle) from which
-// the nine taps' A operands are read by descriptors shifted (dy x 130 + dx) rows of 16 bytes: one load a tile instead
-// of nine. The taps' MMAs read rows [dy x 130 + dx, + 128) of each plane, inside the box.
+// block of the tile's activations with their halo (one TMA box of 32 channels x 130 pixels x 3 rows, 64-byte swizzle) from
+// which the nine taps' A operands are read by descriptors shifted (dy x 130 + dx) rows of 64 bytes: one load a tile
+// instead of nine. The taps' MMAs read rows [dy x 130 + dx, + 128) of the box.
+// The box's rows bound the loads: as four boxes of 8 channels without swizzle, a pixel was four requests of 16 bytes,
+// half of each 32-byte sector fetched; as one of 64 bytes the 1280 x 720 forward went from 957 to 843 us (1920 x 1080,
+// two images: 3,740 -> 3,105), the same bits.
 template <bool HALO>
 __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant__ CUtensorMap xmap,
                                                        const __grid_constant__ CUtensorMap wmap, Conv a) {
     // stages, and a stage's bytes: the halo variant's activations, and where the weights are not resident the nine
     // taps' weight boxes of the stage's 32-channel block after them
     const uint32_t NS = HALO ? a.stages : TS;
-    const uint32_t A_BYTES = HALO ? (a.resident ? HALO_STAGE : HALO_A_ALIGNED + 9u * a.nt * 64u) : A_STAGE;
+    const uint32_t A_BYTES = HALO ? (a.resident ? HALO_STAGE : HALO_STAGE + 9u * a.nt * 64u) : A_STAGE;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t sraw = smem_addr(smem_raw), sbase = (sraw + 1023u) & ~1023u;
@@ -321,15 +315,14 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                     if (it >= NS && !(ok = mbar_wait(empty(s), ((it / NS) - 1u) & 1u, a.err, abort_flag))) break;
                     const bool withhold = a.hold && blockIdx.x == 0 && it == 0;
                     if constexpr (HALO) {
-                        // the tile's rows y0 - 1 .. y0 + 1, pixels x0 - 1 .. x0 + 128, one box a plane of 8 channels
-                        mbar_expect_tx(full(s), 4u * HALO_ROWS * HALO_W * 16u + (a.resident ? 0u : 9u * a.nt * 64u));
+                        // the tile's rows y0 - 1 .. y0 + 1, pixels x0 - 1 .. x0 + 128
+                        mbar_expect_tx(full(s), HALO_BYTES + (a.resident ? 0u : 9u * a.nt * 64u));
                         if (!withhold)
-                            for (uint32_t pl = 0; pl < 4u; ++pl)
-                                tma_load_4d(sA + s * A_BYTES + pl * HALO_PLANE, &xmap, (int)(a.x_off + k * 32u + pl * 8u),
-                                            x0 - 1, y0 - 1, (int)b, full(s));
+                            tma_load_4d(sA + s * A_BYTES, &xmap, (int)(a.x_off + k * 32u), x0 - 1, y0 - 1, (int)b,
+                                        full(s));
                         if (!a.resident)
                             for (uint32_t tap = 0; tap < 9u; ++tap)
-                                tma_load_3d(sA + s * A_BYTES + HALO_A_ALIGNED + tap * a.nt * 64u, &wmap, (int)(k * 32u),
+                                tma_load_3d(sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
                                             (int)n0, (int)tap, full(s));
                     } else {
                         mbar_expect_tx(full(s), A_STAGE + (a.resident ? 0u : a.nt * 64u));
@@ -362,15 +355,15 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                     if (!(ok = mbar_wait(full(s), (it / NS) & 1u, a.err, abort_flag))) break;
                     tc_fence_after();
                     if constexpr (HALO) {
-                        // tap (dy, dx): rows from (dy + 1) x 130 + dx + 1 of planes 2j, 2j + 1 (K 16 each MMA)
+                        // tap (dy, dx): 128 rows of 64 bytes from row (dy + 1) x 130 + dx + 1 (the swizzle goes by
+                        // the address, so a start inside its 8-row pattern reads what the copy wrote)
                         for (uint32_t tap = 0; tap < 9u; ++tap) {
                             const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
 #pragma unroll
                             for (uint32_t j = 0; j < 2u; ++j) {
-                                uint64_t ad = umma_desc_plain(sA + s * A_BYTES + 2u * j * HALO_PLANE + row * 16u,
-                                                              HALO_PLANE, 128u);
+                                uint64_t ad = umma_desc_sw64(sA + s * A_BYTES + row * 64u + j * 32u, 512u);
                                 const uint32_t wb = a.resident ? sB + (k * 9u + tap) * a.nt * 64u
-                                                               : sA + s * A_BYTES + HALO_A_ALIGNED + tap * a.nt * 64u;
+                                                               : sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u;
                                 uint64_t bd = umma_desc_sw64(wb + j * 32u, 512u);
                                 umma_f16(d, ad, bd, idesc, (k | tap | j) != 0u ? 1u : 0u);
                             }
@@ -959,10 +952,9 @@ void tile_shape(uint32_t W, uint32_t H, uint32_t& bw, uint32_t& bh, uint32_t& ti
 }
 
 // A tensor map of an activation: (channels, x, y, image) with `stride` channels a pixel, boxes of 32 channels x bw x bh
-// pixels landing as 64-byte rows with the 64-byte swizzle (halo: boxes of 8 channels x bw x bh pixels, 16 bytes a
-// pixel, no swizzle); reads outside the tensor are zeros.
+// pixels landing as 64-byte rows with the 64-byte swizzle; reads outside the tensor are zeros.
 bool act_map(Net* n, CUtensorMap* m, const bf16* p, uint32_t stride, uint32_t B, uint32_t H, uint32_t W, uint32_t bw,
-             uint32_t bh, bool halo = false) {
+             uint32_t bh) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) {
         n->conv_err = "unet: cuTensorMapEncodeTiled is not available";
@@ -970,9 +962,9 @@ bool act_map(Net* n, CUtensorMap* m, const bf16* p, uint32_t stride, uint32_t B,
     }
     cuuint64_t d[4] = {stride, W, H, B};
     cuuint64_t st[3] = {(cuuint64_t)stride * 2u, (cuuint64_t)W * stride * 2u, (cuuint64_t)H * W * stride * 2u};
-    cuuint32_t box[4] = {halo ? 8u : 32u, bw, bh, 1u}, es[4] = {1u, 1u, 1u, 1u};
+    cuuint32_t box[4] = {32u, bw, bh, 1u}, es[4] = {1u, 1u, 1u, 1u};
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(p), d, st, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, halo ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         n->conv_err = "unet: an activation's tensor map was refused (" + std::to_string((int)r) + ")";
@@ -994,7 +986,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     uint32_t resident = cin == 32u && co_pad == nt && 9u * nt * 64u <= TS * B_STAGE ? 1u : 0u;
     // A layer of one output tile whose weights fit in shared memory beside three halo stages (up to four 32-channel
     // blocks at 64 outputs, two at 128), on an image at least 128 wide, reads its activations once a tile with the
-    // halo: row tiles of 128 pixels (the last of a row ragged), boxes of 8 channels x 130 x 3, the weights resident.
+    // halo: row tiles of 128 pixels (the last of a row ragged), boxes of 32 channels x 130 x 3, the weights resident.
     // (Row tiles that would leave more than an eighth of their pixels outside the image keep the 2-D tiles: at
     // 320 x 180 the row tiles measured 24.2 against 20.8 us.)
     const uint32_t kc = cin / 32u, row_tiles = (W + 127u) / 128u;
@@ -1002,7 +994,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     const bool halo_res = rows_ok && co_pad == nt && conv_smem_halo(kc, nt) <= SMEM_MAX;
     // Other layers on such levels stream each stage's nine weight boxes beside its activations, one CTA an SM: as
     // many stages (up to three) as fit.
-    const uint32_t stream_stage = HALO_A_ALIGNED + 9u * nt * 64u;
+    const uint32_t stream_stage = HALO_STAGE + 9u * nt * 64u;
     const uint32_t stream_ns = std::min(HALO_TS, (SMEM_MAX - 1280u) / stream_stage);
     const bool halo = halo_res || (rows_ok && stream_ns >= 2u);
     const uint32_t stages = halo_res ? HALO_TS : stream_ns;
@@ -1019,9 +1011,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     // the activations: boxes of 32 channels x bw x bh; the weights: (input channel, output channel, tap), boxes of
     // 32 x nt x 1; both 64-byte rows with the 64-byte swizzle
     CUtensorMap xmap, wmap;
-    if (!(halo ? act_map(n, &xmap, x, x_stride, B, H, W, HALO_W, HALO_ROWS, true)
-               : act_map(n, &xmap, x, x_stride, B, H, W, bw, bh)))
-        return;
+    if (!act_map(n, &xmap, x, x_stride, B, H, W, halo ? HALO_W : bw, halo ? HALO_ROWS : bh)) return;
     cuuint64_t wd[3] = {cin, co_pad, 9u};
     cuuint64_t ws[2] = {(cuuint64_t)cin * 2u, (cuuint64_t)co_pad * cin * 2u};
     cuuint32_t wb[3] = {32u, nt, 1u}, es[3] = {1u, 1u, 1u};
