@@ -1593,12 +1593,11 @@ int trt_denoise_atrous(trt_scene* s, uint32_t iterations, float* rgb_host, float
         uint64_t need = 0;
         auto add = [&](uint64_t b) { uint64_t at = need; need += (b + 255) / 256 * 256; return at; };
         uint64_t o_c0 = add(16ull * n), o_c1 = add(16ull * n), o_v0 = add(4ull * n), o_v1 = add(4ull * n),
-                 o_vf = add(4ull * n), o_a = add(16ull * n), o_n = add(16ull * n), o_rgb = add(12ull * n);
-        (void)o_rgb;
+                 o_n = add(16ull * n), o_a = add(8ull * n), o_rgb = add(12ull * n);
         TRT_CUDA(c, cudaMalloc(&s->dn, need));
         char* b = (char*)s->dn;
         s->D = DenoiseBufs{{(float4*)(b + o_c0), (float4*)(b + o_c1)}, {(float*)(b + o_v0), (float*)(b + o_v1)},
-                           (float*)(b + o_vf), (float4*)(b + o_a), (float4*)(b + o_n)};
+                           (float4*)(b + o_n), (float2*)(b + o_a)};
         s->dn_rgb = (float*)(b + o_rgb);
         s->dn_w = w;
         s->dn_h = h;
@@ -1607,13 +1606,11 @@ int trt_denoise_atrous(trt_scene* s, uint32_t iterations, float* rgb_host, float
     uint32_t grid = (n + blk - 1) / blk;
     if (ms) TRT_CUDA(c, cudaEventRecord(c->t0, st));
     k_dn_prep<<<grid, blk, 0, st>>>(s->accum, n, s->D);
-    uint32_t src = 0;
-    for (uint32_t it = 0; it < iterations; ++it) {
-        k_dn_var3<<<grid, blk, 0, st>>>(s->D.var[src], s->D.var_f, w, h);
-        k_dn_atrous<<<grid, blk, 0, st>>>(s->D, src, w, h, 1 << it);
-        src ^= 1u;
-    }
-    k_dn_remod<<<grid, blk, 0, st>>>(s->D, src, n, s->dn_rgb);
+    const uint32_t tiles = (w + DN_TILE_X - 1u) / DN_TILE_X * ((h + DN_TILE_Y - 1u) / DN_TILE_Y);
+    for (uint32_t it = 0; it < iterations; ++it)
+        k_dn_atrous<<<tiles, DN_TILE_X * DN_TILE_Y, 0, st>>>(s->D, it & 1u, w, h, 1 << it,
+                                                                 it + 1u == iterations ? s->dn_rgb : nullptr);
+    if (iterations == 0) k_dn_remod<<<grid, blk, 0, st>>>(s->D, n, s->dn_rgb);
     if (ms) TRT_CUDA(c, cudaEventRecord(c->t1, st));
     TRT_CUDA(c, cudaGetLastError());
     TRT_CUDA(c, cudaMemcpyAsync(rgb_host, s->dn_rgb, 12ull * n, cudaMemcpyDeviceToHost, st));
