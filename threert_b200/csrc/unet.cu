@@ -59,6 +59,8 @@ struct Conv {
     uint32_t B, H, W, x_off;
     uint32_t bw, bh, tiles_x, tiles_y;
     int relu;
+    const bf16* mask;         // or: the ReLU's gradient, outputs zeroed where this activation (NHWC) is not positive
+    uint32_t mask_stride;
     uint32_t* err;
     uint32_t resident;        // 1: every tap's weights loaded once a CTA (one 32-channel block, one output tile)
     uint32_t hold;            // 1: CTA 0 withholds its first activation box (trt_unet_hold_next_load: a test of the
@@ -181,6 +183,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The ReLU's gradient on 8 bf16 values in place: 0 where the activation is not positive.
+__device__ __forceinline__ void relu_mask8(uint4 y, uint32_t v[4]) {
+    const uint32_t w[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        v[i] &= (f.x > 0.0f ? 0xffffu : 0u) | (f.y > 0.0f ? 0xffff0000u : 0u);
+    }
+}
 // The epilogue of one accumulator row (a pixel) and 16 columns from `c`: bias, ReLU, bf16 NHWC (or the f32 output).
 __device__ __forceinline__ void conv_store16(const Conv& a, uint64_t p, uint32_t c, float* v) {
     if (a.bias) {
@@ -208,12 +219,17 @@ __device__ __forceinline__ void conv_store16(const Conv& a, uint64_t p, uint32_t
             __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
             pk[i] = *reinterpret_cast<uint32_t*>(&h2);
         }
+        if (a.mask) {
+            const uint4* m4 = reinterpret_cast<const uint4*>(a.mask + p * a.mask_stride + c);
+            relu_mask8(__ldg(m4), pk);
+            relu_mask8(__ldg(m4 + 1), pk + 4);
+        }
         uint4* dst = reinterpret_cast<uint4*>(a.y + p * a.y_stride + a.y_off + c);
         dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
     } else {
         for (int i = 0; i < 16; ++i)
-            if (c + i < a.cout) a.y[p * a.y_stride + a.y_off + c + i] = __float2bfloat16_rn(v[i]);
+            if (c + i < a.cout) a.y[p * a.y_stride + a.y_off + c + i] = __float2bfloat16_rn(v[i]);  // (never masked)
     }
 }
 
@@ -601,8 +617,8 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ CU
 
 // The partials of k_wgrad summed over a group's runs: a block takes 32 outputs (a group's accumulator row and 4
 // columns each, of the slots that hold a pair and the first row of the ones slot) x 8 segments of runs (segment j:
-// runs j, j + 8, ...), the segments then summed in order; every sum is taken in the same order on every call. Added
-// into dw[t][c][n] and db[n].
+// runs j, j + 8, ...), the segments then summed in order; every sum is taken in the same order on every call. Stored to
+// dw[t][c][n] and db[n] (columns past the outputs' multiple of 32 keep the zeros they were allocated as).
 constexpr uint32_t WS_SEGS = 8u;
 __global__ void __launch_bounds__(32u * WS_SEGS) k_wgrad_sum(const float* __restrict__ part, uint32_t runs,
                                                              uint32_t groups, uint32_t n_cols, uint32_t kc,
@@ -636,10 +652,8 @@ __global__ void __launch_bounds__(32u * WS_SEGS) k_wgrad_sum(const float* __rest
         s.z += v.z;
         s.w += v.w;
     }
-    float4* d = reinterpret_cast<float4*>(
-                    slot < pairs ? dw + ((uint64_t)(slot / kc) * cin + (slot % kc) * 32u + c) * co_pad : db) + q;
-    const float4 o = *d;
-    *d = make_float4(o.x + s.x, o.y + s.y, o.z + s.z, o.w + s.w);
+    *(reinterpret_cast<float4*>(slot < pairs ? dw + ((uint64_t)(slot / kc) * cin + (slot % kc) * 32u + c) * co_pad : db) +
+      q) = s;
 }
 
 // ---- the other layers ----------------------------------------------------------------------------------------------
@@ -675,18 +689,30 @@ __global__ void k_pool(const bf16* x, uint32_t xs, uint32_t xo, bf16* y, uint32_
     for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(0.25f * s[2 * e], 0.25f * s[2 * e + 1]);
     *reinterpret_cast<uint4*>(y + q * ys + c) = o;
 }
-// ... its gradient, added: dx[2y + j][2x + k] += dy[y][x] / 4.
-__global__ void k_pool_back(const bf16* dy, uint32_t dys, bf16* dx, uint32_t dxs, uint32_t dxo, uint32_t C, uint32_t B,
-                            uint32_t H, uint32_t W) {
+// An encoder output's gradient (C channels): the skip's (channels [so, so + C) of the concatenation's gradient) plus the
+// pooling's (dpool[y / 2][x / 2] / 4), zeroed where the output y (channels from yo) is not positive. 8 channels a thread.
+__global__ void k_skip_back(const bf16* __restrict__ dcat, uint32_t ds, uint32_t so, const bf16* __restrict__ dpool,
+                            const bf16* __restrict__ y, uint32_t ys, uint32_t yo, bf16* __restrict__ dx, uint32_t C,
+                            uint32_t B, uint32_t H, uint32_t W) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t n = (uint64_t)B * H * W * C;
-    if (i >= n) return;
-    uint32_t c = (uint32_t)(i % C);
-    uint64_t q = i / C;
-    uint32_t x = (uint32_t)(q % W), y = (uint32_t)((q / W) % H), b = (uint32_t)(q / ((uint64_t)W * H));
-    float g = 0.25f * __bfloat162float(dy[(((uint64_t)b * (H / 2) + y / 2) * (W / 2) + x / 2) * dys + c]);
-    bf16* d = dx + q * dxs + dxo + c;
-    *d = __float2bfloat16_rn(__bfloat162float(*d) + g);
+    const uint32_t c8 = C / 8u;
+    if (i >= (uint64_t)B * H * W * c8) return;
+    const uint32_t c = (uint32_t)(i % c8) * 8u;
+    const uint64_t q = i / c8;
+    const uint32_t px = (uint32_t)(q % W), py = (uint32_t)((q / W) % H), b = (uint32_t)(q / ((uint64_t)W * H));
+    const uint4 d4 = __ldg(reinterpret_cast<const uint4*>(dcat + q * ds + so + c));
+    const uint4 p4 = __ldg(reinterpret_cast<const uint4*>(dpool + (((uint64_t)b * (H / 2) + py / 2) * (W / 2) + px / 2) * C + c));
+    const uint32_t dv[4] = {d4.x, d4.y, d4.z, d4.w}, pv[4] = {p4.x, p4.y, p4.z, p4.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 d = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dv[k]));
+        const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pv[k]));
+        const __nv_bfloat162 r = __floats2bfloat162_rn(d.x + 0.25f * g.x, d.y + 0.25f * g.y);
+        o[k] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    relu_mask8(__ldg(reinterpret_cast<const uint4*>(y + q * ys + yo + c)), o);
+    *reinterpret_cast<uint4*>(dx + q * C + c) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 // Nearest 2x upsampling into channels [0, C) of y: y[2y + j][2x + k] = x[y][x].
 __global__ void k_up(const bf16* x, uint32_t xs, bf16* y, uint32_t ys, uint32_t C, uint32_t B, uint32_t H, uint32_t W) {
@@ -701,40 +727,42 @@ __global__ void k_up(const bf16* x, uint32_t xs, bf16* y, uint32_t ys, uint32_t 
     *reinterpret_cast<uint4*>(y + q * ys + c) =
         *reinterpret_cast<const uint4*>(x + (((uint64_t)b * (H / 2) + py / 2) * (W / 2) + px / 2) * xs + c);
 }
-// ... its gradient: dx[y][x] = sum of dy over the 2 x 2 block (channels [0, C) of dy).
-__global__ void k_up_back(const bf16* dy, uint32_t dys, bf16* dx, uint32_t dxs, uint32_t C, uint32_t B, uint32_t H,
-                          uint32_t W) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // over dx (H, W: dx's)
-    uint64_t n = (uint64_t)B * H * W * C;
-    if (i >= n) return;
-    uint32_t c = (uint32_t)(i % C);
-    uint64_t q = i / C;
-    uint32_t x = (uint32_t)(q % W), y = (uint32_t)((q / W) % H), b = (uint32_t)(q / ((uint64_t)W * H));
-    float s = 0.0f;
+// ... its gradient: dx[y][x] = sum of dy over the 2 x 2 block (channels [0, C) of dy), zeroed where the upsampled
+// activation y is not positive. Over dx (H, W: dx's, C channels a pixel there and in y), 8 channels a thread.
+__global__ void k_up_back(const bf16* __restrict__ dy, uint32_t dys, const bf16* __restrict__ y, bf16* __restrict__ dx,
+                          uint32_t C, uint32_t B, uint32_t H, uint32_t W) {
+    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t c8 = C / 8u;
+    if (i >= (uint64_t)B * H * W * c8) return;
+    const uint32_t c = (uint32_t)(i % c8) * 8u;
+    const uint64_t q = i / c8;
+    const uint32_t px = (uint32_t)(q % W), py = (uint32_t)((q / W) % H), b = (uint32_t)(q / ((uint64_t)W * H));
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
     for (int j = 0; j < 2; ++j)
-        for (int k = 0; k < 2; ++k)
-            s += __bfloat162float(dy[(((uint64_t)b * 2 * H + 2 * y + j) * 2 * W + 2 * x + k) * dys + c]);
-    dx[q * dxs + c] = __float2bfloat16_rn(s);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(
+                dy + (((uint64_t)b * 2 * H + 2 * py + j) * 2 * W + 2 * px + k) * dys + c));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]));
+                s[2 * e] += f.x;
+                s[2 * e + 1] += f.y;
+            }
+        }
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 r = __floats2bfloat162_rn(s[2 * e], s[2 * e + 1]);
+        o[e] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    relu_mask8(__ldg(reinterpret_cast<const uint4*>(y + q * C + c)), o);
+    *reinterpret_cast<uint4*>(dx + q * C + c) = make_uint4(o[0], o[1], o[2], o[3]);
 }
-// ReLU's gradient in place: dy = 0 where the layer's output y was 0.
-__global__ void k_relu_back(bf16* dy, uint32_t dys, uint32_t dyo, const bf16* y, uint32_t ys, uint32_t yo, uint32_t C,
-                            uint64_t P) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P * C) return;
-    uint64_t p = i / C;
-    uint32_t c = (uint32_t)(i % C);
-    if (!(__bfloat162float(y[p * ys + yo + c]) > 0.0f)) dy[p * dys + dyo + c] = __float2bfloat16_rn(0.0f);
-}
-// Copies channels [so, so + C) of a to channels [0, C) of b (the skip part of a concatenation's gradient).
-__global__ void k_copy_ch(const bf16* a, uint32_t as, uint32_t so, bf16* b, uint32_t bs, uint32_t bo, uint32_t C,
-                          uint64_t P) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P * C) return;
-    uint64_t p = i / C;
-    uint32_t c = (uint32_t)(i % C);
-    b[p * bs + bo + c] = a[p * as + so + c];
-}
-// The L1 loss on log radiance and its gradient (as bf16 into a 32-channel buffer): dpred = sign(pred - t) / count.
+// The L1 loss on log radiance and its gradient (as bf16 into a 32-channel buffer, whose channels past the third keep the
+// zeros they were allocated as): dpred = sign(pred - t) / count.
 __global__ void k_loss(const float* pred, const float* target, uint64_t P, bf16* dpred, float* loss) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     float l = 0.0f;
@@ -747,31 +775,42 @@ __global__ void k_loss(const float* pred, const float* target, uint64_t P, bf16*
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(~0u, l, o);
     if ((threadIdx.x & 31u) == 0 && l != 0.0f) atomicAdd(loss, l / (float)(P * 3));
 }
-// Adam (Kingma & Ba 2015) on the f32 master values, then the bf16 forward copy. `args`: the step's learning rate and
-// bias corrections 1 - b1^t, 1 - b2^t (device memory, so that a captured step reads each step's values).
-__global__ void k_adam(float* w, const float* g, float* m, float* v, uint64_t n, const float* args, float b1, float b2,
-                       float eps) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float lr = args[0], c1 = args[1], c2 = args[2];
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-// The bf16 weights of a layer from its f32 masters w[t][c][n], laid out as the convolution's B operand (per tap, the
+// A layer's place among the flat parameters and its bf16 weights, laid out as the convolution's B operand (per tap, the
 // output channels' rows of input channels): forward [t][n][c] (n < co_pad rows of cin), and the input gradient's
 // [8 - t][c][n] (c < cin of ci_pad64 rows: its output; n < cout32: the output gradient's channels, its input).
-__global__ void k_weights(const float* wf, uint32_t cin, uint32_t co_pad, uint32_t cout32, bf16* wfw, bf16* wbw,
-                          uint32_t ci_pad64) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t n = 9ull * cin * co_pad;
+struct LayerWeights {
+    uint32_t first, count, cin, co_pad, cout32, ci_pad64;  // its weights' first parameter and their number
+    bf16 *fw, *bw;                                         // bw: null for the first layer
+};
+constexpr int MAX_LAYERS = 15;
+struct WeightTable { LayerWeights l[MAX_LAYERS]; };
+// Adam (Kingma & Ba 2015) on the f32 master values (`args`, device memory so that a captured step reads each step's
+// values: the learning rate and the bias corrections 1 - b1^t, 1 - b2^t; null: no update), then every layer's bf16
+// weights from them, one launch for all (a launch a layer took 59 us of a training step under ncu, latency-bound).
+__global__ void k_adam_weights(float* w, const float* __restrict__ g, float* m, float* v, uint32_t n,
+                               const float* __restrict__ args, float b1, float b2, float eps,
+                               const __grid_constant__ WeightTable T) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t nn = (uint32_t)(i % co_pad), c = (uint32_t)((i / co_pad) % cin), t = (uint32_t)(i / ((uint64_t)co_pad * cin));
-    bf16 v = __float2bfloat16_rn(wf[i]);
-    wfw[((uint64_t)t * co_pad + nn) * cin + c] = v;
-    if (wbw && nn < cout32) wbw[((uint64_t)(8 - t) * ci_pad64 + c) * cout32 + nn] = v;
+    float wi = w[i];
+    if (args) {
+        const float lr = args[0], c1 = args[1], c2 = args[2];
+        const float gi = g[i];
+        const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+        m[i] = mi;
+        v[i] = vi;
+        wi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        w[i] = wi;
+    }
+    int li = 0;
+    while (li + 1 < MAX_LAYERS && i >= T.l[li + 1].first) ++li;
+    const LayerWeights& L = T.l[li];
+    const uint32_t k = i - L.first;
+    if (k >= L.count) return;  // (a bias)
+    const uint32_t nn = k % L.co_pad, c = (k / L.co_pad) % L.cin, t = k / (L.co_pad * L.cin);
+    const bf16 b = __float2bfloat16_rn(wi);
+    L.fw[(t * L.co_pad + nn) * L.cin + c] = b;
+    if (L.bw && nn < L.cout32) L.bw[((8u - t) * L.ci_pad64 + c) * L.cout32 + nn] = b;
 }
 
 // ---- features from a rendered accum (inference on a scene's result) ----------------------------------------------
@@ -922,6 +961,9 @@ struct Net {
     float *pred = nullptr, *target = nullptr, *feat = nullptr, *loss = nullptr, *sums = nullptr, *rgb = nullptr;
     std::vector<void*> allocs;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    // The backward pass's second stream: the weight gradients beside the chain of input gradients.
+    cudaStream_t aux = nullptr;
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     uint32_t* dev_err = nullptr;  // set by a convolution whose pipeline wait gave up
     bool hold_next = false;       // the next convolution launched outside a graph withholds one copy (a test)
     uint32_t sms = 148;           // the device's SMs (the persistent convolution's grid)
@@ -1011,7 +1053,7 @@ bool act_map(Net* n, CUtensorMap* m, const bf16* p, uint32_t stride, uint32_t B,
 // w [9][co_pad][cin] (each tap's output channels, their input channels contiguous).
 void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t cin, const bf16* w, uint32_t co_pad,
               const float* bias, bf16* y, uint32_t y_stride, uint32_t y_off, uint32_t cout, float* yf, uint32_t B,
-              uint32_t H, uint32_t W, int relu) {
+              uint32_t H, uint32_t W, int relu, const Act* mask = nullptr) {
     uint32_t bw, bh, tiles_x, tiles_y;
     tile_shape(W, H, bw, bh, tiles_x, tiles_y);
     const uint32_t nt = co_pad % 128u == 0u ? 128u : 64u;  // co_pad: a multiple of 64
@@ -1057,7 +1099,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
         return;
     }
     Conv a{cin, co_pad, nt, bias, y, y_stride, y_off, cout, yf, B, H, W, x_off, bw, bh, tiles_x, tiles_y, relu,
-           n->dev_err, resident, n->hold_next ? 1u : 0u, stages};
+           mask ? mask->p : nullptr, mask ? mask->stride : 0u, n->dev_err, resident, n->hold_next ? 1u : 0u, stages};
     n->hold_next = false;
     const uint32_t tiles = B * tiles_x * tiles_y * (co_pad / nt);
     const uint32_t grid = std::min<uint32_t>(tiles, n->sms * per_sm);
@@ -1071,14 +1113,17 @@ void conv(Net* n, int li, const Act& x, uint32_t x_off, const Act& y, uint32_t y
     conv_run(n, x.p, x.stride, x_off, L.cin, n->wf[li], r64(L.cout), n->w + n->off[li] + w_count(L), y.p, y.stride,
              y_off, L.cout, yf, B, H, W, L.relu);
 }
-// The input gradient of layer li: dx (channels [0, cin_logical)) from dy (cout rounded to 32 channels).
-void conv_dx(Net* n, int li, const Act& dy, const Act& dx, uint32_t B, uint32_t H, uint32_t W) {
+// The input gradient of layer li: dx (channels [0, cin_logical)) from dy (cout rounded to 32 channels); mask: the layer's
+// input where that is a ReLU's output, whose gradient it then is.
+void conv_dx(Net* n, int li, const Act& dy, const Act& dx, uint32_t B, uint32_t H, uint32_t W, const Act* mask = nullptr) {
     const Layer& L = LAYERS[li];
     conv_run(n, dy.p, dy.stride, 0u, r32(L.cout), n->wb[li], r64(L.cin), nullptr, dx.p, dx.stride, 0u, L.cin, nullptr,
-             B, H, W, 0);
+             B, H, W, 0, mask);
 }
 // The weight and bias gradients of layer li from its input x (channels [x_off, x_off + cin)) and its output gradient dy
-// (cout rounded to 32 channels), summed into the layer's gradients.
+// (cout rounded to 32 channels), into the layer's gradients: on the second stream, after what the first holds so far
+// (dy, which nothing later in the step writes). Each of these launches leaves SMs idle (a step's layers have 8 to 512
+// tiles), and none of the input gradients waits for them.
 void wgrad(Net* n, int li, const Act& x, uint32_t x_off, const Act& dy, uint32_t B, uint32_t H, uint32_t W) {
     const Layer& L = LAYERS[li];
     uint32_t bw, bh, tiles_x, tiles_y;
@@ -1104,13 +1149,21 @@ void wgrad(Net* n, int li, const Act& x, uint32_t x_off, const Act& dy, uint32_t
         return;
     }
     WGrad a{L.cin, x_off, kc, nb, pairs, n->wpart, bw, bh, tiles_x, tiles_y, tiles, chunk, ts, n->dev_err};
-    k_wgrad<<<dim3(chunks, groups), WG_THREADS, smem, n->stream>>>(xmap, dmap, a);
+    cudaEventRecord(n->fork_ev, n->stream);
+    cudaStreamWaitEvent(n->aux, n->fork_ev, 0);
+    k_wgrad<<<dim3(chunks, groups), WG_THREADS, smem, n->aux>>>(xmap, dmap, a);
     float* dw = n->g + n->off[li];
-    k_wgrad_sum<<<groups * 128u * nb * 8u / 32u, 32u * WS_SEGS, 0, n->stream>>>(
+    k_wgrad_sum<<<groups * 128u * nb * 8u / 32u, 32u * WS_SEGS, 0, n->aux>>>(
         n->wpart, chunks, groups, 32u * nb, kc, pairs, L.cin, r64(L.cout), dw, dw + w_count(L));
 }
-void relu_back(Net* n, const Act& dy, uint32_t dyo, const Act& y, uint32_t yo, uint32_t C, uint64_t P) {
-    k_relu_back<<<blocks(P * C), 256, 0, n->stream>>>(dy.p, dy.stride, dyo, y.p, y.stride, yo, C, P);
+void up_back(Net* n, const Act& dcat, const Act& y, const Act& dx, uint32_t B, uint32_t H, uint32_t W) {
+    k_up_back<<<blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream>>>(dcat.p, dcat.stride, y.p, dx.p,
+                                                                                  dx.stride, B, H, W);
+}
+void skip_back(Net* n, const Act& dcat, uint32_t off, const Act& dpool, const Act& cat, const Act& dx, uint32_t B,
+               uint32_t H, uint32_t W) {
+    k_skip_back<<<blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream>>>(
+        dcat.p, dcat.stride, off, dpool.p, cat.p, cat.stride, off, dx.p, dx.stride, B, H, W);
 }
 
 void forward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
@@ -1142,78 +1195,65 @@ void forward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
 }
 
 void backward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
-    cudaStream_t s = n->stream;
     uint32_t H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
-    uint64_t P0 = (uint64_t)B * H * W, P1 = (uint64_t)B * H1 * W1, P2 = (uint64_t)B * H2 * W2, P3 = (uint64_t)B * H3 * W3;
     // output layer (linear)
     wgrad(n, OUT, n->u0, 0, n->dpred, B, H, W);
-    conv_dx(n, OUT, n->dpred, n->du0, B, H, W);
+    conv_dx(n, OUT, n->dpred, n->du0, B, H, W, &n->u0);
     // level 0 decoder
-    relu_back(n, n->du0, 0, n->u0, 0, 32, P0);
     wgrad(n, D0B, n->t0, 0, n->du0, B, H, W);
-    conv_dx(n, D0B, n->du0, n->dt0, B, H, W);
-    relu_back(n, n->dt0, 0, n->t0, 0, 32, P0);
+    conv_dx(n, D0B, n->du0, n->dt0, B, H, W, &n->t0);
     wgrad(n, D0A, n->cat0, 0, n->dt0, B, H, W);
     conv_dx(n, D0A, n->dt0, n->dcat0, B, H, W);
-    k_up_back<<<blocks(P1 * 64), 256, 0, s>>>(n->dcat0.p, 96, n->du1.p, 64, 64, B, H1, W1);
-    k_copy_ch<<<blocks(P0 * 32), 256, 0, s>>>(n->dcat0.p, 96, 64, n->de0b.p, 32, 0, 32, P0);
+    up_back(n, n->dcat0, n->u1, n->du1, B, H1, W1);
     // level 1 decoder
-    relu_back(n, n->du1, 0, n->u1, 0, 64, P1);
     wgrad(n, D1B, n->t1, 0, n->du1, B, H1, W1);
-    conv_dx(n, D1B, n->du1, n->dt1, B, H1, W1);
-    relu_back(n, n->dt1, 0, n->t1, 0, 64, P1);
+    conv_dx(n, D1B, n->du1, n->dt1, B, H1, W1, &n->t1);
     wgrad(n, D1A, n->cat1, 0, n->dt1, B, H1, W1);
     conv_dx(n, D1A, n->dt1, n->dcat1, B, H1, W1);
-    k_up_back<<<blocks(P2 * 96), 256, 0, s>>>(n->dcat1.p, 160, n->du2.p, 96, 96, B, H2, W2);
-    k_copy_ch<<<blocks(P1 * 64), 256, 0, s>>>(n->dcat1.p, 160, 96, n->de1b.p, 64, 0, 64, P1);
+    up_back(n, n->dcat1, n->u2, n->du2, B, H2, W2);
     // level 2 decoder
-    relu_back(n, n->du2, 0, n->u2, 0, 96, P2);
     wgrad(n, D2B, n->t2, 0, n->du2, B, H2, W2);
-    conv_dx(n, D2B, n->du2, n->dt2, B, H2, W2);
-    relu_back(n, n->dt2, 0, n->t2, 0, 96, P2);
+    conv_dx(n, D2B, n->du2, n->dt2, B, H2, W2, &n->t2);
     wgrad(n, D2A, n->cat2, 0, n->dt2, B, H2, W2);
     conv_dx(n, D2A, n->dt2, n->dcat2, B, H2, W2);
-    k_up_back<<<blocks(P3 * 128), 256, 0, s>>>(n->dcat2.p, 224, n->db3.p, 128, 128, B, H3, W3);
-    k_copy_ch<<<blocks(P2 * 96), 256, 0, s>>>(n->dcat2.p, 224, 128, n->de2b.p, 96, 0, 96, P2);
+    up_back(n, n->dcat2, n->b3, n->db3, B, H3, W3);
     // bottleneck
-    relu_back(n, n->db3, 0, n->b3, 0, 128, P3);
     wgrad(n, E3B, n->a3, 0, n->db3, B, H3, W3);
-    conv_dx(n, E3B, n->db3, n->da3, B, H3, W3);
-    relu_back(n, n->da3, 0, n->a3, 0, 128, P3);
+    conv_dx(n, E3B, n->db3, n->da3, B, H3, W3, &n->a3);
     wgrad(n, E3A, n->pool2, 0, n->da3, B, H3, W3);
     conv_dx(n, E3A, n->da3, n->dpool2, B, H3, W3);
     // level 2 encoder (its output's gradient: the skip's and the pooling's)
-    k_pool_back<<<blocks(P2 * 96), 256, 0, s>>>(n->dpool2.p, 96, n->de2b.p, 96, 0, 96, B, H2, W2);
-    relu_back(n, n->de2b, 0, n->cat2, 128, 96, P2);
+    skip_back(n, n->dcat2, 128, n->dpool2, n->cat2, n->de2b, B, H2, W2);
     wgrad(n, E2B, n->a2, 0, n->de2b, B, H2, W2);
-    conv_dx(n, E2B, n->de2b, n->da2, B, H2, W2);
-    relu_back(n, n->da2, 0, n->a2, 0, 96, P2);
+    conv_dx(n, E2B, n->de2b, n->da2, B, H2, W2, &n->a2);
     wgrad(n, E2A, n->pool1, 0, n->da2, B, H2, W2);
     conv_dx(n, E2A, n->da2, n->dpool1, B, H2, W2);
     // level 1 encoder
-    k_pool_back<<<blocks(P1 * 64), 256, 0, s>>>(n->dpool1.p, 64, n->de1b.p, 64, 0, 64, B, H1, W1);
-    relu_back(n, n->de1b, 0, n->cat1, 96, 64, P1);
+    skip_back(n, n->dcat1, 96, n->dpool1, n->cat1, n->de1b, B, H1, W1);
     wgrad(n, E1B, n->a1, 0, n->de1b, B, H1, W1);
-    conv_dx(n, E1B, n->de1b, n->da1, B, H1, W1);
-    relu_back(n, n->da1, 0, n->a1, 0, 64, P1);
+    conv_dx(n, E1B, n->de1b, n->da1, B, H1, W1, &n->a1);
     wgrad(n, E1A, n->pool0, 0, n->da1, B, H1, W1);
     conv_dx(n, E1A, n->da1, n->dpool0, B, H1, W1);
     // level 0 encoder
-    k_pool_back<<<blocks(P0 * 32), 256, 0, s>>>(n->dpool0.p, 32, n->de0b.p, 32, 0, 32, B, H, W);
-    relu_back(n, n->de0b, 0, n->cat0, 64, 32, P0);
+    skip_back(n, n->dcat0, 64, n->dpool0, n->cat0, n->de0b, B, H, W);
     wgrad(n, E0B, n->a0, 0, n->de0b, B, H, W);
-    conv_dx(n, E0B, n->de0b, n->da0, B, H, W);
-    relu_back(n, n->da0, 0, n->a0, 0, 32, P0);
+    conv_dx(n, E0B, n->de0b, n->da0, B, H, W, &n->a0);
     wgrad(n, E0A, n->in0, 0, n->da0, B, H, W);
+    cudaEventRecord(n->join_ev, n->aux);
+    cudaStreamWaitEvent(n->stream, n->join_ev, 0);
 }
 
-void refresh_weights(Net* n) {
+// Adam's update (args not null) and every layer's bf16 weights.
+void refresh_weights(Net* n, const float* args) {
+    WeightTable T{};
+    static_assert(N_LAYERS == MAX_LAYERS, "the weight table's layers");
     for (int li = 0; li < N_LAYERS; ++li) {
         const Layer& L = LAYERS[li];
-        uint64_t cnt = w_count(L);
-        k_weights<<<blocks(cnt), 256, 0, n->stream>>>(n->w + n->off[li], L.cin, r64(L.cout), r32(L.cout), n->wf[li],
-                                                       li == E0A ? nullptr : n->wb[li], r64(L.cin));
+        T.l[li] = LayerWeights{(uint32_t)n->off[li], (uint32_t)w_count(L), L.cin, r64(L.cout), r32(L.cout), r64(L.cin),
+                               n->wf[li], li == E0A ? nullptr : n->wb[li]};
     }
+    k_adam_weights<<<blocks(n->n_params), 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, (uint32_t)n->n_params, args, 0.9f,
+                                                               0.999f, 1e-8f, T);
 }
 
 int check_size(Net* n, uint32_t B, uint32_t H, uint32_t W) {
@@ -1249,15 +1289,9 @@ void train_kernels(Net* n, uint32_t B, uint32_t H, uint32_t W, int update) {
     k_feat_host<<<blocks(P), 256, 0, s>>>(n->feat, P, n->in0.p);
     forward(n, B, H, W);
     cudaMemsetAsync(n->loss, 0, 4, s);
-    cudaMemsetAsync(n->dpred.p, 0, 2 * 32 * P, s);
-    cudaMemsetAsync(n->g, 0, 4 * n->n_params, s);
     k_loss<<<blocks(P * 3), 256, 0, s>>>(n->pred, n->target, P, n->dpred.p, n->loss);
     backward(n, B, H, W);
-    if (update) {
-        k_adam<<<blocks(n->n_params), 256, 0, s>>>(n->w, n->g, n->m, n->v, n->n_params, n->adam_args, 0.9f, 0.999f,
-                                                    1e-8f);
-        refresh_weights(n);
-    }
+    if (update) refresh_weights(n, n->adam_args);
 }
 
 // The training step's graph for this shape: captured from train_kernels on first use (a tensor map refused during
@@ -1337,6 +1371,9 @@ int trt_unet_create(int device, uint32_t max_batch, uint32_t max_h, uint32_t max
     }
     uint64_t P0 = (uint64_t)max_batch * max_h * max_w, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
     e = cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&n->aux, cudaStreamNonBlocking);
+    for (cudaEvent_t* ev : {&n->fork_ev, &n->join_ev})
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     auto A = [&](Act& a, uint64_t px, uint32_t st) { if (e == cudaSuccess) e = act(n, a, px, st); };
     if (e == cudaSuccess) e = alloc(n, &n->w, n->n_params);
     if (e == cudaSuccess) e = alloc(n, &n->g, n->n_params);
@@ -1393,11 +1430,15 @@ void trt_unet_destroy(trt_unet* n) {
     if (!n) return;
     cudaSetDevice(n->device);
     if (n->stream) cudaStreamSynchronize(n->stream);
+    if (n->aux) cudaStreamSynchronize(n->aux);
     for (const Net::StepGraph& g : n->graphs) cudaGraphExecDestroy(g.exec);
     if (n->adam_host) cudaFreeHost(n->adam_host);
     for (void* p : n->allocs) cudaFree(p);
     if (n->e0) cudaEventDestroy(n->e0);
     if (n->e1) cudaEventDestroy(n->e1);
+    if (n->fork_ev) cudaEventDestroy(n->fork_ev);
+    if (n->join_ev) cudaEventDestroy(n->join_ev);
+    if (n->aux) cudaStreamDestroy(n->aux);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
 }
@@ -1412,7 +1453,7 @@ int trt_unet_set_params(trt_unet* n, const float* params) {
     cudaMemsetAsync(n->m, 0, 4 * n->n_params, n->stream);
     cudaMemsetAsync(n->v, 0, 4 * n->n_params, n->stream);
     n->t = 0;
-    refresh_weights(n);
+    refresh_weights(n, nullptr);
     return cuda_check(n, cudaStreamSynchronize(n->stream), "params");
 }
 
