@@ -18,6 +18,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "threert_cuda.h"
@@ -28,6 +29,31 @@ namespace unet {
 typedef __nv_bfloat16 bf16;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// ---- programmatic dependent launches ----
+// The network's layers are a chain of short launches (5-60 us), so each is launched to start while the one before
+// drains: a kernel lets its successor start at once (pdl_trigger), does what does not depend on its predecessor
+// (barriers, tensor memory, resident weights), and waits for the predecessor's results (pdl_wait) before it reads or
+// writes anything of the chain. Weights are written by launches outside the chain (Adam, set_params), which the chain's
+// first kernel, launched plainly, waits for. early: false for a plain launch (the backward pass: its kernels share the
+// SMs with the weight gradients' stream, and blocks that wait early only held their room: 544 against 526 us a step).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+void launch_pdl(bool early, void (*kernel)(P...), dim3 grid, uint32_t block, uint32_t smem, cudaStream_t stream,
+                A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // ---- convolution (forward; and the input gradient with flipped, transposed weights) -------------------------------
 //
@@ -271,6 +297,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     const uint32_t ncols = 2u * a.nt;  // two accumulators of nt columns: 128 or 256
     const uint32_t per_img = a.tiles_x * a.tiles_y, n_ntiles = a.co_pad / a.nt;
     const uint32_t tiles = a.B * per_img * n_ntiles;
+    pdl_trigger();
 
     if (tid == 0) {
         for (uint32_t s = 0; s < NS; ++s) {
@@ -320,6 +347,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                     for (uint32_t tap = 0; tap < 9u; ++tap)
                         tma_load_3d(sB + (k * 9u + tap) * a.nt * 64u, &wmap, (int)(k * 32u), 0, (int)tap, wfull);
             }
+            pdl_wait();
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -406,6 +434,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
         // pixels of the tile) and half of the tile's columns, (w - 2) / 4 which
         const uint32_t quarter = warp & 3u, half = (warp - 2u) >> 2;
         const uint32_t m = quarter * 32u + lane, cols = a.nt / 2u, c_first = half * cols;
+        pdl_wait();
         uint32_t ti = 0;
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++ti) {
             const uint32_t acc = ti & 1u;
@@ -662,6 +691,8 @@ __global__ void __launch_bounds__(32u * WS_SEGS) k_wgrad_sum(const float* __rest
 __global__ void k_pool(const bf16* x, uint32_t xs, uint32_t xo, bf16* y, uint32_t ys, uint32_t C, uint32_t B,
                        uint32_t H, uint32_t W) {
     // 8 channels (16 bytes) a thread: C, the strides and the offsets are multiples of 32 channels
+    pdl_trigger();
+    pdl_wait();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t h2 = H / 2, w2 = W / 2, c8 = C / 8u;
     uint64_t n = (uint64_t)B * h2 * w2 * c8;
@@ -694,6 +725,8 @@ __global__ void k_pool(const bf16* x, uint32_t xs, uint32_t xo, bf16* y, uint32_
 __global__ void k_skip_back(const bf16* __restrict__ dcat, uint32_t ds, uint32_t so, const bf16* __restrict__ dpool,
                             const bf16* __restrict__ y, uint32_t ys, uint32_t yo, bf16* __restrict__ dx, uint32_t C,
                             uint32_t B, uint32_t H, uint32_t W) {
+    pdl_trigger();
+    pdl_wait();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t c8 = C / 8u;
     if (i >= (uint64_t)B * H * W * c8) return;
@@ -717,6 +750,8 @@ __global__ void k_skip_back(const bf16* __restrict__ dcat, uint32_t ds, uint32_t
 // Nearest 2x upsampling into channels [0, C) of y: y[2y + j][2x + k] = x[y][x].
 __global__ void k_up(const bf16* x, uint32_t xs, bf16* y, uint32_t ys, uint32_t C, uint32_t B, uint32_t H, uint32_t W) {
     // over the output (H, W: the output's), 8 channels (16 bytes) a thread
+    pdl_trigger();
+    pdl_wait();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t c8 = C / 8u;
     uint64_t n = (uint64_t)B * H * W * c8;
@@ -731,6 +766,8 @@ __global__ void k_up(const bf16* x, uint32_t xs, bf16* y, uint32_t ys, uint32_t 
 // activation y is not positive. Over dx (H, W: dx's, C channels a pixel there and in y), 8 channels a thread.
 __global__ void k_up_back(const bf16* __restrict__ dy, uint32_t dys, const bf16* __restrict__ y, bf16* __restrict__ dx,
                           uint32_t C, uint32_t B, uint32_t H, uint32_t W) {
+    pdl_trigger();
+    pdl_wait();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t c8 = C / 8u;
     if (i >= (uint64_t)B * H * W * c8) return;
@@ -963,6 +1000,7 @@ struct Net {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     // The backward pass's second stream: the weight gradients beside the chain of input gradients.
     cudaStream_t aux = nullptr;
+    bool early = true;            // the layers start while the one before drains (launch_pdl)
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     uint32_t* dev_err = nullptr;  // set by a convolution whose pipeline wait gave up
     bool hold_next = false;       // the next convolution launched outside a graph withholds one copy (a test)
@@ -1103,8 +1141,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     n->hold_next = false;
     const uint32_t tiles = B * tiles_x * tiles_y * (co_pad / nt);
     const uint32_t grid = std::min<uint32_t>(tiles, n->sms * per_sm);
-    if (halo) k_conv<true><<<grid, CONV_THREADS, smem, n->stream>>>(xmap, wmap, a);
-    else k_conv<false><<<grid, CONV_THREADS, CONV_SMEM, n->stream>>>(xmap, wmap, a);
+    launch_pdl(n->early, halo ? k_conv<true> : k_conv<false>, grid, CONV_THREADS, smem, n->stream, xmap, wmap, a);
 }
 
 void conv(Net* n, int li, const Act& x, uint32_t x_off, const Act& y, uint32_t y_off, uint32_t B, uint32_t H, uint32_t W,
@@ -1157,12 +1194,12 @@ void wgrad(Net* n, int li, const Act& x, uint32_t x_off, const Act& dy, uint32_t
         n->wpart, chunks, groups, 32u * nb, kc, pairs, L.cin, r64(L.cout), dw, dw + w_count(L));
 }
 void up_back(Net* n, const Act& dcat, const Act& y, const Act& dx, uint32_t B, uint32_t H, uint32_t W) {
-    k_up_back<<<blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream>>>(dcat.p, dcat.stride, y.p, dx.p,
+    launch_pdl(n->early, k_up_back, blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream, dcat.p, dcat.stride, y.p, dx.p,
                                                                                   dx.stride, B, H, W);
 }
 void skip_back(Net* n, const Act& dcat, uint32_t off, const Act& dpool, const Act& cat, const Act& dx, uint32_t B,
                uint32_t H, uint32_t W) {
-    k_skip_back<<<blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream>>>(
+    launch_pdl(n->early, k_skip_back, blocks((uint64_t)B * H * W * dx.stride / 8u), 256, 0, n->stream, 
         dcat.p, dcat.stride, off, dpool.p, cat.p, cat.stride, off, dx.p, dx.stride, B, H, W);
 }
 
@@ -1172,22 +1209,22 @@ void forward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
     uint64_t P0 = (uint64_t)B * H * W, P1 = (uint64_t)B * H1 * W1, P2 = (uint64_t)B * H2 * W2, P3 = (uint64_t)B * H3 * W3;
     conv(n, E0A, n->in0, 0, n->a0, 0, B, H, W);
     conv(n, E0B, n->a0, 0, n->cat0, 64, B, H, W);
-    k_pool<<<blocks(P1 * 32 / 8), 256, 0, s>>>(n->cat0.p, 96, 64, n->pool0.p, 32, 32, B, H, W);
+    launch_pdl(n->early, k_pool, blocks(P1 * 32 / 8), 256, 0, s, n->cat0.p, 96, 64, n->pool0.p, 32, 32, B, H, W);
     conv(n, E1A, n->pool0, 0, n->a1, 0, B, H1, W1);
     conv(n, E1B, n->a1, 0, n->cat1, 96, B, H1, W1);
-    k_pool<<<blocks(P2 * 64 / 8), 256, 0, s>>>(n->cat1.p, 160, 96, n->pool1.p, 64, 64, B, H1, W1);
+    launch_pdl(n->early, k_pool, blocks(P2 * 64 / 8), 256, 0, s, n->cat1.p, 160, 96, n->pool1.p, 64, 64, B, H1, W1);
     conv(n, E2A, n->pool1, 0, n->a2, 0, B, H2, W2);
     conv(n, E2B, n->a2, 0, n->cat2, 128, B, H2, W2);
-    k_pool<<<blocks(P3 * 96 / 8), 256, 0, s>>>(n->cat2.p, 224, 128, n->pool2.p, 96, 96, B, H2, W2);
+    launch_pdl(n->early, k_pool, blocks(P3 * 96 / 8), 256, 0, s, n->cat2.p, 224, 128, n->pool2.p, 96, 96, B, H2, W2);
     conv(n, E3A, n->pool2, 0, n->a3, 0, B, H3, W3);
     conv(n, E3B, n->a3, 0, n->b3, 0, B, H3, W3);
-    k_up<<<blocks(P2 * 128 / 8), 256, 0, s>>>(n->b3.p, 128, n->cat2.p, 224, 128, B, H2, W2);
+    launch_pdl(n->early, k_up, blocks(P2 * 128 / 8), 256, 0, s, n->b3.p, 128, n->cat2.p, 224, 128, B, H2, W2);
     conv(n, D2A, n->cat2, 0, n->t2, 0, B, H2, W2);
     conv(n, D2B, n->t2, 0, n->u2, 0, B, H2, W2);
-    k_up<<<blocks(P1 * 96 / 8), 256, 0, s>>>(n->u2.p, 96, n->cat1.p, 160, 96, B, H1, W1);
+    launch_pdl(n->early, k_up, blocks(P1 * 96 / 8), 256, 0, s, n->u2.p, 96, n->cat1.p, 160, 96, B, H1, W1);
     conv(n, D1A, n->cat1, 0, n->t1, 0, B, H1, W1);
     conv(n, D1B, n->t1, 0, n->u1, 0, B, H1, W1);
-    k_up<<<blocks(P0 * 64 / 8), 256, 0, s>>>(n->u1.p, 64, n->cat0.p, 96, 64, B, H, W);
+    launch_pdl(n->early, k_up, blocks(P0 * 64 / 8), 256, 0, s, n->u1.p, 64, n->cat0.p, 96, 64, B, H, W);
     conv(n, D0A, n->cat0, 0, n->t0, 0, B, H, W);
     conv(n, D0B, n->t0, 0, n->u0, 0, B, H, W);
     conv(n, OUT, n->u0, 0, Act{}, 0, B, H, W, n->pred);
@@ -1195,6 +1232,7 @@ void forward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
 }
 
 void backward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
+    n->early = false;
     uint32_t H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
     // output layer (linear)
     wgrad(n, OUT, n->u0, 0, n->dpred, B, H, W);
@@ -1241,6 +1279,7 @@ void backward(Net* n, uint32_t B, uint32_t H, uint32_t W) {
     wgrad(n, E0A, n->in0, 0, n->da0, B, H, W);
     cudaEventRecord(n->join_ev, n->aux);
     cudaStreamWaitEvent(n->stream, n->join_ev, 0);
+    n->early = true;
 }
 
 // Adam's update (args not null) and every layer's bf16 weights.
