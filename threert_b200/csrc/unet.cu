@@ -142,6 +142,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, uint32_t*
     }
     return true;
 }
+// The same by a whole warp, which goes on together (a wait that one lane gave up, all did).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t a, uint32_t parity, uint32_t* err, volatile uint32_t* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(a, parity, err, abort_flag)) != 0;
+}
 // A wait bounded at about 2^31 cycles that ignores the abort word: the drain of a CTA that gave up.
 __device__ __forceinline__ bool mbar_wait_drain(uint32_t a, uint32_t parity) {
     long long t0 = clock64();
@@ -175,15 +179,27 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr, uint32_t sbo)
 __host__ __device__ constexpr uint32_t umma_idesc(uint32_t M, uint32_t N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+// The warp that issues MMAs runs as one: its lanes compute the descriptors together (uniform values, which the issue
+// takes from uniform registers) and `leader`, one lane, issues. (From a branch of one lane each descriptor was moved
+// there first, and that lane's instructions, not the tensor cores, set the pace.)
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
 }
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-                 : "memory");
+__device__ __forceinline__ void umma_f16(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%6, %6, %6, %6}, p;\n\t}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader), "r"(0u));
+}
+__device__ __forceinline__ void umma_commit(uint32_t leader, uint32_t mbar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar),
+        "r"(leader)
+        : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -381,53 +397,50 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
             counts[0] = it;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one();
             // the MMA issuer: a tile's stages into accumulator (tile count % 2), then that accumulator to the epilogue
             // (a layer of one 64-column output tile with at most 32 outputs: the MMAs' N covers the outputs only, 32
             // or 16 of the tile's rows of weights; the epilogue reads no column past the outputs)
             const uint32_t n_mma = a.co_pad == a.nt && a.nt == 64u && a.cout <= 32u ? (a.cout <= 16u ? 16u : 32u) : a.nt;
             const uint32_t idesc = umma_idesc(128u, n_mma);
             uint32_t it = 0, ti = 0;
-            bool ok = !a.resident || mbar_wait(wfull, 0u, a.err, abort_flag);
+            bool ok = !a.resident || mbar_wait_warp(wfull, 0u, a.err, abort_flag);
             for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++ti) {
                 const uint32_t acc = ti & 1u;
-                if (ti >= 2u && !(ok = mbar_wait(acc_empty(acc), ((ti / 2u) - 1u) & 1u, a.err, abort_flag))) break;
+                if (ti >= 2u && !(ok = mbar_wait_warp(acc_empty(acc), ((ti / 2u) - 1u) & 1u, a.err, abort_flag))) break;
                 tc_fence_after();
                 const uint32_t d = tmem + acc * a.nt;
                 for (uint32_t k = 0; k < nk; ++k, ++it) {
                     const uint32_t s = it % NS;
-                    if (!(ok = mbar_wait(full(s), (it / NS) & 1u, a.err, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(full(s), (it / NS) & 1u, a.err, abort_flag))) break;
                     tc_fence_after();
                     if constexpr (HALO) {
                         // tap (dy, dx): 128 rows of 64 bytes from row (dy + 1) x 130 + dx + 1 (the swizzle goes by
                         // the address, so a start inside its 8-row pattern reads what the copy wrote)
+                        const uint64_t ad0 = umma_desc_sw64(sA + s * A_BYTES, 512u);
+                        const uint64_t bd0 = umma_desc_sw64(
+                            a.resident ? sB + k * 9u * a.nt * 64u : sA + s * A_BYTES + HALO_STAGE, 512u);
+                        const uint32_t b_tap = a.nt * 4u;  // a tap's weights, in the descriptors' 16-byte units
+#pragma unroll
                         for (uint32_t tap = 0; tap < 9u; ++tap) {
                             const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
-#pragma unroll
-                            for (uint32_t j = 0; j < 2u; ++j) {
-                                uint64_t ad = umma_desc_sw64(sA + s * A_BYTES + row * 64u + j * 32u, 512u);
-                                const uint32_t wb = a.resident ? sB + (k * 9u + tap) * a.nt * 64u
-                                                               : sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u;
-                                uint64_t bd = umma_desc_sw64(wb + j * 32u, 512u);
-                                umma_f16(d, ad, bd, idesc, (k | tap | j) != 0u ? 1u : 0u);
-                            }
+                            umma_f16(leader, d, ad0 + row * 4u, bd0 + tap * b_tap, idesc, (k | tap) != 0u ? 1u : 0u);
+                            umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
                         }
                     } else {
                         // (resident weights: one box a tap, kc = 1)
-                        const uint32_t sb = a.resident ? sB + k * a.nt * 64u : sB + s * B_STAGE;
-#pragma unroll
-                        for (uint32_t j = 0; j < 2u; ++j) {
-                            uint64_t ad = umma_desc_sw64(sA + s * A_STAGE + j * 32u, 512u);
-                            uint64_t bd = umma_desc_sw64(sb + j * 32u, 512u);
-                            umma_f16(d, ad, bd, idesc, (k | j) != 0u ? 1u : 0u);
-                        }
+                        const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
+                        const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * a.nt * 64u : sB + s * B_STAGE, 512u);
+                        umma_f16(leader, d, ad, bd, idesc, k != 0u ? 1u : 0u);
+                        umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
                     }
-                    umma_commit(empty(s));
+                    umma_commit(leader, empty(s));
                 }
-                if (ok) umma_commit(acc_full(acc));
+                if (ok) umma_commit(leader, acc_full(acc));
             }
-            counts[1] = it;
-            umma_commit(mma_done);  // every MMA issued is done (after a wait that gave up too)
+            if (lane == 0) counts[1] = it;
+            umma_commit(leader, mma_done);  // every MMA issued is done (after a wait that gave up too)
         }
     } else {
         // the epilogue, eight warps, two a tensor-memory lane quarter: warp w reads lanes 32 (w % 4) ... (its rows:
@@ -591,25 +604,26 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ CU
             counts[0] = it;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one();
             // the MMA issuer: eight K-16 steps a stage into the one accumulator
             const uint32_t idesc = umma_idesc(128u, n_cols) | (1u << 15) | (1u << 16);  // A and B MN-major
             uint32_t it = 0;
             for (uint32_t t = k0; t < k1; ++t, ++it) {
                 const uint32_t s = it % a.ts;
-                if (!mbar_wait(full(s), (it / a.ts) & 1u, a.err, abort_flag)) break;
+                if (!mbar_wait_warp(full(s), (it / a.ts) & 1u, a.err, abort_flag)) break;
                 tc_fence_after();
                 const uint32_t base = sbase + s * stage;
 #pragma unroll
                 for (uint32_t j = 0; j < 8u; ++j) {
                     const uint64_t ad = umma_desc_mn64(base + j * 1024u, WG_BOX);
                     const uint64_t bd = umma_desc_mn64(base + 4u * WG_BOX + j * 1024u, WG_BOX);
-                    umma_f16(tmem, ad, bd, idesc, (it | j) != 0u ? 1u : 0u);
+                    umma_f16(leader, tmem, ad, bd, idesc, (it | j) != 0u ? 1u : 0u);
                 }
-                umma_commit(empty(s));
+                umma_commit(leader, empty(s));
             }
-            counts[1] = it;
-            umma_commit(acc_full);  // every MMA issued is done (after a wait that gave up too)
+            if (lane == 0) counts[1] = it;
+            umma_commit(leader, acc_full);  // every MMA issued is done (after a wait that gave up too)
         }
     } else {
         // the epilogue: warp w reads tensor-memory lanes 32 (w % 4) ..., the rows of slot w % 4
