@@ -77,7 +77,7 @@ void launch_pdl(bool early, void (*kernel)(P...), dim3 grid, uint32_t block, uin
 struct Conv {
     uint32_t cin;             // channels read (a multiple of 32)
     uint32_t co_pad;          // a multiple of 64 (up to 256)
-    uint32_t nt;              // output channels a CTA: 128 where they divide co_pad, else 64 (blockIdx.y the tile)
+    uint32_t nt;              // output channels a tile: 32 for at most 32 outputs, else 128 where they divide co_pad, else 64
     const float* bias;        // co_pad, or null
     bf16* y;                  // output, NHWC
     uint32_t y_stride, y_off, cout;
@@ -91,7 +91,8 @@ struct Conv {
     uint32_t resident;        // 1: every tap's weights loaded once a CTA (one 32-channel block, one output tile)
     uint32_t hold;            // 1: CTA 0 withholds its first activation box (trt_unet_hold_next_load: a test of the
                               // bounded waits), so that the stage's wait runs out
-    uint32_t stages;          // the halo variant's stages (HALO_TS with resident weights; 2 or 3 streaming them)
+    uint32_t stages;          // the halo variant's stages
+    uint32_t k_steps;         // K-16 steps a 32-channel block: 2, or 1 where its second 16 channels are zeros
 };
 
 constexpr uint32_t TS = 5;                  // pipeline stages (82 KB of shared memory: two CTAs an SM)
@@ -101,15 +102,13 @@ constexpr uint32_t CONV_SMEM = TS * (A_STAGE + B_STAGE) + 256u + 1024u;  // + ro
 // 32-channel block's 3 rows x 130 pixels, 64 bytes a pixel in the 64-byte swizzle, padded to a multiple of 1 KB.
 constexpr uint32_t HALO_W = 130u, HALO_ROWS = 3u;
 constexpr uint32_t HALO_BYTES = HALO_ROWS * HALO_W * 64u, HALO_STAGE = (HALO_BYTES + 1023u) / 1024u * 1024u;
-constexpr uint32_t HALO_TS = 3u;
-constexpr uint32_t HALO_W_OFF = HALO_TS * HALO_STAGE;                            // the resident weights
+constexpr uint32_t HALO_TS_MAX = 6u, HALO_TS_STREAM = 3u;  // stages at most, with resident and with streamed weights
 constexpr uint32_t SMEM_MAX = 227u * 1024u;                                      // dynamic shared memory a CTA
-// The halo variant's shared memory: the stages, then every (32-channel block, tap) weight box of the output tile
-// (nt rows of 64 bytes each), then the barriers.
+// The halo variant's shared memory: the output tile's resident weights (every (32-channel block, tap) box of nt rows of
+// 64 bytes), the stages, the barriers (with room to align the whole to 1 KB).
 __host__ __device__ constexpr uint32_t halo_weights(uint32_t kc, uint32_t nt) { return 9u * kc * nt * 64u; }
-__host__ __device__ constexpr uint32_t conv_smem_halo(uint32_t kc, uint32_t nt) {
-    return HALO_W_OFF + halo_weights(kc, nt) + 256u + 1024u;
-}
+constexpr uint32_t CONV_SMEM_EXTRA = 256u + 1024u;
+constexpr uint32_t SM_SMEM = 228u * 1024u, CTA_SMEM_KEPT = 1024u;  // an SM's shared memory, and what it keeps a CTA
 constexpr uint32_t CONV_EPI_THREADS = 256u, CONV_THREADS = 64u + CONV_EPI_THREADS;  // loader, MMA, 8 epilogue warps
 constexpr uint32_t CONV_CTAS_PER_SM = 2u;
 
@@ -203,17 +202,16 @@ __device__ __forceinline__ void umma_commit(uint32_t leader, uint32_t mbar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// 64 accumulator columns of this warp's lanes in one load and one wait.
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float* v) {
-    uint32_t r[64];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+// 16 accumulator columns of this warp's lanes.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-
 // 32 accumulator columns of this warp's lanes.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     uint32_t r[32];
@@ -295,10 +293,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     const uint32_t sraw = smem_addr(smem_raw), sbase = (sraw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (sbase - sraw);
     const uint32_t kc = a.cin / 32u, nk = HALO ? kc : 9u * kc;
-    constexpr uint32_t B_OFF = HALO ? HALO_W_OFF : TS * A_STAGE;
-    const uint32_t BAR_OFF = HALO ? (a.resident ? HALO_W_OFF + halo_weights(kc, a.nt) : NS * A_BYTES)
-                                  : TS * (A_STAGE + B_STAGE);
-    const uint32_t sA = sbase, sB = sbase + B_OFF, sBar = sbase + BAR_OFF;
+    const uint32_t A_OFF = HALO && a.resident ? halo_weights(kc, a.nt) : 0u, B_OFF = HALO ? 0u : TS * A_STAGE;
+    const uint32_t BAR_OFF = HALO ? A_OFF + NS * A_BYTES : TS * (A_STAGE + B_STAGE);
+    const uint32_t sA = sbase + A_OFF, sB = sbase + B_OFF, sBar = sbase + BAR_OFF;
     // barriers: full[NS], empty[NS] (the stages), acc_full[2], acc_empty[2] (the accumulators), mma_done (every MMA
     // issued), wfull (the resident weights); the tensor-memory address, the abort word and the counts of stages issued
     // and consumed after them
@@ -310,8 +307,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + BAR_OFF + 8u * (2u * NS + 6u));
     volatile uint32_t* abort_flag = tslot + 1;
     volatile uint32_t* counts = tslot + 2;
-    const uint32_t ncols = 2u * a.nt;  // two accumulators of nt columns: 128 or 256
-    const uint32_t per_img = a.tiles_x * a.tiles_y, n_ntiles = a.co_pad / a.nt;
+    const uint32_t ncols = 2u * a.nt;  // two accumulators of nt columns: 64, 128 or 256
+    const uint32_t per_img = a.tiles_x * a.tiles_y, n_ntiles = (a.cout + a.nt - 1u) / a.nt;
     const uint32_t tiles = a.B * per_img * n_ntiles;
     pdl_trigger();
 
@@ -400,9 +397,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
         {
             const uint32_t leader = elect_one();
             // the MMA issuer: a tile's stages into accumulator (tile count % 2), then that accumulator to the epilogue
-            // (a layer of one 64-column output tile with at most 32 outputs: the MMAs' N covers the outputs only, 32
-            // or 16 of the tile's rows of weights; the epilogue reads no column past the outputs)
-            const uint32_t n_mma = a.co_pad == a.nt && a.nt == 64u && a.cout <= 32u ? (a.cout <= 16u ? 16u : 32u) : a.nt;
+            // (at most 16 outputs: the MMAs' N covers 16 of the tile's rows of weights; the epilogue reads no column
+            // past the outputs)
+            const uint32_t n_mma = a.cout <= 16u ? 16u : a.nt;
             const uint32_t idesc = umma_idesc(128u, n_mma);
             uint32_t it = 0, ti = 0;
             bool ok = !a.resident || mbar_wait_warp(wfull, 0u, a.err, abort_flag);
@@ -426,14 +423,15 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                         for (uint32_t tap = 0; tap < 9u; ++tap) {
                             const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
                             umma_f16(leader, d, ad0 + row * 4u, bd0 + tap * b_tap, idesc, (k | tap) != 0u ? 1u : 0u);
-                            umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
+                            if (a.k_steps == 2u)
+                                umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
                         }
                     } else {
                         // (resident weights: one box a tap, kc = 1)
                         const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
                         const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * a.nt * 64u : sB + s * B_STAGE, 512u);
                         umma_f16(leader, d, ad, bd, idesc, k != 0u ? 1u : 0u);
-                        umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
+                        if (a.k_steps == 2u) umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
                     }
                     umma_commit(leader, empty(s));
                 }
@@ -460,7 +458,13 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
             const int px = x0 + (int)(m % a.bw), py = y0 + (int)(m / a.bw);
             const bool valid = fin && px < (int)a.W && py < (int)a.H;
             const uint64_t p = ((uint64_t)b * a.H + (uint32_t)py) * a.W + (uint32_t)px;
-            for (uint32_t cc = c_first; cc < c_first + cols; cc += 32u) {
+            if (cols == 16u) {
+                if (n0 + c_first < a.cout) {
+                    float v[16];
+                    tmem_ld16(tmem + ((quarter * 32u) << 16) + acc * a.nt + c_first, v);
+                    if (valid) conv_store16(a, p, n0 + c_first, v);
+                }
+            } else for (uint32_t cc = c_first; cc < c_first + cols; cc += 32u) {
                 if (n0 + cc >= a.cout) break;  // (columns past the layer's outputs: padding, not stored)
                 float v[32];
                 tmem_ld32(tmem + ((quarter * 32u) << 16) + acc * a.nt + cc, v);
@@ -1105,13 +1109,14 @@ bool act_map(Net* n, CUtensorMap* m, const bf16* p, uint32_t stride, uint32_t B,
 // w [9][co_pad][cin] (each tap's output channels, their input channels contiguous).
 void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t cin, const bf16* w, uint32_t co_pad,
               const float* bias, bf16* y, uint32_t y_stride, uint32_t y_off, uint32_t cout, float* yf, uint32_t B,
-              uint32_t H, uint32_t W, int relu, const Act* mask = nullptr) {
+              uint32_t H, uint32_t W, int relu, const Act* mask = nullptr, uint32_t k_steps = 2u) {
     uint32_t bw, bh, tiles_x, tiles_y;
     tile_shape(W, H, bw, bh, tiles_x, tiles_y);
-    const uint32_t nt = co_pad % 128u == 0u ? 128u : 64u;  // co_pad: a multiple of 64
+    // (co_pad: a multiple of 64; a layer of at most 32 outputs takes 32 of its 64 rows of weights)
+    const uint32_t nt = cout <= 32u ? 32u : co_pad % 128u == 0u ? 128u : 64u, n_ntiles = (cout + nt - 1u) / nt;
     // the nine taps' weights stay in the weight stages' room (9 x nt x 64 bytes <= TS x B_STAGE) where the layer
     // reads one 32-channel block into one output tile
-    uint32_t resident = cin == 32u && co_pad == nt && 9u * nt * 64u <= TS * B_STAGE ? 1u : 0u;
+    uint32_t resident = cin == 32u && n_ntiles == 1u && 9u * nt * 64u <= TS * B_STAGE ? 1u : 0u;
     // A layer of one output tile whose weights fit in shared memory beside three halo stages (up to four 32-channel
     // blocks at 64 outputs, two at 128), on an image at least 128 wide, reads its activations once a tile with the
     // halo: row tiles of 128 pixels (the last of a row ragged), boxes of 32 channels x 130 x 3, the weights resident.
@@ -1119,16 +1124,23 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     // 320 x 180 the row tiles measured 24.2 against 20.8 us.)
     const uint32_t kc = cin / 32u, row_tiles = (W + 127u) / 128u;
     const bool rows_ok = cin % 32u == 0u && W >= 128u && row_tiles * 128u - W <= row_tiles * 16u && (x_off % 8u) == 0u;
-    const bool halo_res = rows_ok && co_pad == nt && conv_smem_halo(kc, nt) <= SMEM_MAX;
+    // Two CTAs an SM where each then holds its weights and at least two stages, else one, with as many stages as fit.
+    auto fit = [&](uint32_t ctas, uint32_t fixed, uint32_t stage, uint32_t most) {
+        const uint32_t room = std::min(SMEM_MAX, SM_SMEM / ctas - CTA_SMEM_KEPT), used = fixed + CONV_SMEM_EXTRA;
+        return used >= room ? 0u : std::min(most, (room - used) / stage);
+    };
+    const uint32_t w_res = halo_weights(kc, nt), w_stream = HALO_STAGE + 9u * nt * 64u;
+    const uint32_t two = fit(2u, w_res, HALO_STAGE, HALO_TS_MAX), one = fit(1u, w_res, HALO_STAGE, HALO_TS_MAX);
+    const bool halo_res = rows_ok && n_ntiles == 1u && one >= 3u;
     // Other layers on such levels stream each stage's nine weight boxes beside its activations, one CTA an SM: as
     // many stages (up to three) as fit.
-    const uint32_t stream_stage = HALO_STAGE + 9u * nt * 64u;
-    const uint32_t stream_ns = std::min(HALO_TS, (SMEM_MAX - 1280u) / stream_stage);
+    const uint32_t stream_ns = fit(1u, 0u, w_stream, HALO_TS_STREAM);
     const bool halo = halo_res || (rows_ok && stream_ns >= 2u);
-    const uint32_t stages = halo_res ? HALO_TS : stream_ns;
-    const uint32_t smem = halo_res ? conv_smem_halo(kc, nt) : halo ? stages * stream_stage + 1280u : CONV_SMEM;
-    // two CTAs an SM where their shared memory fits (228 KB an SM, 1 KB of it kept a CTA), else one
-    const uint32_t per_sm = 2u * (smem + 1024u) <= 228u * 1024u ? CONV_CTAS_PER_SM : 1u;
+    const uint32_t stages = halo_res ? (two >= 2u ? two : one) : stream_ns;
+    const uint32_t smem = halo_res ? w_res + stages * HALO_STAGE + CONV_SMEM_EXTRA
+                          : halo   ? stages * w_stream + CONV_SMEM_EXTRA
+                                   : CONV_SMEM;
+    const uint32_t per_sm = halo && !(halo_res && two >= 2u) ? 1u : CONV_CTAS_PER_SM;
     if (halo) {
         resident = halo_res ? 1u : 0u;
         bw = 128u;
@@ -1151,9 +1163,9 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
         return;
     }
     Conv a{cin, co_pad, nt, bias, y, y_stride, y_off, cout, yf, B, H, W, x_off, bw, bh, tiles_x, tiles_y, relu,
-           mask ? mask->p : nullptr, mask ? mask->stride : 0u, n->dev_err, resident, n->hold_next ? 1u : 0u, stages};
+           mask ? mask->p : nullptr, mask ? mask->stride : 0u, n->dev_err, resident, n->hold_next ? 1u : 0u, stages, k_steps};
     n->hold_next = false;
-    const uint32_t tiles = B * tiles_x * tiles_y * (co_pad / nt);
+    const uint32_t tiles = B * tiles_x * tiles_y * n_ntiles;
     const uint32_t grid = std::min<uint32_t>(tiles, n->sms * per_sm);
     launch_pdl(n->early, halo ? k_conv<true> : k_conv<false>, grid, CONV_THREADS, smem, n->stream, xmap, wmap, a);
 }
@@ -1162,7 +1174,7 @@ void conv(Net* n, int li, const Act& x, uint32_t x_off, const Act& y, uint32_t y
           float* yf = nullptr) {
     const Layer& L = LAYERS[li];
     conv_run(n, x.p, x.stride, x_off, L.cin, n->wf[li], r64(L.cout), n->w + n->off[li] + w_count(L), y.p, y.stride,
-             y_off, L.cout, yf, B, H, W, L.relu);
+             y_off, L.cout, yf, B, H, W, L.relu, nullptr, li == E0A ? 1u : 2u);  // (the input: N_FEAT of 32 channels)
 }
 // The input gradient of layer li: dx (channels [0, cin_logical)) from dy (cout rounded to 32 channels); mask: the layer's
 // input where that is a ReLU's output, whose gradient it then is.
