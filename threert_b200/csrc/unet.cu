@@ -92,7 +92,6 @@ struct Conv {
     uint32_t hold;            // 1: CTA 0 withholds its first activation box (trt_unet_hold_next_load: a test of the
                               // bounded waits), so that the stage's wait runs out
     uint32_t stages;          // the halo variant's stages
-    uint32_t k_steps;         // K-16 steps a 32-channel block: 2, or 1 where its second 16 channels are zeros
 };
 
 constexpr uint32_t TS = 5;                  // pipeline stages (82 KB of shared memory: two CTAs an SM)
@@ -112,11 +111,23 @@ constexpr uint32_t SM_SMEM = 228u * 1024u, CTA_SMEM_KEPT = 1024u;  // an SM's sh
 constexpr uint32_t CONV_EPI_THREADS = 256u, CONV_THREADS = 64u + CONV_EPI_THREADS;  // loader, MMA, 8 epilogue warps
 constexpr uint32_t CONV_CTAS_PER_SM = 2u;
 
+// The warps that issue copies and MMAs run as one: their lanes compute the operands together (uniform values, which the
+// issue takes from uniform registers) and `leader`, one lane, issues. (From a branch of one lane each operand was moved
+// there first, and that lane's instructions, not the tensor cores, set the pace: the 720p forward 754 -> 697 us with the
+// MMAs issued so.)
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
+}
 __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
+__device__ __forceinline__ void mbar_expect_tx(uint32_t leader, uint32_t a, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}\n" ::"r"(a),
+        "r"(bytes), "r"(leader)
+        : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t a, uint32_t parity) {
     uint32_t ok;
@@ -152,19 +163,22 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t a, uint32_t parity) {
         if (clock64() - t0 > (1ll << 31)) return false;
     return true;
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int c0, int c1, int c2, int c3,
+__device__ __forceinline__ void tma_load_4d(uint32_t leader, uint32_t dst, const void* map, int c0, int c1, int c2, int c3,
                                             uint32_t mbar) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(mbar)
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];\n\t}\n" ::"r"(dst),
+        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(mbar), "r"(leader)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int c0, int c1, int c2, uint32_t mbar) {
+__device__ __forceinline__ void tma_load_3d(uint32_t leader, uint32_t dst, const void* map, int c0, int c1, int c2,
+                                            uint32_t mbar) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(mbar)
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];\n\t}\n" ::"r"(dst),
+        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(mbar), "r"(leader)
         : "memory");
 }
 // The canonical K-major shared-memory matrix with the 64-byte swizzle: rows of 64 bytes (32 bf16 of K), atoms of 8
@@ -177,14 +191,6 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr, uint32_t sbo)
 // kind::f16 instruction descriptor: f32 accumulator, bf16 A and B, both K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc(uint32_t M, uint32_t N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-// The warp that issues MMAs runs as one: its lanes compute the descriptors together (uniform values, which the issue
-// takes from uniform registers) and `leader`, one lane, issues. (From a branch of one lane each descriptor was moved
-// there first, and that lane's instructions, not the tensor cores, set the pace.)
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
-    return e;
 }
 __device__ __forceinline__ void umma_f16(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -281,7 +287,7 @@ __device__ __forceinline__ void conv_store16(const Conv& a, uint64_t p, uint32_t
 // The box's rows bound the loads: as four boxes of 8 channels without swizzle, a pixel was four requests of 16 bytes,
 // half of each 32-byte sector fetched; as one of 64 bytes the 1280 x 720 forward went from 957 to 843 us (1920 x 1080,
 // two images: 3,740 -> 3,105), the same bits.
-template <bool HALO>
+template <bool HALO, bool HALF_K = false>
 __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant__ CUtensorMap xmap,
                                                        const __grid_constant__ CUtensorMap wmap, Conv a) {
     // stages, and a stage's bytes: the halo variant's activations, and where the weights are not resident the nine
@@ -349,16 +355,17 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one();
             // the loader: the resident weights (the nine taps' boxes, one after another), then the stages of every tile
             // of this CTA, in order
             // (halo: every 32-channel block's nine boxes, block-major)
             if (a.resident) {
                 const uint32_t blocks = HALO ? kc : 1u;
-                mbar_expect_tx(wfull, 9u * blocks * a.nt * 64u);
+                mbar_expect_tx(leader, wfull, 9u * blocks * a.nt * 64u);
                 for (uint32_t k = 0; k < blocks; ++k)
                     for (uint32_t tap = 0; tap < 9u; ++tap)
-                        tma_load_3d(sB + (k * 9u + tap) * a.nt * 64u, &wmap, (int)(k * 32u), 0, (int)tap, wfull);
+                        tma_load_3d(leader, sB + (k * 9u + tap) * a.nt * 64u, &wmap, (int)(k * 32u), 0, (int)tap, wfull);
             }
             pdl_wait();
             uint32_t it = 0;
@@ -369,29 +376,29 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                 tile_of(t, b, x0, y0, n0);
                 for (uint32_t k = 0; k < nk; ++k, ++it) {
                     const uint32_t s = it % NS;
-                    if (it >= NS && !(ok = mbar_wait(empty(s), ((it / NS) - 1u) & 1u, a.err, abort_flag))) break;
+                    if (it >= NS && !(ok = mbar_wait_warp(empty(s), ((it / NS) - 1u) & 1u, a.err, abort_flag))) break;
                     const bool withhold = a.hold && blockIdx.x == 0 && it == 0;
                     if constexpr (HALO) {
                         // the tile's rows y0 - 1 .. y0 + 1, pixels x0 - 1 .. x0 + 128
-                        mbar_expect_tx(full(s), HALO_BYTES + (a.resident ? 0u : 9u * a.nt * 64u));
+                        mbar_expect_tx(leader, full(s), HALO_BYTES + (a.resident ? 0u : 9u * a.nt * 64u));
                         if (!withhold)
-                            tma_load_4d(sA + s * A_BYTES, &xmap, (int)(a.x_off + k * 32u), x0 - 1, y0 - 1, (int)b,
+                            tma_load_4d(leader, sA + s * A_BYTES, &xmap, (int)(a.x_off + k * 32u), x0 - 1, y0 - 1, (int)b,
                                         full(s));
                         if (!a.resident)
                             for (uint32_t tap = 0; tap < 9u; ++tap)
-                                tma_load_3d(sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
+                                tma_load_3d(leader, sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
                                             (int)n0, (int)tap, full(s));
                     } else {
-                        mbar_expect_tx(full(s), A_STAGE + (a.resident ? 0u : a.nt * 64u));
+                        mbar_expect_tx(leader, full(s), A_STAGE + (a.resident ? 0u : a.nt * 64u));
                         const uint32_t tap = k / kc, c0 = (k % kc) * 32u;
                         const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
                         if (!withhold)
-                            tma_load_4d(sA + s * A_STAGE, &xmap, (int)(a.x_off + c0), x0 + dx, y0 + dy, (int)b, full(s));
-                        if (!a.resident) tma_load_3d(sB + s * B_STAGE, &wmap, (int)c0, (int)n0, (int)tap, full(s));
+                            tma_load_4d(leader, sA + s * A_STAGE, &xmap, (int)(a.x_off + c0), x0 + dx, y0 + dy, (int)b, full(s));
+                        if (!a.resident) tma_load_3d(leader, sB + s * B_STAGE, &wmap, (int)c0, (int)n0, (int)tap, full(s));
                     }
                 }
             }
-            counts[0] = it;
+            if (lane == 0) counts[0] = it;
         }
     } else if (warp == 1) {
         {
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                         for (uint32_t tap = 0; tap < 9u; ++tap) {
                             const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
                             umma_f16(leader, d, ad0 + row * 4u, bd0 + tap * b_tap, idesc, (k | tap) != 0u ? 1u : 0u);
-                            if (a.k_steps == 2u)
+                            if (!HALF_K)
                                 umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
                         }
                     } else {
@@ -431,7 +438,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                         const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
                         const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * a.nt * 64u : sB + s * B_STAGE, 512u);
                         umma_f16(leader, d, ad, bd, idesc, k != 0u ? 1u : 0u);
-                        if (a.k_steps == 2u) umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
+                        if (!HALF_K) umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
                     }
                     umma_commit(leader, empty(s));
                 }
@@ -587,25 +594,26 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ CU
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one();
             // the loader: a stage a tile
             uint32_t it = 0;
             for (uint32_t t = k0; t < k1; ++t, ++it) {
                 const uint32_t s = it % a.ts;
-                if (it >= a.ts && !mbar_wait(empty(s), ((it / a.ts) - 1u) & 1u, a.err, abort_flag)) break;
-                mbar_expect_tx(full(s), (loaded + a.nb) * WG_BOX);
+                if (it >= a.ts && !mbar_wait_warp(empty(s), ((it / a.ts) - 1u) & 1u, a.err, abort_flag)) break;
+                mbar_expect_tx(leader, full(s), (loaded + a.nb) * WG_BOX);
                 const uint32_t b = t / per_img, r = t % per_img;
                 const int x0 = (int)((r % a.tiles_x) * a.bw), y0 = (int)((r / a.tiles_x) * a.bh);
                 const uint32_t base = sbase + s * stage;
                 for (uint32_t j = 0; j < loaded; ++j) {
                     const uint32_t pr = slot0 + j, tap = pr / a.kc, cb = pr % a.kc;
-                    tma_load_4d(base + j * WG_BOX, &xmap, (int)(a.x_off + cb * 32u), x0 + (int)(tap % 3u) - 1,
+                    tma_load_4d(leader, base + j * WG_BOX, &xmap, (int)(a.x_off + cb * 32u), x0 + (int)(tap % 3u) - 1,
                                 y0 + (int)(tap / 3u) - 1, (int)b, full(s));
                 }
                 for (uint32_t i = 0; i < a.nb; ++i)
-                    tma_load_4d(base + (4u + i) * WG_BOX, &dymap, (int)(i * 32u), x0, y0, (int)b, full(s));
+                    tma_load_4d(leader, base + (4u + i) * WG_BOX, &dymap, (int)(i * 32u), x0, y0, (int)b, full(s));
             }
-            counts[0] = it;
+            if (lane == 0) counts[0] = it;
         }
     } else if (warp == 1) {
         {
@@ -1109,7 +1117,7 @@ bool act_map(Net* n, CUtensorMap* m, const bf16* p, uint32_t stride, uint32_t B,
 // w [9][co_pad][cin] (each tap's output channels, their input channels contiguous).
 void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t cin, const bf16* w, uint32_t co_pad,
               const float* bias, bf16* y, uint32_t y_stride, uint32_t y_off, uint32_t cout, float* yf, uint32_t B,
-              uint32_t H, uint32_t W, int relu, const Act* mask = nullptr, uint32_t k_steps = 2u) {
+              uint32_t H, uint32_t W, int relu, const Act* mask = nullptr, bool half_k = false) {
     uint32_t bw, bh, tiles_x, tiles_y;
     tile_shape(W, H, bw, bh, tiles_x, tiles_y);
     // (co_pad: a multiple of 64; a layer of at most 32 outputs takes 32 of its 64 rows of weights)
@@ -1163,18 +1171,18 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
         return;
     }
     Conv a{cin, co_pad, nt, bias, y, y_stride, y_off, cout, yf, B, H, W, x_off, bw, bh, tiles_x, tiles_y, relu,
-           mask ? mask->p : nullptr, mask ? mask->stride : 0u, n->dev_err, resident, n->hold_next ? 1u : 0u, stages, k_steps};
+           mask ? mask->p : nullptr, mask ? mask->stride : 0u, n->dev_err, resident, n->hold_next ? 1u : 0u, stages};
     n->hold_next = false;
     const uint32_t tiles = B * tiles_x * tiles_y * n_ntiles;
     const uint32_t grid = std::min<uint32_t>(tiles, n->sms * per_sm);
-    launch_pdl(n->early, halo ? k_conv<true> : k_conv<false>, grid, CONV_THREADS, smem, n->stream, xmap, wmap, a);
+    launch_pdl(n->early, halo ? (half_k ? k_conv<true, true> : k_conv<true>) : half_k ? k_conv<false, true> : k_conv<false>, grid, CONV_THREADS, smem, n->stream, xmap, wmap, a);
 }
 
 void conv(Net* n, int li, const Act& x, uint32_t x_off, const Act& y, uint32_t y_off, uint32_t B, uint32_t H, uint32_t W,
           float* yf = nullptr) {
     const Layer& L = LAYERS[li];
     conv_run(n, x.p, x.stride, x_off, L.cin, n->wf[li], r64(L.cout), n->w + n->off[li] + w_count(L), y.p, y.stride,
-             y_off, L.cout, yf, B, H, W, L.relu, nullptr, li == E0A ? 1u : 2u);  // (the input: N_FEAT of 32 channels)
+             y_off, L.cout, yf, B, H, W, L.relu, nullptr, li == E0A);  // (the input: N_FEAT of 32 channels)
 }
 // The input gradient of layer li: dx (channels [0, cin_logical)) from dy (cout rounded to 32 channels); mask: the layer's
 // input where that is a ReLU's output, whose gradient it then is.
@@ -1468,7 +1476,11 @@ int trt_unet_create(int device, uint32_t max_batch, uint32_t max_h, uint32_t max
     if (e == cudaSuccess) e = alloc(n, &n->partial, 3 * FEAT_BLOCKS);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_conv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_conv<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_conv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_conv<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM_MAX);
     if (e == cudaSuccess) {
