@@ -113,7 +113,7 @@ class Scene:
     def trace(self, params: np.ndarray, rays: np.ndarray, flags: int = 0) -> np.ndarray:
         L = N.lib()
         rays = np.ascontiguousarray(rays, dtype=RAY_DTYPE)
-        hits = np.zeros(len(rays), HIT_DTYPE)
+        hits = np.empty(len(rays), HIT_DTYPE)
         p = np.ascontiguousarray(params, dtype=np.uint32)
         rc = L.trt_trace(self.handle, p.ctypes.data_as(C.POINTER(C.c_uint32)),
                          rays.ctypes.data_as(C.POINTER(N.Ray)), len(rays), flags,
@@ -238,8 +238,8 @@ class Gpu:
 
     def bake_sky(self, atmosphere: N.Atmosphere, tables: bool = False):
         """trt_sky_bake: (texels (height, width, 4) float32, SkyResult[, the tables as TRT_SKY_TABLE_FLOATS floats])."""
-        tex = np.zeros((atmosphere.height, atmosphere.width, 4), np.float32)
-        tab = np.zeros(N.SKY_TABLE_FLOATS, np.float32) if tables else None
+        tex = np.empty((atmosphere.height, atmosphere.width, 4), np.float32)
+        tab = np.empty(N.SKY_TABLE_FLOATS, np.float32) if tables else None
         r = N.SkyResult()
         self._check(N.lib().trt_sky_bake(self.ctx, C.byref(atmosphere), tex.ctypes.data_as(C.POINTER(C.c_float)),
                                          tab.ctypes.data_as(C.POINTER(C.c_float)) if tables else None, C.byref(r)),
@@ -268,7 +268,7 @@ class Gpu:
         """trt_math_eval: the device's cosf / sinf / acosf / atan2f (N.TRT_MATH_*) over float32 arrays."""
         x = np.ascontiguousarray(x, np.float32)
         yy = None if y is None else np.ascontiguousarray(y, np.float32)
-        out = np.zeros_like(x)
+        out = np.empty_like(x)
         fp = lambda a: a.ctypes.data_as(C.POINTER(C.c_float)) if a is not None else None
         self._check(N.lib().trt_math_eval(self.ctx, fn, fp(x), fp(yy), x.size, fp(out)), "trt_math_eval")
         return out

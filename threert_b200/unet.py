@@ -94,14 +94,14 @@ class UNet:
         self._check(N.lib().trt_unet_set_params(self.handle, p.ctypes.data_as(C.POINTER(C.c_float))), "set_params")
 
     def params(self) -> np.ndarray:
-        p = np.zeros(param_count(), np.float32)
+        p = np.empty(param_count(), np.float32)
         self._check(N.lib().trt_unet_get_params(self.handle, p.ctypes.data_as(C.POINTER(C.c_float))), "get_params")
         return p
 
     def forward(self, feats: np.ndarray) -> tuple[np.ndarray, float]:
         f = np.ascontiguousarray(feats, np.float32)
         b, h, w, _ = f.shape
-        out = np.zeros((b, h, w, 3), np.float32)
+        out = np.empty((b, h, w, 3), np.float32)
         ms = C.c_float()
         self._check(N.lib().trt_unet_forward(self.handle, f.ctypes.data_as(C.POINTER(C.c_float)), b, h, w,
                                              out.ctypes.data_as(C.POINTER(C.c_float)), C.byref(ms)), "forward")
@@ -114,7 +114,7 @@ class UNet:
         b, h, w, _ = f.shape
         loss = C.c_float()
         ms = C.c_float()
-        g = np.zeros(param_count(), np.float32) if grads else None
+        g = np.empty(param_count(), np.float32) if grads else None
         self._check(N.lib().trt_unet_train_step(self.handle, f.ctypes.data_as(C.POINTER(C.c_float)),
                                                 t.ctypes.data_as(C.POINTER(C.c_float)), b, h, w, lr,
                                                 1 if update else 0, C.byref(loss),
@@ -132,7 +132,7 @@ class UNet:
         ptr, nbytes = C.c_void_p(), C.c_uint64()
         scene.gpu._check(N.lib().trt_accum_device_ptr(scene.handle, C.byref(ptr), C.byref(nbytes)), "accum")
         w, h = scene.last_size
-        out = np.zeros((h, w, 3), np.float32)
+        out = np.empty((h, w, 3), np.float32)
         ms = C.c_float()
         self._check(N.lib().trt_unet_denoise_accum(self.handle, ptr, w, h, out.ctypes.data_as(C.POINTER(C.c_float)),
                                                    C.byref(ms)), "denoise")
