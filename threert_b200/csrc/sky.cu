@@ -124,20 +124,71 @@ __device__ D3 optical_depth(const Atm& a, double r, double mu) {
     return {fmin(e.x + ground, OPAQUE), fmin(e.y + ground, OPAQUE), fmin(e.z + ground, OPAQUE)};
 }
 
-// sky.rs:203-220 Atmosphere::sun_transmittance, times the sun's illuminance and the clouds' share (sky.rs:694-703).
-__device__ float3 sun_illuminance(const Atm& a, float3 dir, float3 lux, float cover) {
+// optical_depth by a block of at least COLUMN_NODES threads: a node of the quadrature a thread, their terms summed by
+// thread 0 in columns_exact's order, so that it rounds the same. `sh`: COLUMN_NODES entries of shared memory. Valid on
+// thread 0. (One thread's 96 or 192 nodes in double precision, one after another, took 34 us.)
+constexpr int COLUMN_PANELS = 12, COLUMN_NODES = COLUMN_PANELS * 8;
+__device__ D3 block_columns(double r, double mu, D3* sh) {
+    const int i = (int)threadIdx.x;
+    if (i < COLUMN_NODES) {
+        const int p = i / 8, g = (i / 2) % 4;
+        const double d = distance_out(r, mu, R_TOP);
+        const double centre = ((double)p + 0.5) / (double)COLUMN_PANELS, half = 0.5 / (double)COLUMN_PANELS;
+        const double s = i % 2 == 0 ? -1.0 : 1.0;
+        const double u = centre + s * half * GL8_X[g];
+        const double t = d * u * u;
+        const D3 dens = densities(sqrt(r * r + t * t + 2.0 * r * mu * t) - R_GROUND);
+        const double k = GL8_W[g] * half * 2.0 * d * u;
+        sh[i] = {k * dens.x, k * dens.y, k * dens.z};
+    }
+    __syncthreads();
+    D3 n = {0, 0, 0};
+    if (i == 0) {
+#pragma unroll 8
+        for (int j = 0; j < COLUMN_NODES; ++j) {
+            n.x += sh[j].x;
+            n.y += sh[j].y;
+            n.z += sh[j].z;
+        }
+    }
+    __syncthreads();
+    return n;
+}
+__device__ D3 block_optical_depth(const Atm& a, double r, double mu, D3* sh) {
+    D3 n;
+    double ground = 0.0;
+    if (mu >= 0.0) {
+        n = block_columns(r, mu, sh);
+    } else {
+        double p = r * sqrt(fmax(1.0 - mu * mu, 0.0));
+        if (p <= R_BASE) return {OPAQUE, OPAQUE, OPAQUE};
+        D3 level = block_columns(p, 0.0, sh), mirror = block_columns(r, -mu, sh);
+        n = {fmax(2.0 * level.x - mirror.x, 0.0), fmax(2.0 * level.y - mirror.y, 0.0),
+             fmax(2.0 * level.z - mirror.z, 0.0)};
+        double dd = fmax((R_GROUND - p) / 2.0, 0.0);
+        ground = dd * dd * dd * dd;
+    }
+    D3 e = extinction(a, n.x, n.y, n.z);
+    return {fmin(e.x + ground, OPAQUE), fmin(e.y + ground, OPAQUE), fmin(e.z + ground, OPAQUE)};
+}
+
+// sky.rs:203-220 Atmosphere::sun_transmittance (a block's; valid on thread 0).
+__device__ float3 block_sun_transmittance(const Atm& a, float3 dir, D3* sh) {
     float len = sqrtf(dir.x * dir.x + dir.y * dir.y + dir.z * dir.z);
     float rcp = 1.0f / len;
     float y = (isfinite(rcp) && rcp > 0.0f) ? dir.y * rcp : 0.0f;
     double mu = fmin(fmax((double)y, -1.0), 1.0);
-    D3 od = optical_depth(a, R_GROUND, mu);
+    D3 od = block_optical_depth(a, R_GROUND, mu, sh);
     double level = R_GROUND / (R_GROUND + SUN_VEIL_ALTITUDE);
     double veil = SUN_VEIL_COLUMN / sqrt(1.0 - level * level * (1.0 - mu * mu));
-    float t0 = (float)(exp(-od.x) * exp(-veil * (a.rayleigh[0] + a.mie_extinction)));
-    float t1 = (float)(exp(-od.y) * exp(-veil * (a.rayleigh[1] + a.mie_extinction)));
-    float t2 = (float)(exp(-od.z) * exp(-veil * (a.rayleigh[2] + a.mie_extinction)));
+    return make_float3((float)(exp(-od.x) * exp(-veil * (a.rayleigh[0] + a.mie_extinction))),
+                       (float)(exp(-od.y) * exp(-veil * (a.rayleigh[1] + a.mie_extinction))),
+                       (float)(exp(-od.z) * exp(-veil * (a.rayleigh[2] + a.mie_extinction))));
+}
+// ... times the sun's illuminance and the clouds' share (sky.rs:694-703).
+__device__ __forceinline__ float3 sun_illuminance(float3 t, float3 lux, float cover) {
     float cloud = 1.0f - fminf(fmaxf(cover, 0.0f), 1.0f);
-    return make_float3(lux.x * t0 * cloud, lux.y * t1 * cloud, lux.z * t2 * cloud);
+    return make_float3(lux.x * t.x * cloud, lux.y * t.y * cloud, lux.z * t.z * cloud);
 }
 
 // sky.rs:248-284: where a point is in the tables.
@@ -452,7 +503,10 @@ __device__ __forceinline__ float3 fnormalize(float3 v) {
 }
 
 // sky.rs:730-772: a texel of the bake (before the overcast blend): radiance x the sun's illuminance + glow, times
-// the horizon's cover k, k in w.
+// the horizon's cover k; in w k where a cloud cover's blend follows, else the texel's alpha (the planet's limb share, or
+// 1).
+__device__ __forceinline__ float texel_alpha(const Bake& b, float k) { return (b.planet && k > 0.0f) ? k : 1.0f; }
+__device__ __forceinline__ float bake_w(const Bake& b, float k) { return b.cover > 0.0f ? k : texel_alpha(b, k); }
 __global__ void k_bake(Atm a, Bake b, const float* __restrict__ sun, const float* __restrict__ scattered,
                        const float* __restrict__ ground, float4* __restrict__ tex) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -467,7 +521,7 @@ __global__ void k_bake(Atm a, Bake b, const float* __restrict__ sun, const float
     if (b.planet) {
         float k = fminf(fmaxf((PI_F / 2.0f - theta + 0.5f * b.row - b.dip) / b.row, 0.0f), 1.0f);
         if (k <= 0.0f) {
-            tex[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            tex[i] = make_float4(0.0f, 0.0f, 0.0f, bake_w(b, 0.0f));
             return;
         }
         float e = fmaxf(PI_F / 2.0f - theta, b.dip + 1e-4f);
@@ -475,12 +529,12 @@ __global__ void k_bake(Atm a, Bake b, const float* __restrict__ sun, const float
         float3 dir = make_float3(sp * ce + 0.0f * se, 0.0f * ce + 1.0f * se, -cp * ce + 0.0f * se);
         float3 l = sky_radiance(a, sun, scattered, ground, b.altitude_km, make_float3(dir.x, dir.z, dir.y), b.sun_p);
         float3 g = glow_at(b, e);
-        out = make_float4((l.x * b.sun_lux.x + g.x) * k, (l.y * b.sun_lux.y + g.y) * k, (l.z * b.sun_lux.z + g.z) * k, k);
+        out = make_float4((l.x * b.sun_lux.x + g.x) * k, (l.y * b.sun_lux.y + g.y) * k, (l.z * b.sun_lux.z + g.z) * k, bake_w(b, k));
     } else {
         float side = fmaxf(fmaxf(fabsf(d.x), fabsf(d.z)), 1e-6f);
         float r = d.y / side * (0.5f * SKY_LIGHT_CUBE);
         if (r <= -0.5f) {
-            tex[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            tex[i] = make_float4(0.0f, 0.0f, 0.0f, bake_w(b, 0.0f));
             return;
         }
         float3 dir = d;
@@ -491,7 +545,7 @@ __global__ void k_bake(Atm a, Bake b, const float* __restrict__ sun, const float
         }
         float3 l = sky_radiance(a, sun, scattered, ground, b.altitude_km, make_float3(dir.x, dir.z, dir.y), b.sun_p);
         float3 g = glow_at(b, asinf(fminf(fmaxf(dir.y, -1.0f), 1.0f)));
-        out = make_float4((l.x * b.sun_lux.x + g.x) * k, (l.y * b.sun_lux.y + g.y) * k, (l.z * b.sun_lux.z + g.z) * k, k);
+        out = make_float4((l.x * b.sun_lux.x + g.x) * k, (l.y * b.sun_lux.y + g.y) * k, (l.z * b.sun_lux.z + g.z) * k, bake_w(b, k));
     }
     tex[i] = out;
 }
@@ -533,17 +587,21 @@ struct Result {
 };
 
 // sky.rs:783-796 and 802-817: the overcast dome's illuminance (from the block sums), the sun's illuminance at the
-// ground, the planet's limb row. One thread.
-__global__ void k_finish(Atm a, Bake b, const double* __restrict__ partial, int n_partial, Result* __restrict__ res) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// ground, the planet's limb row. One block of FINISH_THREADS.
+constexpr int FINISH_THREADS = 128;
+__global__ void __launch_bounds__(FINISH_THREADS) k_finish(Atm a, Bake b, const double* __restrict__ partial,
+                                                           int n_partial, Result* __restrict__ res) {
+    __shared__ D3 sh[COLUMN_NODES];
     float cover = fminf(fmaxf(b.cover, 0.0f), 1.0f);
+    const float3 sun_t = block_sun_transmittance(a, b.sun_dir, sh);
+    if (threadIdx.x != 0) return;
     if (cover > 0.0f) {
         double es[3] = {0, 0, 0};
         for (int p = 0; p < n_partial; ++p)
             for (int c = 0; c < 3; ++c) es[c] += partial[3 * p + c];
         float dt = PI_F / (float)b.height, dp = 2.0f * PI_F / (float)b.width;
         float3 sd = fnormalize(b.sun_dir);
-        float3 s0 = sun_illuminance(a, b.sun_dir, b.sun_lux, 0.0f);
+        float3 s0 = sun_illuminance(sun_t, b.sun_lux, 0.0f);
         float up = fmaxf(sd.y, 0.0f);
         float3 e_sun = make_float3(s0.x * up, s0.y * up, s0.z * up);
         float3 e_glow = make_float3(0.0f, 0.0f, 0.0f);
@@ -571,14 +629,14 @@ __global__ void k_finish(Atm a, Bake b, const double* __restrict__ partial, int 
         hv = (rowc + 0.5f) / (float)b.height;
     }
     res->horizon_v = hv;
-    float3 s = sun_illuminance(a, b.sun_dir, b.sun_lux, cover);
+    float3 s = sun_illuminance(sun_t, b.sun_lux, cover);
     res->sun[0] = s.x;
     res->sun[1] = s.y;
     res->sun[2] = s.z;
     res->brightest_bits = 0u;
 }
 
-// sky.rs:797-811: the overcast blend (with a cover), then the alpha (the planet's limb share, else 1).
+// sky.rs:797-811: the overcast blend, then the alpha. (Launched with a cover only.)
 __global__ void k_overcast(Bake b, const Result* __restrict__ res, float4* __restrict__ tex) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t n = b.width * b.height;
@@ -599,7 +657,7 @@ __global__ void k_overcast(Bake b, const Result* __restrict__ res, float4* __res
         t.y = t.y + (oy - t.y) * cover;
         t.z = t.z + (oz - t.z) * cover;
     }
-    t.w = (b.planet && t.w > 0.0f) ? t.w : 1.0f;
+    t.w = texel_alpha(b, t.w);
     tex[i] = t;
 }
 
@@ -615,7 +673,38 @@ __global__ void k_env_pack(const float4* __restrict__ tex, uint32_t n, ushort4* 
         lum = fmaxf(0.2126f * t.x + 0.7152f * t.y + 0.0722f * t.z, 0.0f);
     }
     for (int o = 16; o > 0; o >>= 1) lum = fmaxf(lum, __shfl_xor_sync(0xffffffffu, lum, o));
-    if ((threadIdx.x & 31) == 0 && lum > 0.0f) atomicMax(&res->brightest_bits, __float_as_uint(lum));
+    // (a block's maximum first: an atomic a warp on one word took half of the pass)
+    __shared__ float warp_max[8];
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = lum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) lum = fmaxf(lum, warp_max[w]);
+        if (lum > 0.0f) atomicMax(&res->brightest_bits, __float_as_uint(lum));
+    }
+}
+
+// v's running sum in place, in order, by one thread (a chain of additions is all it must wait for: eight values are read
+// ahead of it); the total.
+__device__ __forceinline__ float running_sum(float* v, uint32_t n) {
+    float acc = 0.0f;
+    uint32_t x = 0;
+    for (; x + 8u <= n; x += 8u) {
+        float t[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] = v[x + k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            acc += t[k];
+            t[k] = acc;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[x + k] = t[k];
+    }
+    for (; x < n; ++x) {
+        acc += v[x];
+        v[x] = acc;
+    }
+    return acc;
 }
 
 // lib.rs:916-933: a row's conditional CDF over luminance x sin(theta), its running sum in f32 in texel order.
@@ -629,29 +718,28 @@ __global__ void k_env_rows(const float4* __restrict__ tex, uint32_t w, const flo
         sh[x] = fmaxf(0.2126f * t.x + 0.7152f * t.y + 0.0722f * t.z, 0.0f) * sin_t + 1e-12f;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float acc = 0.0f;
-        for (uint32_t x = 0; x < w; ++x) {
-            acc += sh[x];
-            sh[x] = acc;
-        }
-        rows[y] = acc;
-    }
+    if (threadIdx.x == 0) rows[y] = running_sum(sh, w);
     __syncthreads();
-    float total = rows[y];
+    float total = sh[w - 1u];
     for (uint32_t x = threadIdx.x; x < w; x += blockDim.x) cond[(size_t)y * w + x] = sh[x] / total;
 }
 
-// lib.rs:934-940: the marginal over rows. One thread.
-__global__ void k_env_marginal(const float* __restrict__ rows, uint32_t h, float* __restrict__ marg) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float total = 0.0f;
-    for (uint32_t y = 0; y < h; ++y) total += rows[y];
-    float acc = 0.0f;
-    for (uint32_t y = 0; y < h; ++y) {
-        acc += rows[y] / total;
-        marg[y] = acc;
-    }
+// lib.rs:934-940: the marginal over rows, one block: the total and the running sum in row order by one thread, over
+// shared memory (h floats); the loads and divisions by all. (All of it by one thread took 29 us for 512 rows.)
+constexpr uint32_t MARGINAL_THREADS = 256u;
+__global__ void __launch_bounds__(MARGINAL_THREADS) k_env_marginal(const float* __restrict__ rows, uint32_t h,
+                                                                   float* __restrict__ marg) {
+    extern __shared__ float sh[];
+    __shared__ float total;
+    for (uint32_t y = threadIdx.x; y < h; y += MARGINAL_THREADS) sh[y] = rows[y];
+    __syncthreads();
+    if (threadIdx.x == 0) total = running_sum(sh, h);
+    __syncthreads();
+    for (uint32_t y = threadIdx.x; y < h; y += MARGINAL_THREADS) sh[y] = rows[y] / total;
+    __syncthreads();
+    if (threadIdx.x == 0) running_sum(sh, h);
+    __syncthreads();
+    for (uint32_t y = threadIdx.x; y < h; y += MARGINAL_THREADS) marg[y] = sh[y];
 }
 
 }  // namespace trt_sky
@@ -801,8 +889,8 @@ int sky_bake(SkyState** stp, int device, cudaStream_t stream, const trt_atmosphe
     k_bake<<<(n + 127) / 128, 128, 0, stream>>>(atm, b, st->sun, st->scattered, st->ground, st->tex);
     float cover = std::fmin(std::fmax(a.cloud_cover, 0.0f), 1.0f);
     if (cover > 0.0f) k_cover_partial<<<COVER_BLOCKS, COVER_THREADS, 0, stream>>>(b, st->tex, st->partial);
-    k_finish<<<1, 32, 0, stream>>>(atm, b, st->partial, COVER_BLOCKS, st->res);
-    k_overcast<<<(n + 255) / 256, 256, 0, stream>>>(b, st->res, st->tex);
+    k_finish<<<1, FINISH_THREADS, 0, stream>>>(atm, b, st->partial, COVER_BLOCKS, st->res);
+    if (cover > 0.0f) k_overcast<<<(n + 255) / 256, 256, 0, stream>>>(b, st->res, st->tex);
     SKY_CUDA(cudaGetLastError());
     SKY_CUDA(cudaEventRecord(st->ev[2], stream));
     Result r;
@@ -854,7 +942,7 @@ int sky_env(SkyState* st, cudaStream_t stream, const float* sin_rows_host, void*
     SKY_CUDA(cudaMemsetAsync(&st->res->brightest_bits, 0, 4, stream));
     k_env_pack<<<(n + 255) / 256, 256, 0, stream>>>(st->tex, n, (ushort4*)env, st->res);
     k_env_rows<<<h, 256, w * 4, stream>>>(st->tex, w, st->sin_rows, st->rows, cdf + h);
-    k_env_marginal<<<1, 32, 0, stream>>>(st->rows, h, cdf);
+    k_env_marginal<<<1, MARGINAL_THREADS, h * 4u, stream>>>(st->rows, h, cdf);
     SKY_CUDA(cudaGetLastError());
     SKY_CUDA(cudaEventRecord(st->ev[2], stream));
     Result r;
