@@ -22,8 +22,9 @@ constexpr uint32_t TOP_MAX_DEPTH = TOP_DEPTH - 1u;  // build_sah's max_depth
 constexpr uint32_t TOP_LEVELS = TOP_MAX_DEPTH + 1u; // levels 0 .. TOP_MAX_DEPTH
 constexpr uint32_t MAX_UNITS = 1u << TOP_MAX_DEPTH;
 constexpr uint32_t TOP_BINS = 32u;                  // units.rs:121
-// Top-tree nodes of more units than this are built by a CTA each (k_top_big), the rest by a warp each (k_top_level).
-constexpr uint32_t TOP_SMALL = 256u, BIG_WARPS = 16u;
+// Top-tree nodes of more units than this are split by a block each, a launch a level (k_top_big); the subtree of a node
+// of at most as many is built by one block in its shared memory (k_top_rest).
+constexpr uint32_t TOP_SMALL = 256u, TOP_WARPS = 32u, TOP_THREADS = TOP_WARPS * 32u;
 // Error bits the kernels record.
 constexpr uint32_t E_TREE = 1u, E_DEPTH = 2u, E_ROOT = 4u, E_INDEX = 8u;
 
@@ -171,11 +172,13 @@ struct TopBuild {
     float4* box;      // 2 a unit: lo, hi
     float4* centre;   // a unit's box centre
     uint32_t* order[2];
-    // A level's nodes, (start, end, final index, interior nodes before it in preorder), in two lists: those of at most
-    // TOP_SMALL units (a warp's each) and the larger (a CTA's each); cnt[2 * level + {0, 1}] counts them.
-    uint4* tasks[2];
+    // Nodes to build, (start, end, final index, interior nodes before it in preorder): a level's nodes of more than
+    // TOP_SMALL units (cnt[level] of them), and the roots of the subtrees left to k_top_rest (cnt[TOP_LEVELS] of them, the
+    // node's level in the last word's upper 8 bits).
     uint4* big[2];
+    uint4* rest;
     uint32_t* cnt;
+    uint32_t big_levels;  // levels k_top_big is launched for; larger nodes further down are k_top_rest's
     uint32_t* err;
     uint4* nodes;
     uint32_t top_first, n_units;
@@ -185,10 +188,10 @@ struct TopBuild {
 __global__ void k_unit_boxes(const uint4* __restrict__ tables, uint32_t t_instances, uint64_t n_nodes, TopBuild T) {
     uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u == 0) {
-        bool large = T.n_units > TOP_SMALL;
-        (large ? T.big[0] : T.tasks[0])[0] = make_uint4(0u, T.n_units, 0u, 0u);
-        for (uint32_t l = 0; l <= TOP_LEVELS; ++l) T.cnt[2 * l] = T.cnt[2 * l + 1] = 0u;
-        T.cnt[large ? 1 : 0] = 1u;
+        bool large = T.big_levels > 0u;
+        (large ? T.big[0] : T.rest)[0] = make_uint4(0u, T.n_units, 0u, 0u);
+        for (uint32_t l = 0; l <= TOP_LEVELS; ++l) T.cnt[l] = 0u;
+        T.cnt[large ? 0u : TOP_LEVELS] = 1u;
     }
     if (u >= T.n_units) return;
     T.order[0][u] = u;
@@ -242,18 +245,13 @@ __device__ __forceinline__ int32_t total_key(float f) {
     return b ^ (int32_t)(((uint32_t)(b >> 31)) >> 1);
 }
 
-// A node's two children onto the next level's lists: the left one's place and preorder count follow from its
-// parent's, the right one's from the left side's unit count.
-__device__ __forceinline__ void push_children(const TopBuild& T, uint32_t level, uint32_t start, uint32_t mid,
-                                              uint32_t end, uint32_t pre) {
-    uint4 kids[2] = {make_uint4(start, start + mid, 1u + 2u * pre, pre + 1u),
-                     make_uint4(start + mid, end, 2u + 2u * pre, pre + mid)};
-    for (int c = 0; c < 2; ++c) {
-        bool large = kids[c].y - kids[c].x > TOP_SMALL;
-        uint32_t at = atomicAdd(&T.cnt[2 * (level + 1u) + (large ? 1 : 0)], 1u);
-        (large ? T.big : T.tasks)[(level + 1u) & 1u][at] = kids[c];
-    }
+// A node's two children: the left one's place and preorder count follow from its parent's, the right one's from the left
+// side's unit count.
+__device__ __forceinline__ uint4 child_of(uint4 task, uint32_t mid, int c) {
+    return c == 0 ? make_uint4(task.x, task.x + mid, 1u + 2u * task.w, task.w + 1u)
+                  : make_uint4(task.x + mid, task.y, 2u + 2u * task.w, task.w + mid);
 }
+__device__ __forceinline__ uint4 with_level(uint4 t, uint32_t level) { return make_uint4(t.x, t.y, t.z, t.w | level << 24); }
 
 // A set of bins in shared memory ([axis][component][bin] boxes, [axis][bin] counts). While the units are added the
 // boxes hold f32::total_cmp keys, joined by integer atomic min / max (exact whatever order the lanes and warps come
@@ -393,234 +391,323 @@ __device__ __forceinline__ bool median_left(const TopBuild& T, const uint32_t* o
     return rank < (end - start) / 2u;
 }
 
-// Tasks of more units than this are the CTA kernel's (k_top_big); the rest a warp's (k_top_level).
+// A build block's shared memory (dynamic): each warp's bins, a node's reductions, and a subtree of at most TOP_SMALL
+// units: its units (by slot), their order and the nodes to build, two of each by level.
+struct TopShared {
+    BinBoxes lo[TOP_WARPS][3], hi[TOP_WARPS][3];
+    uint32_t n[TOP_WARPS][3][TOP_BINS];
+    float red[TOP_WARPS][12];
+    uint32_t side[TOP_WARPS][2];
+    float cost;
+    uint32_t best[3];
+    float4 box[2 * TOP_SMALL], centre[TOP_SMALL];
+    uint32_t id[TOP_SMALL], order[2][TOP_SMALL];
+    uint4 tasks[2][TOP_SMALL];
+    uint32_t n_tasks[2];
+    uint4 stack[TOP_LEVELS + 2u];
+};
 
-constexpr uint32_t TOP_WARPS = 8u;
-
-// One level of the build: a warp a node. It takes the node's boxes (order[level & 1][start, end)), picks the split
-// build_sah picks (the cheapest binned split along the centres' axes among those the depth allows, else the median
-// along the widest axis), writes the node where build_sah's depth-first layout puts it and hands its two children to
-// the next level with their items partitioned into order[(level + 1) & 1]. In that layout a node's children sit at
-// 1 + 2 * I and 2 + 2 * I, where I counts the interior nodes before it in preorder: a left child's I is its parent's
-// plus one, a right child's its parent's plus the left side's item count (a subtree of k items has k - 1 interior
-// nodes), so each node's place is known when it is made.
-__global__ void __launch_bounds__(TOP_WARPS * 32) k_top_level(TopBuild T, uint32_t level) {
-    __shared__ float s_lo[TOP_WARPS][3][3][TOP_BINS], s_hi[TOP_WARPS][3][3][TOP_BINS];
-    __shared__ uint32_t s_n[TOP_WARPS][3][TOP_BINS];
-    uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    uint32_t n_tasks = T.cnt[2 * level];
+// build_sah's step for a node of more than TOP_SMALL units, by a block: it takes the node's boxes (order[level & 1][start,
+// end)), picks the split build_sah picks (the cheapest binned split along the centres' axes among those the depth allows,
+// else the median along the widest axis), writes the node where build_sah's depth-first layout puts it and partitions its
+// items into order[(level + 1) & 1]. In that layout a node's children sit at 1 + 2 * I and 2 + 2 * I, where I counts the
+// interior nodes before it in preorder: a left child's I is its parent's plus one, a right child's its parent's plus the
+// left side's item count (a subtree of k items has k - 1 interior nodes), so each node's place is known when it is made.
+// Each warp bins its share of the units into its own set of bins, the sets are joined, a warp sweeps them, and the
+// partition is a block-wide stable scan. The left side's count, or 0 for a node that cannot be split (recorded).
+__device__ uint32_t split_block(const TopBuild& T, TopShared& S, uint4 task, uint32_t level) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    const float pinf = __uint_as_float(0x7f800000u), ninf = __uint_as_float(0xff800000u);
     const uint32_t* order = T.order[level & 1u];
     uint32_t* out = T.order[(level + 1u) & 1u];
-    const uint4* tasks = T.tasks[level & 1u];
-    for (uint32_t ti = blockIdx.x * TOP_WARPS + wib; ti < n_tasks; ti += gridDim.x * TOP_WARPS) {
-        uint4 task = tasks[ti];
-        uint32_t start = task.x, end = task.y, fin = task.z, pre = task.w, count = end - start;
-        V3 lo = v3(__uint_as_float(0x7f800000u)), hi = v3(__uint_as_float(0xff800000u)), clo = lo, chi = hi;
-        for (uint32_t j = start + lane; j < end; j += 32u) {
-            uint32_t k = order[j];
-            float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
-            lo = V3{gmin(lo.x, bl.x), gmin(lo.y, bl.y), gmin(lo.z, bl.z)};
-            hi = V3{gmax(hi.x, bh.x), gmax(hi.y, bh.y), gmax(hi.z, bh.z)};
-            clo = V3{gmin(clo.x, c.x), gmin(clo.y, c.y), gmin(clo.z, c.z)};
-            chi = V3{gmax(chi.x, c.x), gmax(chi.y, c.y), gmax(chi.z, c.z)};
-        }
+    const uint32_t start = task.x, end = task.y, fin = task.z, pre = task.w, count = end - start;
+    if (fin >= 2u * T.n_units - 1u || end > T.n_units || level >= TOP_MAX_DEPTH) {
+        if (tid == 0) atomicOr(T.err, level >= TOP_MAX_DEPTH ? E_DEPTH : E_TREE);
+        return 0u;
+    }
+    // The node's box and its units' centres' box.
+    float r[12] = {pinf, pinf, pinf, ninf, ninf, ninf, pinf, pinf, pinf, ninf, ninf, ninf};
+#pragma unroll 4
+    for (uint32_t j = start + tid; j < end; j += TOP_THREADS) {
+        uint32_t k = order[j];
+        float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
+        r[0] = gmin(r[0], bl.x); r[1] = gmin(r[1], bl.y); r[2] = gmin(r[2], bl.z);
+        r[3] = gmax(r[3], bh.x); r[4] = gmax(r[4], bh.y); r[5] = gmax(r[5], bh.z);
+        r[6] = gmin(r[6], c.x); r[7] = gmin(r[7], c.y); r[8] = gmin(r[8], c.z);
+        r[9] = gmax(r[9], c.x); r[10] = gmax(r[10], c.y); r[11] = gmax(r[11], c.z);
+    }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo = V3{gmin(lo.x, __shfl_xor_sync(~0u, lo.x, o)), gmin(lo.y, __shfl_xor_sync(~0u, lo.y, o)), gmin(lo.z, __shfl_xor_sync(~0u, lo.z, o))};
-            hi = V3{gmax(hi.x, __shfl_xor_sync(~0u, hi.x, o)), gmax(hi.y, __shfl_xor_sync(~0u, hi.y, o)), gmax(hi.z, __shfl_xor_sync(~0u, hi.z, o))};
-            clo = V3{gmin(clo.x, __shfl_xor_sync(~0u, clo.x, o)), gmin(clo.y, __shfl_xor_sync(~0u, clo.y, o)), gmin(clo.z, __shfl_xor_sync(~0u, clo.z, o))};
-            chi = V3{gmax(chi.x, __shfl_xor_sync(~0u, chi.x, o)), gmax(chi.y, __shfl_xor_sync(~0u, chi.y, o)), gmax(chi.z, __shfl_xor_sync(~0u, chi.z, o))};
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 12; ++q) {
+            float v = __shfl_xor_sync(~0u, r[q], o);
+            r[q] = (q % 6) < 3 ? gmin(r[q], v) : gmax(r[q], v);
         }
-        if (fin >= 2u * T.n_units - 1u || count == 0 || end > T.n_units) {  // (a build of n leaves has 2n - 1 nodes)
-            if (lane == 0) atomicOr(T.err, E_TREE);
-            continue;
+    if (lane == 0)
+        for (int q = 0; q < 12; ++q) S.red[w][q] = r[q];
+    bins_clear(S.lo[w], S.hi[w], S.n[w], lane, 32u);
+    __syncthreads();
+    // (each warp joins the warps' parts: a lane a warp's)
+#pragma unroll
+    for (int q = 0; q < 12; ++q) r[q] = S.red[lane][q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 12; ++q) {
+            float v = __shfl_xor_sync(~0u, r[q], o);
+            r[q] = (q % 6) < 3 ? gmin(r[q], v) : gmax(r[q], v);
         }
-        uint32_t node = T.top_first + fin;
-        if (count == 1) {
-            if (lane == 0) store_box(T.nodes, node, lo, hi, order[start], 1u);
-            continue;
-        }
-        if (level >= TOP_MAX_DEPTH || count > MAX_UNITS) {
-            if (lane == 0) atomicOr(T.err, E_DEPTH);
-            continue;
-        }
-        uint32_t room = 1u << (TOP_MAX_DEPTH - level - 1u);
-        V3 ext = chi - clo;
-        float scale[3] = {(float)TOP_BINS / ext.x, (float)TOP_BINS / ext.y, (float)TOP_BINS / ext.z};
-        bool use[3] = {ext.x > 0.0f, ext.y > 0.0f, ext.z > 0.0f};
-        bins_clear(s_lo[wib], s_hi[wib], s_n[wib], lane, 32u);
-        __syncwarp();
-        for (uint32_t base = start; base < end; base += 32u) {
-            uint32_t j = base + lane;
-            bool valid = j < end;
-            uint32_t k = valid ? order[j] : order[start];
-            float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
-            bins_add(s_lo[wib], s_hi[wib], s_n[wib], pack_bins(valid, c, clo, scale, use), bl, bh);
-        }
-        __syncwarp();
-        bins_to_floats(s_lo[wib], s_hi[wib], lane, 32u);
-        __syncwarp();
-        float best_cost = 0.0f;
-        uint32_t best_axis = 0, best_split = 0, best_left = 0;
-        sah_sweep(s_lo[wib], s_hi[wib], s_n[wib], use, count, room, best_cost, best_axis, best_split, best_left);
-        bool binned = finite1(best_cost);
-        uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
-        uint32_t mid = binned ? best_left : count / 2u;
-        // Partition, left side first (stable: the order inside a side does not change the tree).
-        uint32_t nl_run = 0, nr_run = 0;
-        for (uint32_t base = start; base < end; base += 32u) {
-            uint32_t j = base + lane;
-            bool valid = j < end, left = false;
-            uint32_t k = valid ? order[j] : 0u;
-            if (valid) {
-                if (binned) {
-                    left = bin_of(comp(T.centre[k], best_axis), comp3(clo, best_axis), scale[best_axis]) < best_split;
-                } else {
-                    left = median_left(T, order, start, end, k, med_axis);
-                }
+    V3 lo{r[0], r[1], r[2]}, hi{r[3], r[4], r[5]}, clo{r[6], r[7], r[8]}, chi{r[9], r[10], r[11]};
+    uint32_t room = 1u << (TOP_MAX_DEPTH - level - 1u);
+    V3 ext = chi - clo;
+    float scale[3] = {(float)TOP_BINS / ext.x, (float)TOP_BINS / ext.y, (float)TOP_BINS / ext.z};
+    bool use[3] = {ext.x > 0.0f, ext.y > 0.0f, ext.z > 0.0f};
+#pragma unroll 2
+    for (uint32_t base = start + 32u * w; base < end; base += TOP_THREADS) {
+        uint32_t j = base + lane;
+        bool valid = j < end;
+        uint32_t k = valid ? order[j] : order[start];
+        float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
+        bins_add(S.lo[w], S.hi[w], S.n[w], pack_bins(valid, c, clo, scale, use), bl, bh);
+    }
+    __syncthreads();
+    // The warps' bins joined into warp 0's, on their keys (min / max and sums do not depend on the order): seven values
+    // a bin, a thread a value.
+    for (uint32_t i = tid; i < 7u * 3u * TOP_BINS; i += TOP_THREADS) {
+        const uint32_t q = i / (3u * TOP_BINS), ax = i / TOP_BINS % 3u, b = i % TOP_BINS;
+        if (q == 6u) {
+            uint32_t sum = 0u;
+            for (uint32_t ww = 0; ww < TOP_WARPS; ++ww) sum += S.n[ww][ax][b];
+            S.n[0][ax][b] = sum;
+        } else {
+            BinBoxes(*set)[3] = q < 3u ? S.lo : S.hi;
+            int v = __float_as_int(set[0][ax][q % 3u][b]);
+            for (uint32_t ww = 1; ww < TOP_WARPS; ++ww) {
+                const int o = __float_as_int(set[ww][ax][q % 3u][b]);
+                v = q < 3u ? min(v, o) : max(v, o);
             }
-            unsigned lm = __ballot_sync(~0u, valid && left), rm = __ballot_sync(~0u, valid && !left);
-            unsigned below = (1u << lane) - 1u;
-            if (valid) {
-                if (left) out[start + nl_run + __popc(lm & below)] = k;
-                else out[start + mid + nr_run + __popc(rm & below)] = k;
-            }
-            nl_run += __popc(lm);
-            nr_run += __popc(rm);
+            set[0][ax][q % 3u][b] = key_float(v);
         }
+    }
+    __syncthreads();
+    if (w == 0) {
+        float c;
+        uint32_t a, sp, l;
+        sah_sweep(S.lo[0], S.hi[0], S.n[0], use, count, room, c, a, sp, l);
         if (lane == 0) {
-            if (nl_run != mid) atomicOr(T.err, E_TREE);
-            store_box(T.nodes, node, lo, hi, 1u + 2u * pre, 0u);
-            push_children(T, level, start, mid, end, pre);
+            S.cost = c;
+            S.best[0] = a; S.best[1] = sp; S.best[2] = l;
         }
+    }
+    __syncthreads();
+    const bool binned = finite1(S.cost);
+    const uint32_t best_axis = S.best[0], best_split = S.best[1];
+    const uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
+    const uint32_t mid = binned ? S.best[2] : count / 2u;
+    // Stable partition, a block-wide chunk at a time.
+    uint32_t nl_run = 0, nr_run = 0;
+    for (uint32_t base = start; base < end; base += TOP_THREADS) {
+        uint32_t j = base + tid;
+        bool valid = j < end, left = false;
+        uint32_t k = valid ? order[j] : 0u;
+        if (valid)
+            left = binned ? bin_of(comp(T.centre[k], best_axis), comp3(clo, best_axis), scale[best_axis]) < best_split
+                          : median_left(T, order, start, end, k, med_axis);
+        unsigned lm = __ballot_sync(~0u, valid && left), rm = __ballot_sync(~0u, valid && !left);
+        if (lane == 0) { S.side[w][0] = __popc(lm); S.side[w][1] = __popc(rm); }
+        __syncthreads();
+        // (the warps' sides by a scan over the lanes)
+        uint32_t pl = S.side[lane][0], pr = S.side[lane][1];
+        const uint32_t own_l = pl, own_r = pr;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t tl = __shfl_up_sync(~0u, pl, o), tr = __shfl_up_sync(~0u, pr, o);
+            if (lane >= o) { pl += tl; pr += tr; }
+        }
+        const uint32_t lb = __shfl_sync(~0u, pl - own_l, w), rb = __shfl_sync(~0u, pr - own_r, w);
+        unsigned below = (1u << lane) - 1u;
+        if (valid) {
+            if (left) out[start + nl_run + lb + __popc(lm & below)] = k;
+            else out[start + mid + nr_run + rb + __popc(rm & below)] = k;
+        }
+        nl_run += __shfl_sync(~0u, pl, 31);
+        nr_run += __shfl_sync(~0u, pr, 31);
+        __syncthreads();
+    }
+    if (tid == 0) {
+        if (nl_run != mid) atomicOr(T.err, E_TREE);
+        store_box(T.nodes, T.top_first + fin, lo, hi, 1u + 2u * pre, 0u);
+    }
+    return mid;
+}
+
+// A level's nodes of more than TOP_SMALL units, a block a node; their children to the next level's list or to
+// k_top_rest's.
+__global__ void __launch_bounds__(TOP_THREADS) k_top_big(TopBuild T, uint32_t level) {
+    extern __shared__ __align__(16) uint8_t top_smem[];
+    TopShared& S = *reinterpret_cast<TopShared*>(top_smem);
+    const uint32_t n_tasks = T.cnt[level];
+    for (uint32_t ti = blockIdx.x; ti < n_tasks; ti += gridDim.x) {
+        const uint4 task = T.big[level & 1u][ti];
+        const uint32_t mid = split_block(T, S, task, level);
+        if (threadIdx.x == 0 && mid != 0u)
+            for (int c = 0; c < 2; ++c) {
+                const uint4 kid = child_of(task, mid, c);
+                if (kid.y - kid.x > TOP_SMALL && level + 1u < T.big_levels)
+                    T.big[(level + 1u) & 1u][atomicAdd(&T.cnt[level + 1u], 1u)] = kid;
+                else
+                    T.rest[atomicAdd(&T.cnt[TOP_LEVELS], 1u)] = with_level(kid, level + 1u);
+            }
+        __syncthreads();
     }
 }
 
-
-// The same step for nodes of more than TOP_SMALL units, a CTA a node: each warp bins its share of the units into its
-// own set of bins, the sets are joined, one thread sweeps them, and the partition is a CTA-wide stable scan.
-__global__ void __launch_bounds__(BIG_WARPS * 32) k_top_big(TopBuild T, uint32_t level) {
-    __shared__ float s_lo[BIG_WARPS][3][3][TOP_BINS], s_hi[BIG_WARPS][3][3][TOP_BINS];
-    __shared__ uint32_t s_n[BIG_WARPS][3][TOP_BINS];
-    __shared__ float s_red[BIG_WARPS][12];
-    __shared__ uint32_t s_side[BIG_WARPS][2];
-    __shared__ float s_cost;
-    __shared__ uint32_t s_best[3];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, nt = BIG_WARPS * 32u;
-    const float pinf = __uint_as_float(0x7f800000u), ninf = __uint_as_float(0xff800000u);
-    uint32_t n_tasks = T.cnt[2 * level + 1];
-    const uint32_t* order = T.order[level & 1u];
-    uint32_t* out = T.order[(level + 1u) & 1u];
-    const uint4* tasks = T.big[level & 1u];
-    for (uint32_t ti = blockIdx.x; ti < n_tasks; ti += gridDim.x) {
-        uint4 task = tasks[ti];
-        uint32_t start = task.x, end = task.y, fin = task.z, pre = task.w, count = end - start;
-        if (fin >= 2u * T.n_units - 1u || end > T.n_units || level >= TOP_MAX_DEPTH) {
-            if (tid == 0) atomicOr(T.err, level >= TOP_MAX_DEPTH ? E_DEPTH : E_TREE);
-            continue;
-        }
-        // The node's box and its units' centres' box.
-        float r[12] = {pinf, pinf, pinf, ninf, ninf, ninf, pinf, pinf, pinf, ninf, ninf, ninf};
-        for (uint32_t j = start + tid; j < end; j += nt) {
-            uint32_t k = order[j];
-            float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
-            r[0] = gmin(r[0], bl.x); r[1] = gmin(r[1], bl.y); r[2] = gmin(r[2], bl.z);
-            r[3] = gmax(r[3], bh.x); r[4] = gmax(r[4], bh.y); r[5] = gmax(r[5], bh.z);
-            r[6] = gmin(r[6], c.x); r[7] = gmin(r[7], c.y); r[8] = gmin(r[8], c.z);
-            r[9] = gmax(r[9], c.x); r[10] = gmax(r[10], c.y); r[11] = gmax(r[11], c.z);
-        }
+// The same step for a node of a subtree in shared memory, by a warp: slots order[level & 1][start, end) of the subtree.
+__device__ void split_warp(const TopBuild& T, TopShared& S, uint4 task, uint32_t level) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t* order = S.order[level & 1u];
+    uint32_t* out = S.order[(level + 1u) & 1u];
+    const uint32_t start = task.x, end = task.y, fin = task.z, pre = task.w, count = end - start;
+    V3 lo = v3(__uint_as_float(0x7f800000u)), hi = v3(__uint_as_float(0xff800000u)), clo = lo, chi = hi;
+    for (uint32_t j = start + lane; j < end; j += 32u) {
+        const uint32_t k = order[j];
+        const float4 bl = S.box[2u * k], bh = S.box[2u * k + 1u], c = S.centre[k];
+        lo = V3{gmin(lo.x, bl.x), gmin(lo.y, bl.y), gmin(lo.z, bl.z)};
+        hi = V3{gmax(hi.x, bh.x), gmax(hi.y, bh.y), gmax(hi.z, bh.z)};
+        clo = V3{gmin(clo.x, c.x), gmin(clo.y, c.y), gmin(clo.z, c.z)};
+        chi = V3{gmax(chi.x, c.x), gmax(chi.y, c.y), gmax(chi.z, c.z)};
+    }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < 12; ++q) {
-                float v = __shfl_xor_sync(~0u, r[q], o);
-                r[q] = (q % 6) < 3 ? gmin(r[q], v) : gmax(r[q], v);
-            }
-        if (lane == 0)
-            for (int q = 0; q < 12; ++q) s_red[w][q] = r[q];
-        for (uint32_t i = tid; i < BIG_WARPS * 3u * TOP_BINS; i += nt)
-            bins_clear(s_lo[i / (3u * TOP_BINS)], s_hi[i / (3u * TOP_BINS)], s_n[i / (3u * TOP_BINS)],
-                       i % (3u * TOP_BINS), 3u * TOP_BINS);
-        __syncthreads();
-        for (int q = 0; q < 12; ++q) {
-            float v = s_red[0][q];
-            for (uint32_t ww = 1; ww < BIG_WARPS; ++ww) v = (q % 6) < 3 ? gmin(v, s_red[ww][q]) : gmax(v, s_red[ww][q]);
-            r[q] = v;
-        }
-        V3 lo{r[0], r[1], r[2]}, hi{r[3], r[4], r[5]}, clo{r[6], r[7], r[8]}, chi{r[9], r[10], r[11]};
-        uint32_t room = 1u << (TOP_MAX_DEPTH - level - 1u);
-        V3 ext = chi - clo;
-        float scale[3] = {(float)TOP_BINS / ext.x, (float)TOP_BINS / ext.y, (float)TOP_BINS / ext.z};
-        bool use[3] = {ext.x > 0.0f, ext.y > 0.0f, ext.z > 0.0f};
-        for (uint32_t base = start + 32u * w; base < end; base += nt) {
-            uint32_t j = base + lane;
-            bool valid = j < end;
-            uint32_t k = valid ? order[j] : order[start];
-            float4 bl = T.box[2ull * k], bh = T.box[2ull * k + 1], c = T.centre[k];
-            bins_add(s_lo[w], s_hi[w], s_n[w], pack_bins(valid, c, clo, scale, use), bl, bh);
-        }
-        __syncthreads();
-        // The warps' bins joined into warp 0's, on their keys (min / max and sums do not depend on the order).
-        for (uint32_t i = tid; i < 3u * TOP_BINS; i += nt) {
-            uint32_t ax = i / TOP_BINS, bn = i % TOP_BINS;
-            for (uint32_t ww = 1; ww < BIG_WARPS; ++ww) {
-                for (int q = 0; q < 3; ++q) {
-                    s_lo[0][ax][q][bn] = __int_as_float(
-                        min(__float_as_int(s_lo[0][ax][q][bn]), __float_as_int(s_lo[ww][ax][q][bn])));
-                    s_hi[0][ax][q][bn] = __int_as_float(
-                        max(__float_as_int(s_hi[0][ax][q][bn]), __float_as_int(s_hi[ww][ax][q][bn])));
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = V3{gmin(lo.x, __shfl_xor_sync(~0u, lo.x, o)), gmin(lo.y, __shfl_xor_sync(~0u, lo.y, o)), gmin(lo.z, __shfl_xor_sync(~0u, lo.z, o))};
+        hi = V3{gmax(hi.x, __shfl_xor_sync(~0u, hi.x, o)), gmax(hi.y, __shfl_xor_sync(~0u, hi.y, o)), gmax(hi.z, __shfl_xor_sync(~0u, hi.z, o))};
+        clo = V3{gmin(clo.x, __shfl_xor_sync(~0u, clo.x, o)), gmin(clo.y, __shfl_xor_sync(~0u, clo.y, o)), gmin(clo.z, __shfl_xor_sync(~0u, clo.z, o))};
+        chi = V3{gmax(chi.x, __shfl_xor_sync(~0u, chi.x, o)), gmax(chi.y, __shfl_xor_sync(~0u, chi.y, o)), gmax(chi.z, __shfl_xor_sync(~0u, chi.z, o))};
+    }
+    if (fin >= 2u * T.n_units - 1u || count == 0) {  // (a build of n leaves has 2n - 1 nodes)
+        if (lane == 0) atomicOr(T.err, E_TREE);
+        return;
+    }
+    const uint32_t node = T.top_first + fin;
+    if (count == 1) {
+        if (lane == 0) store_box(T.nodes, node, lo, hi, S.id[order[start]], 1u);
+        return;
+    }
+    if (level >= TOP_MAX_DEPTH) {
+        if (lane == 0) atomicOr(T.err, E_DEPTH);
+        return;
+    }
+    const uint32_t room = 1u << (TOP_MAX_DEPTH - level - 1u);
+    const V3 ext = chi - clo;
+    const float scale[3] = {(float)TOP_BINS / ext.x, (float)TOP_BINS / ext.y, (float)TOP_BINS / ext.z};
+    const bool use[3] = {ext.x > 0.0f, ext.y > 0.0f, ext.z > 0.0f};
+    bins_clear(S.lo[w], S.hi[w], S.n[w], lane, 32u);
+    __syncwarp();
+    for (uint32_t base = start; base < end; base += 32u) {
+        const uint32_t j = base + lane;
+        const bool valid = j < end;
+        const uint32_t k = order[valid ? j : start];
+        bins_add(S.lo[w], S.hi[w], S.n[w], pack_bins(valid, S.centre[k], clo, scale, use), S.box[2u * k], S.box[2u * k + 1u]);
+    }
+    __syncwarp();
+    bins_to_floats(S.lo[w], S.hi[w], lane, 32u);
+    __syncwarp();
+    float best_cost = 0.0f;
+    uint32_t best_axis = 0, best_split = 0, best_left = 0;
+    sah_sweep(S.lo[w], S.hi[w], S.n[w], use, count, room, best_cost, best_axis, best_split, best_left);
+    const bool binned = finite1(best_cost);
+    const uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
+    const uint32_t mid = binned ? best_left : count / 2u;
+    // Partition, left side first (stable: the order inside a side does not change the tree).
+    uint32_t nl_run = 0, nr_run = 0;
+    for (uint32_t base = start; base < end; base += 32u) {
+        const uint32_t j = base + lane;
+        const bool valid = j < end;
+        bool left = false;
+        const uint32_t k = order[valid ? j : start];
+        if (valid) {
+            if (binned) {
+                left = bin_of(comp(S.centre[k], best_axis), comp3(clo, best_axis), scale[best_axis]) < best_split;
+            } else {
+                const int32_t kk = total_key(comp(S.centre[k], med_axis));
+                uint32_t rank = 0;
+                for (uint32_t q = start; q < end; ++q) {
+                    const uint32_t o = order[q];
+                    const int32_t ko = total_key(comp(S.centre[o], med_axis));
+                    rank += (ko < kk || (ko == kk && S.id[o] < S.id[k])) ? 1u : 0u;
                 }
-                s_n[0][ax][bn] += s_n[ww][ax][bn];
+                left = rank < count / 2u;
             }
         }
-        __syncthreads();
-        bins_to_floats(s_lo[0], s_hi[0], tid, nt);
-        __syncthreads();
-        if (w == 0) {
-            float c;
-            uint32_t a, sp, l;
-            sah_sweep(s_lo[0], s_hi[0], s_n[0], use, count, room, c, a, sp, l);
-            if (lane == 0) {
-                s_cost = c;
-                s_best[0] = a; s_best[1] = sp; s_best[2] = l;
-            }
+        const unsigned lm = __ballot_sync(~0u, valid && left), rm = __ballot_sync(~0u, valid && !left);
+        const unsigned below = (1u << lane) - 1u;
+        if (valid) {
+            if (left) out[start + nl_run + __popc(lm & below)] = k;
+            else out[start + mid + nr_run + __popc(rm & below)] = k;
         }
+        nl_run += __popc(lm);
+        nr_run += __popc(rm);
+    }
+    if (lane == 0) {
+        if (nl_run != mid) atomicOr(T.err, E_TREE);
+        store_box(T.nodes, node, lo, hi, 1u + 2u * pre, 0u);
+        const uint32_t at = atomicAdd(&S.n_tasks[(level + 1u) & 1u], 2u);
+        S.tasks[(level + 1u) & 1u][at] = child_of(task, mid, 0);
+        S.tasks[(level + 1u) & 1u][at + 1u] = child_of(task, mid, 1);
+    }
+}
+
+// What k_top_big left, a block a subtree: nodes still larger than TOP_SMALL one after another, then each node of at most
+// as many units with everything below it, in shared memory, a level at a time with a barrier between, a warp a node.
+// (Every level of the whole tree as two launches took 19 of them and 0.41 ms for 5,002 units, 5-10 us of latency each.)
+__global__ void __launch_bounds__(TOP_THREADS) k_top_rest(TopBuild T) {
+    extern __shared__ __align__(16) uint8_t top_smem[];
+    TopShared& S = *reinterpret_cast<TopShared*>(top_smem);
+    const uint32_t tid = threadIdx.x, w = tid >> 5, n_rest = T.cnt[TOP_LEVELS];
+    for (uint32_t ti = blockIdx.x; ti < n_rest; ti += gridDim.x) {
+        if (tid == 0) S.stack[0] = T.rest[ti];
+        uint32_t sp = 1u;  // (a node's two children are a level down: at most a level's worth more than the levels)
         __syncthreads();
-        bool binned = finite1(s_cost);
-        uint32_t best_axis = s_best[0], best_split = s_best[1];
-        uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
-        uint32_t mid = binned ? s_best[2] : count / 2u;
-        // Stable partition, a CTA-wide chunk at a time.
-        uint32_t nl_run = 0, nr_run = 0;
-        for (uint32_t base = start; base < end; base += nt) {
-            uint32_t j = base + tid;
-            bool valid = j < end, left = false;
-            uint32_t k = valid ? order[j] : 0u;
-            if (valid)
-                left = binned ? bin_of(comp(T.centre[k], best_axis), comp3(clo, best_axis), scale[best_axis]) < best_split
-                              : median_left(T, order, start, end, k, med_axis);
-            unsigned lm = __ballot_sync(~0u, valid && left), rm = __ballot_sync(~0u, valid && !left);
-            if (lane == 0) { s_side[w][0] = __popc(lm); s_side[w][1] = __popc(rm); }
+        while (sp > 0u) {
+            uint4 task = S.stack[--sp];
+            uint32_t level = task.w >> 24;
+            task.w &= 0xffffffu;
             __syncthreads();
-            uint32_t lb = 0, rb = 0, lt = 0, rt = 0;
-            for (uint32_t ww = 0; ww < BIG_WARPS; ++ww) {
-                if (ww < w) { lb += s_side[ww][0]; rb += s_side[ww][1]; }
-                lt += s_side[ww][0];
-                rt += s_side[ww][1];
+            const uint32_t count = task.y - task.x;
+            if (count > TOP_SMALL) {
+                const uint32_t mid = split_block(T, S, task, level);
+                if (mid != 0u) {
+                    if (tid < 2u) S.stack[sp + tid] = with_level(child_of(task, mid, (int)tid), level + 1u);
+                    sp += 2u;
+                }
+                __syncthreads();
+                continue;
             }
-            unsigned below = (1u << lane) - 1u;
-            if (valid) {
-                if (left) out[start + nl_run + lb + __popc(lm & below)] = k;
-                else out[start + mid + nr_run + rb + __popc(rm & below)] = k;
+            if (task.y > T.n_units || count == 0u) {
+                if (tid == 0) atomicOr(T.err, E_TREE);
+                continue;
             }
-            nl_run += lt;
-            nr_run += rt;
-            __syncthreads();
-        }
-        if (tid == 0) {
-            if (nl_run != mid) atomicOr(T.err, E_TREE);
-            store_box(T.nodes, T.top_first + fin, lo, hi, 1u + 2u * pre, 0u);
-            push_children(T, level, start, mid, end, pre);
+            // the subtree's units by slot
+            for (uint32_t k = tid; k < count; k += TOP_THREADS) {
+                const uint32_t u = T.order[level & 1u][task.x + k];
+                S.id[k] = u;
+                S.order[level & 1u][k] = k;
+                S.box[2u * k] = T.box[2ull * u];
+                S.box[2u * k + 1u] = T.box[2ull * u + 1];
+                S.centre[k] = T.centre[u];
+            }
+            if (tid == 0) {
+                S.tasks[level & 1u][0] = make_uint4(0u, count, task.z, task.w);
+                S.n_tasks[level & 1u] = 1u;
+            }
+            for (;; ++level) {
+                if (tid == 0) S.n_tasks[(level + 1u) & 1u] = 0u;
+                __syncthreads();
+                const uint32_t n = S.n_tasks[level & 1u];
+                if (n == 0u) break;
+                for (uint32_t q = w; q < n; q += TOP_WARPS) split_warp(T, S, S.tasks[level & 1u][q], level);
+                __syncthreads();
+            }
         }
         __syncthreads();
     }
@@ -675,16 +762,17 @@ int ensure_top(DeformState* st, uint32_t n_units, std::string& err) {
     auto add = [&](uint64_t b) { uint64_t at = need; need += (b + 255) / 256 * 256; return at; };
     uint64_t n_big = n_units / (TOP_SMALL + 1u) + 1u;  // nodes of a level are disjoint: at most this many large
     uint64_t o_box = add(32ull * n_units), o_c = add(16ull * n_units), o_o0 = add(4ull * n_units),
-             o_o1 = add(4ull * n_units), o_t0 = add(16ull * n_units), o_t1 = add(16ull * n_units),
-             o_b0 = add(16ull * n_big), o_b1 = add(16ull * n_big), o_cnt = add(8ull * (TOP_LEVELS + 1));
+             o_o1 = add(4ull * n_units), o_r = add(16ull * n_units), o_b0 = add(16ull * n_big), o_b1 = add(16ull * n_big),
+             o_cnt = add(4ull * (TOP_LEVELS + 1));
+    DF_CUDA(cudaFuncSetAttribute(k_top_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopShared)));
+    DF_CUDA(cudaFuncSetAttribute(k_top_rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopShared)));
     DF_CUDA(cudaMalloc(&st->top, need));
     char* b = (char*)st->top;
     st->T.box = (float4*)(b + o_box);
     st->T.centre = (float4*)(b + o_c);
     st->T.order[0] = (uint32_t*)(b + o_o0);
     st->T.order[1] = (uint32_t*)(b + o_o1);
-    st->T.tasks[0] = (uint4*)(b + o_t0);
-    st->T.tasks[1] = (uint4*)(b + o_t1);
+    st->T.rest = (uint4*)(b + o_r);
     st->T.big[0] = (uint4*)(b + o_b0);
     st->T.big[1] = (uint4*)(b + o_b1);
     st->T.cnt = (uint32_t*)(b + o_cnt);
@@ -887,14 +975,21 @@ int deform_run(DeformState* st, const SceneBuffers& sb, const uint32_t* P, const
     T.nodes = nodes;
     T.top_first = top;
     T.n_units = n_units;
-    k_unit_boxes<<<(n_units + 255) / 256, 256, 0, s>>>((const uint4*)sb.buf[3], t_instances, n_nodes, T);
-    for (uint32_t level = 0; level < TOP_LEVELS; ++level) {
-        uint32_t most = std::min<uint32_t>(1u << level, n_units);  // a level holds at most 2^level nodes
-        uint32_t big = std::min(most, n_units / (TOP_SMALL + 1u));  // ... and at most this many of over TOP_SMALL
-        if (big) k_top_big<<<std::min(big, 148u * 2u), BIG_WARPS * 32, 0, s>>>(T, level);
-        uint32_t blocks = std::max(1u, std::min((most + TOP_WARPS - 1) / TOP_WARPS, 148u * 8u));
-        k_top_level<<<blocks, TOP_WARPS * 32, 0, s>>>(T, level);
+    // A launch a level while nodes larger than TOP_SMALL are to be expected (halving, and three levels more for uneven
+    // splits; larger nodes below them are k_top_rest's too).
+    T.big_levels = 0u;
+    if (n_units > TOP_SMALL) {
+        T.big_levels = 3u;
+        for (uint32_t k = n_units; k > TOP_SMALL; k = (k + 1u) / 2u) ++T.big_levels;
+        T.big_levels = std::min(T.big_levels, TOP_LEVELS);
     }
+    k_unit_boxes<<<(n_units + 255) / 256, 256, 0, s>>>((const uint4*)sb.buf[3], t_instances, n_nodes, T);
+    for (uint32_t level = 0; level < T.big_levels; ++level) {
+        // a level holds at most 2^level nodes, and at most this many of over TOP_SMALL units
+        const uint32_t most = std::min<uint32_t>(1u << level, n_units / (TOP_SMALL + 1u));
+        k_top_big<<<std::min(most, 148u), TOP_THREADS, sizeof(TopShared), s>>>(T, level);
+    }
+    k_top_rest<<<std::min(n_units / 64u + 1u, 148u * 2u), TOP_THREADS, sizeof(TopShared), s>>>(T);
     if (stats) DF_CUDA(cudaEventRecord(st->ev[4], s));
     DF_CUDA(cudaGetLastError());
     if (stats) {
