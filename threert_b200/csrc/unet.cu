@@ -94,8 +94,11 @@ struct Conv {
     uint32_t stages;          // the halo variant's stages
 };
 
-constexpr uint32_t TS = 5;                  // pipeline stages (82 KB of shared memory: two CTAs an SM)
-constexpr uint32_t A_STAGE = 128u * 32u * 2u, B_STAGE = 128u * 32u * 2u;
+// The 2-D tiles' pipeline: KB K blocks (one tap, 32 channels each; a layer has a multiple of 9) a stage, so that a
+// stage's waits are paid once for them, TS stages (99 KB of shared memory: two CTAs an SM). Five stages of one block took
+// 185 us for the 264 x 136 forward and 487 for a training step on 16 crops of 64 x 64; two of three, 161 and 455.
+constexpr uint32_t TS = 2u, KB = 3u;
+constexpr uint32_t A_BOX = 128u * 32u * 2u, B_BOX = 128u * 32u * 2u, A_STAGE = KB * A_BOX, B_STAGE = KB * B_BOX;
 constexpr uint32_t CONV_SMEM = TS * (A_STAGE + B_STAGE) + 256u + 1024u;  // + room to align the stages to 1 KB
 // The halo variant (a row tile of 128 pixels read once with its halo, the taps as shifted descriptors): a stage is a
 // 32-channel block's 3 rows x 130 pixels, 64 bytes a pixel in the 64-byte swizzle, padded to a multiple of 1 KB.
@@ -298,7 +301,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t sraw = smem_addr(smem_raw), sbase = (sraw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (sbase - sraw);
-    const uint32_t kc = a.cin / 32u, nk = HALO ? kc : 9u * kc;
+    const uint32_t kc = a.cin / 32u, nb = 9u * kc, nk = HALO ? kc : (nb + KB - 1u) / KB;  // (nk: a tile's stages)
     const uint32_t A_OFF = HALO && a.resident ? halo_weights(kc, a.nt) : 0u, B_OFF = HALO ? 0u : TS * A_STAGE;
     const uint32_t BAR_OFF = HALO ? A_OFF + NS * A_BYTES : TS * (A_STAGE + B_STAGE);
     const uint32_t sA = sbase + A_OFF, sB = sbase + B_OFF, sBar = sbase + BAR_OFF;
@@ -389,12 +392,17 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                                 tma_load_3d(leader, sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
                                             (int)n0, (int)tap, full(s));
                     } else {
-                        mbar_expect_tx(leader, full(s), A_STAGE + (a.resident ? 0u : a.nt * 64u));
-                        const uint32_t tap = k / kc, c0 = (k % kc) * 32u;
-                        const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
-                        if (!withhold)
-                            tma_load_4d(leader, sA + s * A_STAGE, &xmap, (int)(a.x_off + c0), x0 + dx, y0 + dy, (int)b, full(s));
-                        if (!a.resident) tma_load_3d(leader, sB + s * B_STAGE, &wmap, (int)c0, (int)n0, (int)tap, full(s));
+                        const uint32_t here = min(KB, nb - k * KB);
+                        mbar_expect_tx(leader, full(s), here * (A_BOX + (a.resident ? 0u : a.nt * 64u)));
+                        for (uint32_t i = 0; i < here; ++i) {
+                            const uint32_t tap = (k * KB + i) / kc, c0 = (k * KB + i) % kc * 32u;
+                            const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
+                            if (!withhold || i != 0u)
+                                tma_load_4d(leader, sA + s * A_STAGE + i * A_BOX, &xmap, (int)(a.x_off + c0), x0 + dx,
+                                            y0 + dy, (int)b, full(s));
+                            if (!a.resident)
+                                tma_load_3d(leader, sB + s * B_STAGE + i * B_BOX, &wmap, (int)c0, (int)n0, (int)tap, full(s));
+                        }
                     }
                 }
             }
@@ -436,9 +444,15 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                     } else {
                         // (resident weights: one box a tap, kc = 1)
                         const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
-                        const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * a.nt * 64u : sB + s * B_STAGE, 512u);
-                        umma_f16(leader, d, ad, bd, idesc, k != 0u ? 1u : 0u);
-                        if (!HALF_K) umma_f16(leader, d, ad + 2u, bd + 2u, idesc, 1u);
+                        const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * KB * a.nt * 64u : sB + s * B_STAGE, 512u);
+                        const uint32_t b_box = a.resident ? a.nt * 4u : B_BOX / 16u;  // (in the descriptors' 16-byte units)
+#pragma unroll
+                        for (uint32_t i = 0; i < KB; ++i) {
+                            if (i != 0u && k * KB + i >= nb) break;
+                            umma_f16(leader, d, ad + i * (A_BOX / 16u), bd + i * b_box, idesc, (k | i) != 0u ? 1u : 0u);
+                            if (!HALF_K)
+                                umma_f16(leader, d, ad + i * (A_BOX / 16u) + 2u, bd + i * b_box + 2u, idesc, 1u);
+                        }
                     }
                     umma_commit(leader, empty(s));
                 }
@@ -1124,6 +1138,7 @@ void conv_run(Net* n, const bf16* x, uint32_t x_stride, uint32_t x_off, uint32_t
     const uint32_t nt = cout <= 32u ? 32u : co_pad % 128u == 0u ? 128u : 64u, n_ntiles = (cout + nt - 1u) / nt;
     // the nine taps' weights stay in the weight stages' room (9 x nt x 64 bytes <= TS x B_STAGE) where the layer
     // reads one 32-channel block into one output tile
+    static_assert(9u * 64u * 64u <= TS * B_STAGE, "a 64-output tile's weights in the weight stages' room");
     uint32_t resident = cin == 32u && n_ntiles == 1u && 9u * nt * 64u <= TS * B_STAGE ? 1u : 0u;
     // A layer of one output tile whose weights fit in shared memory beside three halo stages (up to four 32-channel
     // blocks at 64 outputs, two at 128), on an image at least 128 wide, reads its activations once a tile with the
