@@ -18,7 +18,7 @@ SPREADS = {
 
 
 @pytest.mark.parametrize("spread", list(SPREADS))
-@pytest.mark.parametrize("n", [1, 2, 3, 33, 255, 256, 257, 700, 2049, 5003])
+@pytest.mark.parametrize("n", [1, 2, 3, 10, 11, 33, 127, 128, 129, 256, 257, 700, 2049, 5003])
 def test_the_devices_top_tree_is_the_preps(gpu, n, spread):
     rng = np.random.default_rng(n)
     at = SPREADS[spread](rng, n)

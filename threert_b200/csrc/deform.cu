@@ -24,7 +24,9 @@ constexpr uint32_t MAX_UNITS = 1u << TOP_MAX_DEPTH;
 constexpr uint32_t TOP_BINS = 32u;                  // units.rs:121
 // Top-tree nodes of more units than this are split by a block each, a launch a level (k_top_big); the subtree of a node
 // of at most as many is built by one block in its shared memory (k_top_rest).
-constexpr uint32_t TOP_SMALL = 256u, TOP_WARPS = 32u, TOP_THREADS = TOP_WARPS * 32u;
+// (Subtrees of 128 units build the crowd's 5,002 units in 228 us, of 256 in 236, of 64 in 255: one block's warps are slow
+// through a large subtree, and a launch a level costs 12 us of latency however small its nodes are.)
+constexpr uint32_t TOP_SMALL = 128u, TOP_WARPS = 32u, TOP_THREADS = TOP_WARPS * 32u;
 // Error bits the kernels record.
 constexpr uint32_t E_TREE = 1u, E_DEPTH = 2u, E_ROOT = 4u, E_INDEX = 8u;
 
@@ -311,15 +313,16 @@ __device__ __forceinline__ uint32_t pack_bins(bool valid, float4 c, V3 clo, cons
 // holds split i (bins 0 .. i-1 to the left). The left sides are an inclusive scan over the bins before, the right
 // sides one over the bins from i on (min, max and sums: exact, as the reference's running folds are), each lane then
 // computes the split's cost as build_sah does, and the warp takes the first cheapest in build_sah's order (axis, then
-// split) among the splits that leave both sides non-empty and within `room`. Every lane gets the result.
+// split) among the splits that leave both sides non-empty and within `room`, over the axes ax0 .. ax1 - 1. Every lane gets
+// the result.
 __device__ void sah_sweep(const float (*blo)[3][TOP_BINS], const float (*bhi)[3][TOP_BINS], const uint32_t (*bn)[TOP_BINS],
-                          const bool use[3], uint32_t count, uint32_t room, float& best_cost, uint32_t& best_axis,
-                          uint32_t& best_split, uint32_t& best_left) {
+                          const bool use[3], uint32_t ax0, uint32_t ax1, uint32_t count, uint32_t room, float& best_cost,
+                          uint32_t& best_axis, uint32_t& best_split, uint32_t& best_left) {
     const uint32_t lane = threadIdx.x & 31u;
     const float pinf = __uint_as_float(0x7f800000u);
     float cost_best = pinf;
     uint32_t key_best = 0xffffffffu, left_best = 0;
-    for (uint32_t ax = 0; ax < 3; ++ax) {
+    for (uint32_t ax = ax0; ax < ax1; ++ax) {
         if (!use[ax]) continue;
         // this lane's bin
         float l0 = blo[ax][0][lane], l1 = blo[ax][1][lane], l2 = blo[ax][2][lane];
@@ -398,8 +401,8 @@ struct TopShared {
     uint32_t n[TOP_WARPS][3][TOP_BINS];
     float red[TOP_WARPS][12];
     uint32_t side[TOP_WARPS][2];
-    float cost;
-    uint32_t best[3];
+    float cost[3];
+    uint32_t best[3][2];
     float4 box[2 * TOP_SMALL], centre[TOP_SMALL];
     uint32_t id[TOP_SMALL], order[2][TOP_SMALL];
     uint4 tasks[2][TOP_SMALL];
@@ -490,20 +493,25 @@ __device__ uint32_t split_block(const TopBuild& T, TopShared& S, uint4 task, uin
         }
     }
     __syncthreads();
-    if (w == 0) {
+    // (a warp an axis, then the first cheapest of the three)
+    if (w < 3u) {
         float c;
         uint32_t a, sp, l;
-        sah_sweep(S.lo[0], S.hi[0], S.n[0], use, count, room, c, a, sp, l);
+        sah_sweep(S.lo[0], S.hi[0], S.n[0], use, w, w + 1u, count, room, c, a, sp, l);
         if (lane == 0) {
-            S.cost = c;
-            S.best[0] = a; S.best[1] = sp; S.best[2] = l;
+            S.cost[w] = c;
+            S.best[w][0] = sp;
+            S.best[w][1] = l;
         }
     }
     __syncthreads();
-    const bool binned = finite1(S.cost);
-    const uint32_t best_axis = S.best[0], best_split = S.best[1];
+    uint32_t best_axis = 0u;
+    for (uint32_t ax = 1; ax < 3u; ++ax)
+        if (S.cost[ax] < S.cost[best_axis]) best_axis = ax;
+    const bool binned = finite1(S.cost[best_axis]);
+    const uint32_t best_split = S.best[best_axis][0];
     const uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
-    const uint32_t mid = binned ? S.best[2] : count / 2u;
+    const uint32_t mid = binned ? S.best[best_axis][1] : count / 2u;
     // Stable partition, a block-wide chunk at a time.
     uint32_t nl_run = 0, nr_run = 0;
     for (uint32_t base = start; base < end; base += TOP_THREADS) {
@@ -562,6 +570,51 @@ __global__ void __launch_bounds__(TOP_THREADS) k_top_big(TopBuild T, uint32_t le
     }
 }
 
+// build_sah's choice for a node of at most FEW units (most of a tree's), by a warp without bins: the splits between the
+// same two occupied bins leave the same sides, and the first of them comes right after the lower bin, so there is one
+// to weigh for each unit's bin on each axis: lane ax * FEW + u weighs the split after unit u's bin on axis ax. Sides,
+// costs and order are sah_sweep's.
+constexpr uint32_t FEW = 10u;
+__device__ void few_split(const TopShared& S, const uint32_t* order, uint32_t start, uint32_t count, V3 clo,
+                          const float scale[3], const bool use[3], uint32_t room, float& best_cost, uint32_t& best_axis,
+                          uint32_t& best_split, uint32_t& best_left) {
+    const uint32_t lane = threadIdx.x & 31u, ax = min(lane / FEW, 2u), u = lane - ax * FEW;
+    const float pinf = __uint_as_float(0x7f800000u), ninf = __uint_as_float(0xff800000u);
+    const float axis_lo = comp3(clo, ax), axis_scale = ax == 0u ? scale[0] : ax == 1u ? scale[1] : scale[2];
+    const bool mine = u < count && (ax == 0u ? use[0] : ax == 1u ? use[1] : use[2]);
+    const uint32_t own = bin_of(comp(S.centre[order[start + min(u, count - 1u)]], ax), axis_lo, axis_scale);
+    V3 llo = v3(pinf), lhi = v3(ninf), rlo = llo, rhi = lhi;
+    uint32_t nl = 0u;
+    for (uint32_t j = 0; j < count; ++j) {
+        const uint32_t k = order[start + j];
+        const float4 bl = S.box[2u * k], bh = S.box[2u * k + 1u];
+        const bool left = bin_of(comp(S.centre[k], ax), axis_lo, axis_scale) <= own;
+        if (left) {
+            llo = V3{gmin(llo.x, bl.x), gmin(llo.y, bl.y), gmin(llo.z, bl.z)};
+            lhi = V3{gmax(lhi.x, bh.x), gmax(lhi.y, bh.y), gmax(lhi.z, bh.z)};
+            ++nl;
+        } else {
+            rlo = V3{gmin(rlo.x, bl.x), gmin(rlo.y, bl.y), gmin(rlo.z, bl.z)};
+            rhi = V3{gmax(rhi.x, bh.x), gmax(rhi.y, bh.y), gmax(rhi.z, bh.z)};
+        }
+    }
+    const uint32_t nr = count - nl;
+    float cv = pinf;
+    if (mine && nr != 0u && nl <= room && nr <= room) cv = area3(llo, lhi) * (float)nl + area3(rlo, rhi) * (float)nr;
+    if (!(cv < pinf)) cv = pinf;
+    uint32_t key = cv < pinf ? ax * 32u + own + 1u : 0xffffffffu;
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1) {
+        const float oc = __shfl_xor_sync(~0u, cv, o);
+        const uint32_t ok = __shfl_xor_sync(~0u, key, o), ol = __shfl_xor_sync(~0u, nl, o);
+        if (oc < cv || (oc == cv && ok < key)) { cv = oc; key = ok; nl = ol; }
+    }
+    best_cost = cv;
+    best_axis = key == 0xffffffffu ? 0u : key / 32u;
+    best_split = key == 0xffffffffu ? 0u : key % 32u;
+    best_left = nl;
+}
+
 // The same step for a node of a subtree in shared memory, by a warp: slots order[level & 1][start, end) of the subtree.
 __device__ void split_warp(const TopBuild& T, TopShared& S, uint4 task, uint32_t level) {
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
@@ -601,20 +654,24 @@ __device__ void split_warp(const TopBuild& T, TopShared& S, uint4 task, uint32_t
     const V3 ext = chi - clo;
     const float scale[3] = {(float)TOP_BINS / ext.x, (float)TOP_BINS / ext.y, (float)TOP_BINS / ext.z};
     const bool use[3] = {ext.x > 0.0f, ext.y > 0.0f, ext.z > 0.0f};
-    bins_clear(S.lo[w], S.hi[w], S.n[w], lane, 32u);
-    __syncwarp();
-    for (uint32_t base = start; base < end; base += 32u) {
-        const uint32_t j = base + lane;
-        const bool valid = j < end;
-        const uint32_t k = order[valid ? j : start];
-        bins_add(S.lo[w], S.hi[w], S.n[w], pack_bins(valid, S.centre[k], clo, scale, use), S.box[2u * k], S.box[2u * k + 1u]);
-    }
-    __syncwarp();
-    bins_to_floats(S.lo[w], S.hi[w], lane, 32u);
-    __syncwarp();
     float best_cost = 0.0f;
     uint32_t best_axis = 0, best_split = 0, best_left = 0;
-    sah_sweep(S.lo[w], S.hi[w], S.n[w], use, count, room, best_cost, best_axis, best_split, best_left);
+    if (count <= FEW) {
+        few_split(S, order, start, count, clo, scale, use, room, best_cost, best_axis, best_split, best_left);
+    } else {
+        bins_clear(S.lo[w], S.hi[w], S.n[w], lane, 32u);
+        __syncwarp();
+        for (uint32_t base = start; base < end; base += 32u) {
+            const uint32_t j = base + lane;
+            const bool valid = j < end;
+            const uint32_t k = order[valid ? j : start];
+            bins_add(S.lo[w], S.hi[w], S.n[w], pack_bins(valid, S.centre[k], clo, scale, use), S.box[2u * k], S.box[2u * k + 1u]);
+        }
+        __syncwarp();
+        bins_to_floats(S.lo[w], S.hi[w], lane, 32u);
+        __syncwarp();
+        sah_sweep(S.lo[w], S.hi[w], S.n[w], use, 0u, 3u, count, room, best_cost, best_axis, best_split, best_left);
+    }
     const bool binned = finite1(best_cost);
     const uint32_t med_axis = (ext.x >= ext.y && ext.x >= ext.z) ? 0u : (ext.y >= ext.z ? 1u : 2u);
     const uint32_t mid = binned ? best_left : count / 2u;
@@ -659,7 +716,8 @@ __device__ void split_warp(const TopBuild& T, TopShared& S, uint4 task, uint32_t
 
 // What k_top_big left, a block a subtree: nodes still larger than TOP_SMALL one after another, then each node of at most
 // as many units with everything below it, in shared memory, a level at a time with a barrier between, a warp a node.
-// (Every level of the whole tree as two launches took 19 of them and 0.41 ms for 5,002 units, 5-10 us of latency each.)
+// (Every level of the whole tree as two launches took 38 of them, 5-10 us of latency each: 0.42 ms for 5,002 units, 0.33
+// for 2,002, 0.24 for 302; so built 0.22, 0.18 and 0.10.)
 __global__ void __launch_bounds__(TOP_THREADS) k_top_rest(TopBuild T) {
     extern __shared__ __align__(16) uint8_t top_smem[];
     TopShared& S = *reinterpret_cast<TopShared*>(top_smem);
@@ -976,7 +1034,7 @@ int deform_run(DeformState* st, const SceneBuffers& sb, const uint32_t* P, const
     T.top_first = top;
     T.n_units = n_units;
     // A launch a level while nodes larger than TOP_SMALL are to be expected (halving, and three levels more for uneven
-    // splits; larger nodes below them are k_top_rest's too).
+    // splits: without them 2,002 units took 0.26 ms; larger nodes below are k_top_rest's too).
     T.big_levels = 0u;
     if (n_units > TOP_SMALL) {
         T.big_levels = 3u;
