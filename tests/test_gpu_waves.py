@@ -70,3 +70,26 @@ def test_a_scene_of_four_suns_and_one_of_no_lights(gpu):
         P = prep.prepare(desc)
         S = gpu.upload(P)
         same(S, sized(P, 61, 43), 3, 0, N.TRT_RENDER_SORT_RAYS)
+
+
+def many_units():
+    """264 units turned, scaled unevenly, mirrored or moved alone, some that cast no shadow."""
+    d = scaled_units_scene()
+    rng = np.random.default_rng(11)
+    for k in range(240):
+        w = scenes.translate_rot_y(rng.uniform(-9, 9, 3), rng.uniform(0, 6.28), rng.uniform(-1.5, 1.5, 3))
+        if k % 3 == 0:
+            w = scenes.translate_rot_y(rng.uniform(-9, 9, 3))
+        d.instances.append(prep.Instance(k % 2, [k % 2], w, object=24 + k, cast_shadow=k % 4 != 0))
+    return d
+
+
+# Waves around the sizes from which the walks run as streams of rays (131,072 paths for shadow rays, 262,144 for the
+# others), and of two halves; the counted render walks ray by ray.
+@pytest.mark.parametrize("w,h,spp", [(359, 362, 1), (363, 363, 1), (515, 509, 1), (1030, 514, 1), (201, 163, 9)])
+@pytest.mark.parametrize("make", [many_units, lambda: small_city(n_objects=260), lambda: small_crowd(260).desc])
+def test_streams_of_rays_hit_what_single_walks_hit(gpu, make, w, h, spp):
+    P = prep.prepare(make())
+    assert int(P.params[71]) >= 256
+    S = gpu.upload(P)
+    same(S, sized(P, w, h), spp, N.TRT_RENDER_DEPTH, N.TRT_RENDER_DEPTH | N.TRT_RENDER_COUNT)

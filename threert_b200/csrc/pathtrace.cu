@@ -34,6 +34,9 @@
 #ifndef TRT_BLOCKS_SHADOW
 #define TRT_BLOCKS_SHADOW 8
 #endif
+#ifndef TRT_BLOCKS_SHADOW_STREAM
+#define TRT_BLOCKS_SHADOW_STREAM 9
+#endif
 #ifndef TRT_BLOCKS_SHADE
 #define TRT_BLOCKS_SHADE 8
 #endif
@@ -266,6 +269,33 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend(const Job* __
     warp_add64(&Q.totals[T_GUARD], guard_trips);
 }
 
+// The closest-hit rays past the first depth as a stream (trace_stream). A ray's record says "no hit" from its start on
+// and is written again at each nearer hit: kept in registers until the ray ends, it took the walk past 64 of them.
+__global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend_stream(const Job one, PathBufs B, Queues Q, uint32_t depth,
+                                                                         const uint32_t* __restrict__ queue) {
+    uint32_t* cnt = Q.cnt + depth * CNT_STRIDE;
+    const uint32_t n = *(volatile uint32_t*)&cnt[0];
+    unsigned long long guard_trips = 0;
+    trace_stream(
+        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, &cnt[2], n,
+        [&](uint32_t i, uint32_t& ray, V3& o, V3& d, float& t, uint32_t& mode) {
+            ray = queue[i];
+            o = xyz(B.o[ray]);
+            d = xyz(B.d[ray]);
+            t = INF;
+            mode = TRACE_CLOSEST;
+            Q.hit_a[ray] = make_float4(INF, 0.0f, 0.0f, bf(MISS));
+            Q.hit_b[ray] = make_uint2(NO_INST, 0u);
+        },
+        [&](uint32_t& ray, const float3& x, uint32_t tri, uint32_t rec) {
+            Q.hit_a[ray] = make_float4(x.x, x.y, x.z, bf(tri));
+            Q.hit_b[ray] = make_uint2(rec, bu(__ldg(one.wk.S.leaves + 3ull * tri).w));
+            return false;
+        },
+        [&](uint32_t) {}, guard_trips);
+    warp_add64(&Q.totals[T_GUARD], guard_trips);
+}
+
 // The j-th shadow ray of a depth, counting the classes' regions one after another.
 __device__ __forceinline__ uint32_t shadow_slot(const Queues& Q, uint32_t j, uint32_t n0, uint32_t n1) {
     return j < n0 ? Q.class_base[0] + j : (j < n0 + n1 ? Q.class_base[1] + (j - n0) : Q.class_base[2] + (j - n0 - n1));
@@ -302,6 +332,34 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADOW) k_shadow(const Job* __
         warp_add64(&Q.totals[T_S_TRIS], wc.tris);
         warp_add64(&Q.totals[T_S_UNITS], wc.units);
     }
+    warp_add64(&Q.totals[T_GUARD], guard_trips);
+}
+
+// The shadow rays as a stream (trace_stream). (Nine blocks an SM: a shadow ray keeps no hit, and 56 registers hold the
+// walk; the town 15.43 ms with eight, 15.26 with nine, 15.99 with ten, which spill.)
+__global__ void __launch_bounds__(128, TRT_BLOCKS_SHADOW_STREAM) k_shadow_stream(const Job one, PathBufs B, Queues Q, uint32_t depth,
+                                                                                const uint32_t* __restrict__ perm) {
+    uint32_t* cnt = Q.cnt + depth * CNT_STRIDE;
+    const uint32_t n0 = min(*(volatile uint32_t*)&cnt[4], Q.class_cap[0]);
+    const uint32_t n1 = min(*(volatile uint32_t*)&cnt[5], Q.class_cap[1]);
+    const uint32_t n2 = min(*(volatile uint32_t*)&cnt[6], Q.class_cap[2]);
+    unsigned long long guard_trips = 0;
+    trace_stream(
+        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, &cnt[3], n0 + n1 + n2,
+        [&](uint32_t j, uint32_t& ray, V3& o, V3& d, float& t, uint32_t& mode) {
+            const uint32_t i = perm ? perm[j] : shadow_slot(Q, j, n0, n1);
+            ray = Q.sp[i];
+            const float4 a = Q.so[i], b = Q.sd[i];
+            o = xyz(a);
+            d = xyz(b);
+            t = a.w;
+            mode = bu(b.w);
+        },
+        [&](uint32_t& ray, const float3&, uint32_t, uint32_t) {
+            ray = NO_RAY;
+            return true;
+        },
+        [&](uint32_t ray) { atomicOr(&B.vis[ray >> 3], 1u << (ray & 7u)); }, guard_trips);
     warp_add64(&Q.totals[T_GUARD], guard_trips);
 }
 
@@ -1128,7 +1186,8 @@ std::pair<cudaEvent_t, cudaEvent_t> take_events(trt_scene* s) {
 // the driver may give a block would hold few of their blocks (the wide walk fell from 912-944 to 336 Mrays/s).
 void prefer_l1() {
     const void* fns[] = {(const void*)k_extend<false, false, false>, (const void*)k_extend<true, false, false>,
-                         (const void*)k_extend<false, false, true>,  (const void*)k_shadow<false, false, false>,
+                         (const void*)k_extend<false, false, true>,  (const void*)k_extend_stream,
+                         (const void*)k_shadow_stream, (const void*)k_shadow<false, false, false>,
                          (const void*)k_shadow<true, false, false>,  (const void*)k_shadow<false, false, true>,
                          (const void*)k_shade<false>,                (const void*)k_shade<true>};
     for (const void* f : fns) cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
@@ -1157,10 +1216,11 @@ void launch_sort(trt_scene* s, Wave& W, const uint32_t* in, uint32_t* out, uint3
 }
 
 // A wave's launches on a stream pair (st, aux): ray generation, then each depth's walks, sorts, shading and resolve,
-// then the accumulation. g_ext / g_sha: the persistent walks' grids.
+// then the accumulation.
+struct WalkGrids { int extend, shadow, extend_stream, shadow_stream; };  // (the persistent walks')
 template <bool COUNT, bool WIDE>
 void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t last, uint32_t flags_eff,
-                 cudaStream_t st, cudaStream_t aux, cudaEvent_t fork_ev, cudaEvent_t join_ev, int g_ext, int g_sha) {
+                 cudaStream_t st, cudaStream_t aux, cudaEvent_t fork_ev, cudaEvent_t join_ev, const WalkGrids& grids) {
     const bool sort_rays = (flags_eff & TRT_RENDER_SORT_RAYS) != 0;
     const bool sort_hits = (flags_eff & TRT_RENDER_UNSORTED_HITS) == 0;
     const bool sort_shadows = (flags_eff & TRT_RENDER_SORT_SHADOWS) != 0;
@@ -1174,6 +1234,24 @@ void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t las
     // depth's shading wrote and write apart (visibility bits; hit records), so their tails overlap. (Not with the ray
     // sort, whose output buffer is the previous depth's shading order, which that depth's resolve still reads.)
     const bool overlap = !sort_rays;
+    // The walks run as streams of rays where a wave has the rays to refill its warps with and rays differ enough in what
+    // they meet: among many units, past the first depth's closest hits (a camera's neighbours: 25 of 32 lanes without).
+    // Both ways, without -> as streams, 4 spp at 512 x 512 unless said: the city (4,002 units, 720p, 1 spp) 4.46 -> 4.26 ms;
+    // 1,002 units 4.12-5.12 -> 3.86-4.65; 502, 5.34-6.16 -> 4.99-5.63; 302, 3.56-4.83 -> 3.43-4.43, spread out (most of
+    // the view ground and sky) 2.67-3.75 -> 2.65-3.58; 122, 3.24 -> 3.49; 12, 3.12 -> 3.40; the Cornell box 1.70 -> 1.72. By
+    // size, the town of 302 units at 1 spp: 102,400 paths 0.92 -> 0.93 ms, 147,456 1.075 -> 1.070, 200,704 1.31 -> 1.29,
+    // 262,144 1.58 -> 1.53 (the closest hits' share of it nothing), 409,600 2.21 -> 2.13 (1.5 % of it).
+    constexpr uint32_t STREAM_MIN_UNITS = 256u, STREAM_MIN_SHADOW = 131072u, STREAM_MIN_EXTEND = 262144u;
+    const bool many = !COUNT && !WIDE && job.wk.n_units >= STREAM_MIN_UNITS;
+    const bool ext_stream = many && n >= STREAM_MIN_EXTEND, sha_stream = many && n >= STREAM_MIN_SHADOW;
+    auto extend = [&](uint32_t depth, const uint32_t* queue) {
+        if (ext_stream && depth > 0u) k_extend_stream<<<grids.extend_stream, blk, 0, st>>>(job, W.B, W.Q, depth, queue);
+        else k_extend<COUNT, WIDE, false><<<grids.extend, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth, queue);
+    };
+    auto shadow = [&](uint32_t depth, const uint32_t* perm, cudaStream_t on) {
+        if (sha_stream) k_shadow_stream<<<grids.shadow_stream, blk, 0, on>>>(job, W.B, W.Q, depth, perm);
+        else k_shadow<COUNT, WIDE, false><<<grids.shadow, blk, 0, on>>>(W.jobs, job, W.B, W.Q, depth, perm);
+    };
     k_put_job<<<1, 128, 0, st>>>(job, W.jobs, 0u);
     k_raygen<<<(n + blk - 1) / blk, blk, 0, st>>>(W.jobs, 1u, W.B, W.Q, n, nullptr);
     s->launches += 2;
@@ -1190,7 +1268,7 @@ void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t las
         }
         if (!overlap || depth == 0u) {  // (past depth 0 with the overlap, launched beside the last shadow walk)
             mark(s->ev_extend, true, st);
-            k_extend<COUNT, WIDE, false><<<g_ext, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth, ext_q);
+            extend(depth, ext_q);
             mark(s->ev_extend, false, st);
         }
         uint32_t* shade_q = ext_q;
@@ -1214,18 +1292,18 @@ void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t las
             cudaEventRecord(fork_ev, st);
             cudaStreamWaitEvent(aux, fork_ev, 0);
             mark(s->ev_shadow, true, aux);
-            k_shadow<COUNT, WIDE, false><<<g_sha, blk, 0, aux>>>(W.jobs, job, W.B, W.Q, depth, perm);
+            shadow(depth, perm, aux);
             mark(s->ev_shadow, false, aux);
             if (depth < last) {
                 mark(s->ev_extend, true, st);
-                k_extend<COUNT, WIDE, false><<<g_ext, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth + 1u, next);
+                extend(depth + 1u, next);
                 mark(s->ev_extend, false, st);
             }
             cudaEventRecord(join_ev, aux);
             cudaStreamWaitEvent(st, join_ev, 0);
         } else {
             mark(s->ev_shadow, true, st);
-            k_shadow<COUNT, WIDE, false><<<g_sha, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth, perm);
+            shadow(depth, perm, st);
             mark(s->ev_shadow, false, st);
         }
         k_resolve<false><<<(n + blk - 1) / blk, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth, shade_q);
@@ -1274,8 +1352,10 @@ int render_waves(trt_scene* s, const Params& P, uint32_t first_sample, uint32_t 
                            (uint64_t)n_idx * K >= TRT_SORT_HITS_MIN_PATHS;
     const uint32_t flags_eff = (flags & ~TRT_RENDER_UNSORTED_HITS) | (sort_hits ? 0u : TRT_RENDER_UNSORTED_HITS);
     const int blk = 128;
-    int g_ext = grid_for((const void*)k_extend<COUNT, WIDE, false>, blk, c->sm_count);
-    int g_sha = grid_for((const void*)k_shadow<COUNT, WIDE, false>, blk, c->sm_count);
+    const WalkGrids grids{grid_for((const void*)k_extend<COUNT, WIDE, false>, blk, c->sm_count),
+                          grid_for((const void*)k_shadow<COUNT, WIDE, false>, blk, c->sm_count),
+                          grid_for((const void*)k_extend_stream, blk, c->sm_count),
+                          grid_for((const void*)k_shadow_stream, blk, c->sm_count)};
     std::vector<uint32_t> host_cnt(MAX_DEPTH * CNT_STRIDE + CNT_STRIDE, 0);
     // A wave that the GPU holds in one round of blocks takes k_paths (the counted, the wide and the profiled walks and the
     // optional sorts are the wavefront's).
@@ -1305,15 +1385,15 @@ int render_waves(trt_scene* s, const Params& P, uint32_t first_sample, uint32_t 
             TRT_CUDA(c, cudaMemcpyAsync(s->wave2.Q.cnt, host_cnt.data(), host_cnt.size() * 4, cudaMemcpyHostToDevice,
                                         c->half_stream));
             launch_wave<COUNT, WIDE>(s, s->wave, job_a, n_idx_a * k, last, flags_eff, st, c->aux_stream, c->fork_ev,
-                                     c->join_ev, g_ext, g_sha);
+                                     c->join_ev, grids);
             launch_wave<COUNT, WIDE>(s, s->wave2, job_b, n_idx_b * k, last, flags_eff, c->half_stream, c->half_aux,
-                                     c->half_fork2, c->half_join2, g_ext, g_sha);
+                                     c->half_fork2, c->half_join2, grids);
             k_tally<<<1, 32, 0, c->half_stream>>>(s->wave2.Q, last + 1, 0u, nullptr);
             TRT_CUDA(c, cudaEventRecord(c->half_join, c->half_stream));
             TRT_CUDA(c, cudaStreamWaitEvent(st, c->half_join, 0));
         } else {
             launch_wave<COUNT, WIDE>(s, s->wave, job_a, n_idx_a * k, last, flags_eff, st, c->aux_stream, c->fork_ev,
-                                     c->join_ev, g_ext, g_sha);
+                                     c->join_ev, grids);
         }
         k_tally<<<1, 32, 0, st>>>(s->wave.Q, last + 1, w * h * k, nullptr);
         s->launches += halves ? 2 : 1;

@@ -195,4 +195,169 @@ __device__ __forceinline__ Hit trace_binary(const DScene& S, const Sections& X, 
     return hit;
 }
 
+// The same walk over a stream of rays, for waves whose rays go many ways through deep trees: a warp keeps its lanes in
+// work. trace_binary's lanes wait for each other twice: those at a leaf until the last of the warp has left the inner
+// loop, and those whose ray has ended until the warp's longest ray has; 7-9 of 32 lanes are left a warp instruction.
+// Here the warp runs, each round, the phase that most of its lanes wait for (a few interior steps, or entering a
+// unit, or a leaf's triangles), and when STREAM_REFILL lanes are idle these take the next rays together. Neither half
+// gives anything alone (refilling trace_binary's lanes made it 6 % slower, the vote without refills 0 %), and a round
+// for both leaf kinds at once or an inner loop that runs until few lanes are left in it were slower too (town below:
+// 15.95-16.6 ms). A town's second depth (640 x 512, 1 spp): 7.6 -> 13.4 lanes and 175 -> 140 M warp instructions for its
+// shadow rays, 8.8 -> 13.7 and 101 -> 92 M closest; the more rays a warp gets, the better (34 of them, no gain; 400,
+// 30 % by a count of the phases), and short walks lose (the rounds cost a quarter more thread instructions): the caller
+// chooses. The town at 512 x 512, 16 spp, 16.85 -> 15.26 ms; the city frame (720p, 1 spp)
+// 4.46 -> 4.25. STREAM_STEPS / STREAM_REFILL 3 / 12: 15.69, 4 / 16: 15.63, 6 / 16: 15.66, 2 / 8: 16.14 (before the other
+// ballots were put off).
+//
+// n rays, handed out by `counter`. load(i, ray, o, d, t, mode) fetches the i-th and names it; hit(ray, x, tri, rec)
+// takes a nearer hit (t, u, v) and says whether the ray is done; done(ray) ends one, unless hit() set it to NO_RAY. What a
+// ray meets, and in which order, is trace_binary's, and so are the checks of every index and WALK_GUARD (a ray each).
+constexpr uint32_t NO_RAY = 0xffffffffu;
+constexpr int STREAM_STEPS = 4, STREAM_REFILL = 16;
+template <class Load, class Take, class Done>
+__device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instances, uint32_t top, uint32_t n_units,
+                                             uint32_t* counter, uint32_t n, Load load, Take hit, Done done,
+                                             unsigned long long& guard_trips) {
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr uint32_t IDLE = 0xffffffffu, NO_BASE = 0xffffffffu;
+    const uint32_t last_node = (uint32_t)min((unsigned long long)S.n_nodes - 1ull, 0xffffffffull);
+    const uint32_t tris_end = (uint32_t)min((unsigned long long)S.n_tris, 0xffffffffull);
+    const uint32_t tables_end = (uint32_t)min((unsigned long long)S.n_table_vec4, 0xffffffffull);
+    const uint32_t lane = threadIdx.x & 31u;
+    V3 o{0.0f, 0.0f, 0.0f}, d = o, inv_d = o, ro = o, rd = o, rinv = o;
+    float t = 0.0f;
+    // `count` IDLE: the lane has no ray, or its ray has ended (`ray`: it is not handed on yet).
+    uint32_t ray = NO_RAY, mode = 0, at = 0, count = IDLE, off = 0, first = 0, rec = NO_INST, iter = 0;
+    uint32_t stack[64];
+    uint32_t sp = 0, base = NO_BASE;
+    auto trip = [&]() { guard_trips++; count = IDLE; };
+    auto pop = [&]() {
+        if (sp == base) {
+            rec = NO_INST;
+            base = NO_BASE;
+            ro = o; rd = d; rinv = inv_d;
+            off = top;
+        }
+        if (sp == 0) { count = IDLE; return; }
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * stack[--sp]);
+        at = __ldg(q + 3);
+        count = __ldg(q + 7);
+        if (count == 0) at += off;
+    };
+    bool more = n != 0;
+    for (;;) {
+        const unsigned busy = __ballot_sync(ALL, count != IDLE);
+        const int n_busy = __popc(busy);
+        if (more && n_busy <= 32 - STREAM_REFILL) {
+            const uint32_t want = 32u - (uint32_t)n_busy;
+            uint32_t b = 0;
+            if (lane == 0) b = atomicAdd(counter, want);
+            b = __shfl_sync(ALL, b, 0);
+            more = b < n && n - b > want;
+            if (count == IDLE) {
+                if (ray != NO_RAY) done(ray);
+                ray = NO_RAY;
+                const uint32_t i = b + (uint32_t)__popc(~busy & ((1u << lane) - 1u));
+                if (b < n && i < n) {
+                    load(i, ray, o, d, t, mode);
+                    inv_d = safe_inv(d);
+                    ro = o; rd = d; rinv = inv_d;
+                    off = top; rec = NO_INST; iter = 0;
+                    sp = 0; base = NO_BASE;
+                    if (n_units != 0) {
+                        if (top >= S.n_nodes) trip();
+                        else {
+                            const uint4* q = S.nodes + 2ull * top;
+                            const uint4 x = __ldg(q), y = __ldg(q + 1);
+                            float tn;
+                            if (box_hit(o, inv_d, x, y, t, tn)) {
+                                count = y.w;
+                                at = count == 0 ? x.w + top : x.w;
+                            }
+                        }
+                    }
+                }
+            }
+            continue;
+        }
+        if (busy == 0) break;
+        // The lanes at an interior node, at a unit, at triangles (the last two counted only when they could be more).
+        const int n_inner = __popc(__ballot_sync(ALL, count == 0)), n_leaf = n_busy - n_inner;
+        unsigned units = 0;
+        if (n_inner < n_leaf) units = __ballot_sync(ALL, count - 1u < IDLE - 1u && rec == NO_INST);
+        const int n_unit = __popc(units), n_tri = n_leaf - n_unit;
+        if (n_inner >= n_leaf || n_inner >= max(n_unit, n_tri)) {
+#pragma unroll
+            for (int step = 0; step < STREAM_STEPS; ++step) {
+                if (count == 0) {
+                    if (iter++ >= WALK_GUARD || at >= last_node) trip();
+                    else {
+                        const uint4* q = S.nodes + 2ull * at;
+                        const uint4 l0 = __ldg(q), l1 = __ldg(q + 1), r0 = __ldg(q + 2), r1 = __ldg(q + 3);
+                        float tl, tr;
+                        const bool hl = box_hit(ro, rinv, l0, l1, t, tl), hr = box_hit(ro, rinv, r0, r1, t, tr);
+                        if (hl || hr) {
+                            const bool swap = hr && (!hl || tr < tl);
+                            const uint32_t link = swap ? r0.w : l0.w;
+                            count = swap ? r1.w : l1.w;
+                            if (hl && hr && sp < 64) stack[sp++] = swap ? at : at + 1u;
+                            at = count == 0 ? link + off : link;
+                        } else {
+                            pop();
+                        }
+                    }
+                }
+            }
+        } else if (n_unit >= n_tri) {
+            if (units >> lane & 1u) {
+                const uint32_t b = t_instances + at * 10u;
+                if (iter++ >= WALK_GUARD || tables_end < 10u || b > tables_end - 10u) trip();
+                else {
+                    const uint4* u = S.tables + b;
+                    const float4* uf = reinterpret_cast<const float4*>(u);
+                    const float4 n1 = __ldg(uf + 4);
+                    const uint32_t ubits = bu(n1.w);
+                    if (mode != TRACE_SHADOW || (ubits & UNIT_SHADOW) != 0) {
+                        const float4 n0 = __ldg(uf + 3), n2 = __ldg(uf + 5);
+                        rec = at;
+                        ro = o - V3{__ldg(&uf[0].w), __ldg(&uf[1].w), __ldg(&uf[2].w)};
+                        first = __ldg(&u[6].x);
+                        if ((ubits & UNIT_SHIFTED) == 0) {
+                            ro = proc_dir(n0, n1, n2, ro);
+                            rd = proc_dir(n0, n1, n2, d);
+                            rinv = safe_inv(rd);
+                        }
+                        off = bu(n0.w);
+                        base = sp;
+                        if (off > last_node) trip();
+                        else {
+                            const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * off);
+                            at = __ldg(q + 3);
+                            count = __ldg(q + 7);
+                            if (count == 0) at += off;
+                        }
+                    } else {
+                        pop();
+                    }
+                }
+            }
+        } else if (count - 1u < IDLE - 1u && rec != NO_INST) {
+            bool ended = iter++ >= WALK_GUARD;
+            if (ended) trip();
+            for (uint32_t k = 0; !ended && k < count; ++k) {
+                const uint32_t ti = first + at + k;
+                if (ti >= tris_end) { trip(); ended = true; break; }
+                const float3 x = intersect_tri(S, ro, rd, ti, t);
+                if (x.x < t) {
+                    t = x.x;
+                    if (hit(ray, x, ti, rec)) { count = IDLE; ended = true; break; }
+                }
+            }
+            if (!ended) pop();
+        }
+        __syncwarp();
+    }
+    if (ray != NO_RAY) done(ray);
+}
+
 }  // namespace trt
