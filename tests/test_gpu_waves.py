@@ -6,6 +6,7 @@ import pytest
 
 from threert_b200 import _native as N
 from threert_b200 import prep, scenes
+from threert_b200.serve import Request, Server, run_stream
 from util import scaled_units_scene, small_city, small_crowd
 
 pytestmark = pytest.mark.gpu
@@ -93,3 +94,21 @@ def test_streams_of_rays_hit_what_single_walks_hit(gpu, make, w, h, spp):
     assert int(P.params[71]) >= 256
     S = gpu.upload(P)
     same(S, sized(P, w, h), spp, N.TRT_RENDER_DEPTH, N.TRT_RENDER_DEPTH | N.TRT_RENDER_COUNT)
+
+
+# The server's steps of several scenes, of the size classes 65,536 (ray by ray), 131,072 (the shadow rays as a stream) and
+# 524,288 (both, and the hits sorted): each request's image is its own render's.
+@pytest.mark.parametrize("side,spp", [(60, 3), (91, 3), (181, 3)])
+def test_a_servers_streams_of_several_scenes_rays(gpu, side, spp):
+    Ps = [prep.prepare(d) for d in (scenes.cornell(16, 16), small_city(), many_units())]
+    S = [gpu.upload(P) for P in Ps]
+    reqs = [Request(k % 3, sized(Ps[k % 3], side + 2 * k, side - k), spp) for k in range(4)]
+    srv = Server(gpu, wave_slots=1 << 20)
+    try:
+        res = run_stream(srv, S, reqs, rate=0.0)
+    finally:
+        srv.close()
+    assert res["failed"] == 0
+    for r in reqs:
+        alone, _ = S[r.scene].render_raw(r.params, r.spp)
+        assert np.array_equal(r.accum.view(np.uint32), alone.view(np.uint32))

@@ -20,6 +20,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "deform.h"
@@ -269,17 +270,47 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend(const Job* __
     warp_add64(&Q.totals[T_GUARD], guard_trips);
 }
 
+// Where a stream's rays find their scene: the one job's, from the kernel's constant bank; or, in a step of several
+// requests, the ray's job's, of which the walk's hot values are kept in registers and the rest is read from the table.
+struct OneScene {
+    static constexpr bool ON = false;
+    __device__ __forceinline__ void bind(const Job*) {}
+    __device__ __forceinline__ const DScene& scene(const DScene& one) const { return one; }
+    __device__ __forceinline__ uint32_t units() const { return 0; }
+    __device__ __forceinline__ uint32_t instances() const { return 0; }
+};
+struct LaneScene {
+    static constexpr bool ON = true;
+    const Job* J = nullptr;
+    const uint4* nodes = nullptr;
+    uint32_t last = 0;
+    __device__ __forceinline__ void bind(const Job* j) {
+        J = j;
+        nodes = j->wk.S.nodes;
+        last = end32(j->wk.S.n_nodes - 1ull);
+    }
+    __device__ __forceinline__ const DScene& scene(const DScene&) const { return J->wk.S; }
+    __device__ __forceinline__ uint32_t top() const { return J->wk.top; }
+    __device__ __forceinline__ uint32_t units() const { return J->wk.n_units; }
+    __device__ __forceinline__ uint32_t instances() const { return Sections(J->P).t_instances; }
+};
+template <bool MULTI> using StreamScene = std::conditional_t<MULTI, LaneScene, OneScene>;
+
 // The closest-hit rays past the first depth as a stream (trace_stream). A ray's record says "no hit" from its start on
 // and is written again at each nearer hit: kept in registers until the ray ends, it took the walk past 64 of them.
+template <bool MULTI>
 __global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend_stream(const Job one, PathBufs B, Queues Q, uint32_t depth,
-                                                                         const uint32_t* __restrict__ queue) {
+                                                                         const uint32_t* __restrict__ queue,
+                                                                         const Job* __restrict__ jobs) {
     uint32_t* cnt = Q.cnt + depth * CNT_STRIDE;
     const uint32_t n = *(volatile uint32_t*)&cnt[0];
     unsigned long long guard_trips = 0;
+    StreamScene<MULTI> view;
     trace_stream(
-        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, &cnt[2], n,
+        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, view, &cnt[2], n,
         [&](uint32_t i, uint32_t& ray, V3& o, V3& d, float& t, uint32_t& mode) {
             ray = queue[i];
+            if constexpr (MULTI) view.bind(jobs + B.job[ray]);
             o = xyz(B.o[ray]);
             d = xyz(B.d[ray]);
             t = INF;
@@ -289,7 +320,7 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_EXTEND) k_extend_stream(const 
         },
         [&](uint32_t& ray, const float3& x, uint32_t tri, uint32_t rec) {
             Q.hit_a[ray] = make_float4(x.x, x.y, x.z, bf(tri));
-            Q.hit_b[ray] = make_uint2(rec, bu(__ldg(one.wk.S.leaves + 3ull * tri).w));
+            Q.hit_b[ray] = make_uint2(rec, bu(__ldg((MULTI ? view.scene(one.wk.S).leaves : one.wk.S.leaves) + 3ull * tri).w));
             return false;
         },
         [&](uint32_t) {}, guard_trips);
@@ -337,18 +368,22 @@ __global__ void __launch_bounds__(128, TRT_BLOCKS_SHADOW) k_shadow(const Job* __
 
 // The shadow rays as a stream (trace_stream). (Nine blocks an SM: a shadow ray keeps no hit, and 56 registers hold the
 // walk; the town 15.43 ms with eight, 15.26 with nine, 15.99 with ten, which spill.)
-__global__ void __launch_bounds__(128, TRT_BLOCKS_SHADOW_STREAM) k_shadow_stream(const Job one, PathBufs B, Queues Q, uint32_t depth,
-                                                                                const uint32_t* __restrict__ perm) {
+template <bool MULTI>
+__global__ void __launch_bounds__(128, MULTI ? TRT_BLOCKS_SHADOW : TRT_BLOCKS_SHADOW_STREAM)
+    k_shadow_stream(const Job one, PathBufs B, Queues Q, uint32_t depth, const uint32_t* __restrict__ perm,
+                    const Job* __restrict__ jobs) {
     uint32_t* cnt = Q.cnt + depth * CNT_STRIDE;
     const uint32_t n0 = min(*(volatile uint32_t*)&cnt[4], Q.class_cap[0]);
     const uint32_t n1 = min(*(volatile uint32_t*)&cnt[5], Q.class_cap[1]);
     const uint32_t n2 = min(*(volatile uint32_t*)&cnt[6], Q.class_cap[2]);
     unsigned long long guard_trips = 0;
+    StreamScene<MULTI> view;
     trace_stream(
-        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, &cnt[3], n0 + n1 + n2,
+        one.wk.S, Sections(one.P).t_instances, one.wk.top, one.wk.n_units, view, &cnt[3], n0 + n1 + n2,
         [&](uint32_t j, uint32_t& ray, V3& o, V3& d, float& t, uint32_t& mode) {
             const uint32_t i = perm ? perm[j] : shadow_slot(Q, j, n0, n1);
             ray = Q.sp[i];
+            if constexpr (MULTI) view.bind(jobs + B.job[ray >> 3]);
             const float4 a = Q.so[i], b = Q.sd[i];
             o = xyz(a);
             d = xyz(b);
@@ -1186,8 +1221,9 @@ std::pair<cudaEvent_t, cudaEvent_t> take_events(trt_scene* s) {
 // the driver may give a block would hold few of their blocks (the wide walk fell from 912-944 to 336 Mrays/s).
 void prefer_l1() {
     const void* fns[] = {(const void*)k_extend<false, false, false>, (const void*)k_extend<true, false, false>,
-                         (const void*)k_extend<false, false, true>,  (const void*)k_extend_stream,
-                         (const void*)k_shadow_stream, (const void*)k_shadow<false, false, false>,
+                         (const void*)k_extend<false, false, true>,  (const void*)k_extend_stream<false>,
+                         (const void*)k_extend_stream<true>,  (const void*)k_shadow_stream<true>,
+                         (const void*)k_shadow_stream<false>, (const void*)k_shadow<false, false, false>,
                          (const void*)k_shadow<true, false, false>,  (const void*)k_shadow<false, false, true>,
                          (const void*)k_shade<false>,                (const void*)k_shade<true>};
     for (const void* f : fns) cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
@@ -1217,6 +1253,8 @@ void launch_sort(trt_scene* s, Wave& W, const uint32_t* in, uint32_t* out, uint3
 
 // A wave's launches on a stream pair (st, aux): ray generation, then each depth's walks, sorts, shading and resolve,
 // then the accumulation.
+// What the walks run from as streams of rays (the reasons and figures: launch_wave).
+constexpr uint32_t STREAM_MIN_UNITS = 256u, STREAM_MIN_SHADOW = 131072u, STREAM_MIN_EXTEND = 262144u;
 struct WalkGrids { int extend, shadow, extend_stream, shadow_stream; };  // (the persistent walks')
 template <bool COUNT, bool WIDE>
 void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t last, uint32_t flags_eff,
@@ -1241,15 +1279,14 @@ void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t las
     // the view ground and sky) 2.67-3.75 -> 2.65-3.58; 122, 3.24 -> 3.49; 12, 3.12 -> 3.40; the Cornell box 1.70 -> 1.72. By
     // size, the town of 302 units at 1 spp: 102,400 paths 0.92 -> 0.93 ms, 147,456 1.075 -> 1.070, 200,704 1.31 -> 1.29,
     // 262,144 1.58 -> 1.53 (the closest hits' share of it nothing), 409,600 2.21 -> 2.13 (1.5 % of it).
-    constexpr uint32_t STREAM_MIN_UNITS = 256u, STREAM_MIN_SHADOW = 131072u, STREAM_MIN_EXTEND = 262144u;
     const bool many = !COUNT && !WIDE && job.wk.n_units >= STREAM_MIN_UNITS;
     const bool ext_stream = many && n >= STREAM_MIN_EXTEND, sha_stream = many && n >= STREAM_MIN_SHADOW;
     auto extend = [&](uint32_t depth, const uint32_t* queue) {
-        if (ext_stream && depth > 0u) k_extend_stream<<<grids.extend_stream, blk, 0, st>>>(job, W.B, W.Q, depth, queue);
+        if (ext_stream && depth > 0u) k_extend_stream<false><<<grids.extend_stream, blk, 0, st>>>(job, W.B, W.Q, depth, queue, nullptr);
         else k_extend<COUNT, WIDE, false><<<grids.extend, blk, 0, st>>>(W.jobs, job, W.B, W.Q, depth, queue);
     };
     auto shadow = [&](uint32_t depth, const uint32_t* perm, cudaStream_t on) {
-        if (sha_stream) k_shadow_stream<<<grids.shadow_stream, blk, 0, on>>>(job, W.B, W.Q, depth, perm);
+        if (sha_stream) k_shadow_stream<false><<<grids.shadow_stream, blk, 0, on>>>(job, W.B, W.Q, depth, perm, nullptr);
         else k_shadow<COUNT, WIDE, false><<<grids.shadow, blk, 0, on>>>(W.jobs, job, W.B, W.Q, depth, perm);
     };
     k_put_job<<<1, 128, 0, st>>>(job, W.jobs, 0u);
@@ -1354,8 +1391,8 @@ int render_waves(trt_scene* s, const Params& P, uint32_t first_sample, uint32_t 
     const int blk = 128;
     const WalkGrids grids{grid_for((const void*)k_extend<COUNT, WIDE, false>, blk, c->sm_count),
                           grid_for((const void*)k_shadow<COUNT, WIDE, false>, blk, c->sm_count),
-                          grid_for((const void*)k_extend_stream, blk, c->sm_count),
-                          grid_for((const void*)k_shadow_stream, blk, c->sm_count)};
+                          grid_for((const void*)k_extend_stream<false>, blk, c->sm_count),
+                          grid_for((const void*)k_shadow_stream<false>, blk, c->sm_count)};
     std::vector<uint32_t> host_cnt(MAX_DEPTH * CNT_STRIDE + CNT_STRIDE, 0);
     // A wave that the GPU holds in one round of blocks takes k_paths (the counted, the wide and the profiled walks and the
     // optional sorts are the wavefront's).

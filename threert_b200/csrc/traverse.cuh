@@ -195,6 +195,8 @@ __device__ __forceinline__ Hit trace_binary(const DScene& S, const Sections& X, 
     return hit;
 }
 
+__device__ __forceinline__ uint32_t end32(unsigned long long n) { return (uint32_t)min(n, 0xffffffffull); }
+
 // The same walk over a stream of rays, for waves whose rays go many ways through deep trees: a warp keeps its lanes in
 // work. trace_binary's lanes wait for each other twice: those at a leaf until the last of the warp has left the inner
 // loop, and those whose ray has ended until the warp's longest ray has; 7-9 of 32 lanes are left a warp instruction.
@@ -205,24 +207,27 @@ __device__ __forceinline__ Hit trace_binary(const DScene& S, const Sections& X, 
 // 15.95-16.6 ms). A town's second depth (640 x 512, 1 spp): 7.6 -> 13.4 lanes and 175 -> 140 M warp instructions for its
 // shadow rays, 8.8 -> 13.7 and 101 -> 92 M closest; the more rays a warp gets, the better (34 of them, no gain; 400,
 // 30 % by a count of the phases), and short walks lose (the rounds cost a quarter more thread instructions): the caller
-// chooses. The town at 512 x 512, 16 spp, 16.85 -> 15.26 ms; the city frame (720p, 1 spp)
-// 4.46 -> 4.25. STREAM_STEPS / STREAM_REFILL 3 / 12: 15.69, 4 / 16: 15.63, 6 / 16: 15.66, 2 / 8: 16.14 (before the other
-// ballots were put off).
+// chooses. The town at 512 x 512, 16 spp, 16.85 -> 15.36 ms; the city frame (720p, 1 spp) 4.46 -> 4.27. STREAM_STEPS /
+// STREAM_REFILL 3 / 12: 15.69, 4 / 16: 15.63, 6 / 16: 15.66, 2 / 8: 16.14 (before the other ballots were put off).
 //
-// n rays, handed out by `counter`. load(i, ray, o, d, t, mode) fetches the i-th and names it; hit(ray, x, tri, rec)
-// takes a nearer hit (t, u, v) and says whether the ray is done; done(ray) ends one, unless hit() set it to NO_RAY. What a
-// ray meets, and in which order, is trace_binary's, and so are the checks of every index and WALK_GUARD (a ray each).
+// n rays, handed out by `counter`. load(i, ray, o, d, t, mode) fetches the i-th and names it; its scene is `one`, or, where
+// Lane::ON, what load has bound `view` to; hit(ray, x, tri, rec) takes a nearer hit (t, u, v) and says whether the ray is
+// done; done(ray) ends one, unless hit() set it to NO_RAY. What a ray meets, and in which order, is trace_binary's, and so
+// are the checks of every index and WALK_GUARD (a ray each).
 constexpr uint32_t NO_RAY = 0xffffffffu;
 constexpr int STREAM_STEPS = 4, STREAM_REFILL = 16;
-template <class Load, class Take, class Done>
-__device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instances, uint32_t top, uint32_t n_units,
-                                             uint32_t* counter, uint32_t n, Load load, Take hit, Done done,
+template <class Lane, class Load, class Take, class Done>
+__device__ __forceinline__ void trace_stream(const DScene& one, uint32_t one_instances, uint32_t one_top, uint32_t one_units,
+                                             Lane& view, uint32_t* counter, uint32_t n, Load load, Take hit, Done done,
                                              unsigned long long& guard_trips) {
     constexpr unsigned ALL = 0xffffffffu;
     constexpr uint32_t IDLE = 0xffffffffu, NO_BASE = 0xffffffffu;
-    const uint32_t last_node = (uint32_t)min((unsigned long long)S.n_nodes - 1ull, 0xffffffffull);
-    const uint32_t tris_end = (uint32_t)min((unsigned long long)S.n_tris, 0xffffffffull);
-    const uint32_t tables_end = (uint32_t)min((unsigned long long)S.n_table_vec4, 0xffffffffull);
+    const uint32_t one_last = end32(one.n_nodes - 1ull);
+    const uint32_t one_tris = end32(one.n_tris);
+    const uint32_t one_tables = end32(one.n_table_vec4);
+    auto nodes = [&]() -> const uint4* { if constexpr (Lane::ON) return view.nodes; else return one.nodes; };
+    auto last_node = [&]() -> uint32_t { if constexpr (Lane::ON) return view.last; else return one_last; };
+    auto top_of = [&]() -> uint32_t { if constexpr (Lane::ON) return view.top(); else return one_top; };
     const uint32_t lane = threadIdx.x & 31u;
     V3 o{0.0f, 0.0f, 0.0f}, d = o, inv_d = o, ro = o, rd = o, rinv = o;
     float t = 0.0f;
@@ -236,10 +241,10 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
             rec = NO_INST;
             base = NO_BASE;
             ro = o; rd = d; rinv = inv_d;
-            off = top;
+            off = top_of();
         }
         if (sp == 0) { count = IDLE; return; }
-        const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * stack[--sp]);
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(nodes() + 2ull * stack[--sp]);
         at = __ldg(q + 3);
         count = __ldg(q + 7);
         if (count == 0) at += off;
@@ -262,17 +267,17 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
                     load(i, ray, o, d, t, mode);
                     inv_d = safe_inv(d);
                     ro = o; rd = d; rinv = inv_d;
-                    off = top; rec = NO_INST; iter = 0;
+                    off = top_of(); rec = NO_INST; iter = 0;
                     sp = 0; base = NO_BASE;
-                    if (n_units != 0) {
-                        if (top >= S.n_nodes) trip();
+                    if ((Lane::ON ? view.units() : one_units) != 0) {
+                        if (off >= (Lane::ON ? view.scene(one).n_nodes : one.n_nodes)) trip();
                         else {
-                            const uint4* q = S.nodes + 2ull * top;
+                            const uint4* q = nodes() + 2ull * off;
                             const uint4 x = __ldg(q), y = __ldg(q + 1);
                             float tn;
                             if (box_hit(o, inv_d, x, y, t, tn)) {
                                 count = y.w;
-                                at = count == 0 ? x.w + top : x.w;
+                                at = count == 0 ? x.w + off : x.w;
                             }
                         }
                     }
@@ -290,9 +295,9 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
 #pragma unroll
             for (int step = 0; step < STREAM_STEPS; ++step) {
                 if (count == 0) {
-                    if (iter++ >= WALK_GUARD || at >= last_node) trip();
+                    if (iter++ >= WALK_GUARD || at >= last_node()) trip();
                     else {
-                        const uint4* q = S.nodes + 2ull * at;
+                        const uint4* q = nodes() + 2ull * at;
                         const uint4 l0 = __ldg(q), l1 = __ldg(q + 1), r0 = __ldg(q + 2), r1 = __ldg(q + 3);
                         float tl, tr;
                         const bool hl = box_hit(ro, rinv, l0, l1, t, tl), hr = box_hit(ro, rinv, r0, r1, t, tr);
@@ -310,10 +315,20 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
             }
         } else if (n_unit >= n_tri) {
             if (units >> lane & 1u) {
-                const uint32_t b = t_instances + at * 10u;
+                uint32_t b, tables_end;
+                const uint4* tables;
+                if constexpr (Lane::ON) {
+                    tables = view.scene(one).tables;
+                    b = view.instances() + at * 10u;
+                    tables_end = end32(view.scene(one).n_table_vec4);
+                } else {
+                    tables = one.tables;
+                    b = one_instances + at * 10u;
+                    tables_end = one_tables;
+                }
                 if (iter++ >= WALK_GUARD || tables_end < 10u || b > tables_end - 10u) trip();
                 else {
-                    const uint4* u = S.tables + b;
+                    const uint4* u = tables + b;
                     const float4* uf = reinterpret_cast<const float4*>(u);
                     const float4 n1 = __ldg(uf + 4);
                     const uint32_t ubits = bu(n1.w);
@@ -329,9 +344,9 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
                         }
                         off = bu(n0.w);
                         base = sp;
-                        if (off > last_node) trip();
+                        if (off > last_node()) trip();
                         else {
-                            const uint32_t* q = reinterpret_cast<const uint32_t*>(S.nodes + 2ull * off);
+                            const uint32_t* q = reinterpret_cast<const uint32_t*>(nodes() + 2ull * off);
                             at = __ldg(q + 3);
                             count = __ldg(q + 7);
                             if (count == 0) at += off;
@@ -342,6 +357,8 @@ __device__ __forceinline__ void trace_stream(const DScene& S, uint32_t t_instanc
                 }
             }
         } else if (count - 1u < IDLE - 1u && rec != NO_INST) {
+            const DScene& S = view.scene(one);
+            const uint32_t tris_end = Lane::ON ? end32(S.n_tris) : one_tris;
             bool ended = iter++ >= WALK_GUARD;
             if (ended) trip();
             for (uint32_t k = 0; !ended && k < count; ++k) {
