@@ -783,7 +783,11 @@ __global__ void __launch_bounds__(PATHS_BLOCK, TRT_BLOCKS_PATHS) k_paths(const J
 //     the material row it stands for lay behind three dependent loads (the job, the instance, its row), which bounded
 //     the count (latency; 720p city frame 36 us a launch of 460,800 items under ncu). The frame 4.36 -> 4.32 ms.
 //   SORT_SHADOWS: the shadow rays by (position chunk, direction octant) in each light class.
-constexpr uint32_t SORT_BINS = 4096u, SORT_THREADS = 256u, SORT_PER_THREAD = 8u;
+// Blocks of 1,024 threads with two items each: the keys' loads and the atomics behind them are latency, which more
+// warps hide, while a block's clearing of the bins and its atomic a key it meets want many items a block. The 720p city
+// frame 4.27 ms with 256 x 8, 4.25 with 512 x 8 or 256 x 4, 4.21 with 1,024 x 2 (3 and 4 alike, 8: 4.23); an 800 x 800 view
+// of it 3.77 -> 3.65, the town at 512 x 512, 16 spp, 15.39 -> 15.25.
+constexpr uint32_t SORT_BINS = 4096u, SORT_THREADS = 1024u, SORT_PER_THREAD = 2u;
 constexpr uint32_t SORT_ITEMS = SORT_THREADS * SORT_PER_THREAD;
 enum : uint32_t { SORT_RAYS = 0u, SORT_HITS = 1u, SORT_SHADOWS = 2u };
 
