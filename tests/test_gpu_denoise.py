@@ -41,3 +41,18 @@ def test_depth_guide_is_the_first_hit_distance(gpu):
     # against the camera rays' hits: the mean over samples of t, 0 on escape; the walk's own t on sample 0's rays
     assert (depth > 0).mean() > 0.5 and np.isfinite(depth).all()
     S.close()
+
+
+# The filter's 32 x 8 tiles: one pixel, less than a tile, a column and a row past it, many tiles with a ragged edge; no
+# pass (the modulation alone), one, and steps past the image. The tolerance is the one above, for four passes or fewer
+# (a weight's few ulps of expf enter once a pass).
+@pytest.mark.parametrize("w,h,iterations", [(1, 1, 4), (5, 3, 1), (32, 8, 2), (33, 9, 3), (65, 41, 0), (97, 23, 4), (131, 50, 5)])
+def test_atrous_on_ragged_tiles_matches_the_oracle(gpu, w, h, iterations):
+    P = prep.prepare(small_city(width=w, height=h))
+    S = gpu.upload(P)
+    acc, _ = S.render_raw(P.params, 2)
+    got, _ = S.denoise_atrous(iterations)
+    want = oracle.denoise(acc, w, h, iterations)
+    rtol = 2e-4 * max(1.0, iterations / 4)
+    assert np.allclose(got, want, rtol=rtol, atol=0.5 * rtol * float(np.abs(want).mean()))
+    S.close()
