@@ -59,16 +59,16 @@ void launch_pdl(bool early, void (*kernel)(P...), dim3 grid, uint32_t block, uin
 //
 // y[p][n] = bias[n] + sum over taps t and channels c of x[p + off(t)][c] * w[t][c][n], zero outside the image.
 // A CTA computes a tile of 128 pixels (a bw x bh rectangle of one image, bw the largest power of two <= 128 that
-// divides the width) x N output channels (N 128 where 128 divides co_pad, else 64; blockIdx.y their tile) on the
-// 5th-generation tensor cores:
-//  - one thread issues the loads: per K stage (one tap, 32 input channels) a TMA box of 32 channels x bw x bh pixels,
-//    shifted by the tap (the halo and the image's border read as zeros), and a TMA box of the tap's weights (N
-//    output channels x the 32 input channels); both land as 64-byte rows with the 64-byte swizzle, the canonical
-//    K-major layout the MMA reads (8-row atoms of 512 bytes);
-//  - one thread issues two tcgen05.mma (M 128, N, K 16, bf16 in, f32 accumulate in tensor memory) a stage and
-//    commits each stage's buffers back to the loader through an mbarrier; TS stages in flight;
+// divides the width) x N output channels (N = nt: 32, 64 or 128; blockIdx.y their tile) on the 5th-generation tensor
+// cores:
+//  - a warp issues the loads by one elected lane: per K block (one tap, 32 input channels; KB of them a stage) a TMA box
+//    of 32 channels x bw x bh pixels, shifted by the tap (the halo and the image's border read as zeros), and a TMA box
+//    of the tap's weights (N output channels x the 32 input channels); both land as 64-byte rows with the 64-byte
+//    swizzle, the canonical K-major layout the MMA reads (8-row atoms of 512 bytes);
+//  - a warp issues, by one elected lane, two tcgen05.mma (M 128, N, K 16, bf16 in, f32 accumulate in tensor memory) a K
+//    block and commits each stage's buffers back to the loader through an mbarrier; TS stages in flight;
 //  - where the layer reads one 32-channel block into one output tile (cin 32, co_pad = N), the nine taps' weight boxes
-//    (36 KB) are loaded once a CTA into the weight stages' room, and a stage loads the activations alone;
+//    are loaded once a CTA into the weight stages' room, and a stage loads the activations alone;
 //  - eight warps read the accumulator out of tensor memory (two a 32-lane quarter = 32 pixels, each half of the
 //    columns), add the bias, apply the ReLU and store bf16 (or f32) NHWC.
 // Every mbarrier wait is bounded (about a second); a wait that gives up sets the error word, and the CTA waits
