@@ -715,7 +715,6 @@ __global__ void __launch_bounds__(PATHS_BLOCK, TRT_BLOCKS_PATHS) k_paths(const J
             const uint32_t n_own = s_count[0], n_rays = n_own + s_count[1];
             for (uint32_t m = pending; m != 0u; m &= m - 1u) s_ray[n_own + at1++] = (tid << 3) | (__ffs(m) - 1);
             __syncthreads();
-            if (n_rays == 0u) break;
             const uint32_t chunk = min(32u, (n_rays + PATHS_BLOCK / 32u - 1u) / (PATHS_BLOCK / 32u));
             for (;;) {
                 uint32_t at = 0;
@@ -752,7 +751,10 @@ __global__ void __launch_bounds__(PATHS_BLOCK, TRT_BLOCKS_PATHS) k_paths(const J
                 __syncwarp();
             }
             __syncthreads();
+            // (the vertices of a depth that left no ray are resolved too: their light that asks for none, and the
+            // ended paths' last fixes)
             if (shaded) resolve_vertex(B, p, pf(P, P_MISC), s_vis[tid]);
+            if (n_rays == 0u) break;
             shaded = live;
             pending = 0u;
             if (live) {
