@@ -249,7 +249,8 @@ typedef struct {
 
 /* Device times of one deformation (filled when stats is given: the call then waits for it) and the errors the device
  * found (a tree that is not one, a top tree that came out deeper than TOP_DEPTH; bit 16: the wide BVH's refit met an
- * index out of its buffers). wide_ms: the wide BVH's refit (0 when the scene has none built), after device_ms. */
+ * index out of its buffers; bit 32: a unit's transform makes its box not a number, and a point at the origin stands for
+ * it). wide_ms: the wide BVH's refit (0 when the scene has none built), after device_ms. */
 typedef struct { float device_ms, skin_ms, gather_ms, refit_ms, top_ms, wide_ms; uint32_t errors; } trt_deform_stats;
 
 /* Uploads the skinned models' corners and the deforming meshes, checks each mesh's tree (on the host copy taken at

@@ -28,7 +28,7 @@ constexpr uint32_t TOP_BINS = 32u;                  // units.rs:121
 // through a large subtree, and a launch a level costs 12 us of latency however small its nodes are.)
 constexpr uint32_t TOP_SMALL = 128u, TOP_WARPS = 32u, TOP_THREADS = TOP_WARPS * 32u;
 // Error bits the kernels record.
-constexpr uint32_t E_TREE = 1u, E_DEPTH = 2u, E_ROOT = 4u, E_INDEX = 8u;
+constexpr uint32_t E_TREE = 1u, E_DEPTH = 2u, E_ROOT = 4u, E_INDEX = 8u, E_BOX = 32u;  // (16: DEFORM_E_WIDE)
 
 struct DMesh { uint32_t first_vertex, n_vertices, first_corner, palette, first_tri, n_tris, root, n_nodes; };
 static_assert(sizeof(DMesh) == sizeof(trt_deform_mesh), "DMesh mirrors trt_deform_mesh");
@@ -186,6 +186,8 @@ struct TopBuild {
     uint32_t top_first, n_units;
 };
 
+__device__ __forceinline__ bool nan3(V3 v) { return v.x != v.x || v.y != v.y || v.z != v.z; }
+
 // units.rs:288-300 UnitBox::new of each unit's tree root box under its world rows, its centre, and the build's start.
 __global__ void k_unit_boxes(const uint4* __restrict__ tables, uint32_t t_instances, uint64_t n_nodes, TopBuild T) {
     uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
@@ -223,10 +225,17 @@ __global__ void k_unit_boxes(const uint4* __restrict__ tables, uint32_t t_instan
     V3 e = bb - a;
     V3 m = V3{gmax(fabsf(a.x), fabsf(bb.x)), gmax(fabsf(a.y), fabsf(bb.y)), gmax(fabsf(a.z), fabsf(bb.z))};
     float pad = gmax(e.x, gmax(e.y, e.z)) * 1e-4f + gmax(m.x, gmax(m.y, m.z)) * 1e-5f + 1e-6f;
-    V3 blo = a - v3(pad), bhi = bb + v3(pad);
+    V3 blo = a - v3(pad), bhi = bb + v3(pad), mid = (blo + bhi) * 0.5f;
+    // A box or centre that is not a number is refused where there is anything to split, and a point stands for it: what
+    // gmin and gmax make of a NaN depends on their operands' order, so a reduction would leave a warp's lanes with
+    // different boxes, and lanes that then leave an axis out of the sweep would miss the others' shuffles.
+    if (T.n_units > 1u && (nan3(blo) || nan3(bhi) || nan3(mid))) {
+        atomicOr(T.err, E_BOX);
+        blo = bhi = mid = v3(0.0f);
+    }
     T.box[2ull * u] = f4(blo, 0.0f);
     T.box[2ull * u + 1] = f4(bhi, 0.0f);
-    T.centre[u] = f4((blo + bhi) * 0.5f, 0.0f);
+    T.centre[u] = f4(mid, 0.0f);
 }
 
 __device__ __forceinline__ float area3(V3 lo, V3 hi) {
@@ -546,7 +555,7 @@ __device__ uint32_t split_block(const TopBuild& T, TopShared& S, uint4 task, uin
         if (nl_run != mid) atomicOr(T.err, E_TREE);
         store_box(T.nodes, T.top_first + fin, lo, hi, 1u + 2u * pre, 0u);
     }
-    return mid;
+    return nl_run == mid ? mid : 0u;  // (the lists have room for children that share no unit)
 }
 
 // A level's nodes of more than TOP_SMALL units, a block a node; their children to the next level's list or to
@@ -706,8 +715,8 @@ __device__ void split_warp(const TopBuild& T, TopShared& S, uint4 task, uint32_t
         nr_run += __popc(rm);
     }
     if (lane == 0) {
-        if (nl_run != mid) atomicOr(T.err, E_TREE);
         store_box(T.nodes, node, lo, hi, 1u + 2u * pre, 0u);
+        if (nl_run != mid) { atomicOr(T.err, E_TREE); return; }
         const uint32_t at = atomicAdd(&S.n_tasks[(level + 1u) & 1u], 2u);
         S.tasks[(level + 1u) & 1u][at] = child_of(task, mid, 0);
         S.tasks[(level + 1u) & 1u][at + 1u] = child_of(task, mid, 1);
@@ -1061,7 +1070,9 @@ int deform_run(DeformState* st, const SceneBuffers& sb, const uint32_t* P, const
         rc = deform_errors(st, s, &stats->errors);
         if (rc) return rc;
         if (stats->errors) {
-            err = "trt_deform: the device found a bad tree (error bits " + std::to_string(stats->errors) + ")";
+            err = std::string("trt_deform: the device found ") +
+                  ((stats->errors & E_BOX) != 0u ? "a unit whose box is not a number" : "a bad tree") + " (error bits " +
+                  std::to_string(stats->errors) + ")";
             return TRT_EGUARD;
         }
     }
