@@ -112,3 +112,16 @@ def test_a_servers_streams_of_several_scenes_rays(gpu, side, spp):
     for r in reqs:
         alone, _ = S[r.scene].render_raw(r.params, r.spp)
         assert np.array_equal(r.accum.view(np.uint32), alone.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h", [(363, 363), (630, 640)])
+def test_a_leafs_count_is_any_number_but_zero(gpu, w, h):
+    """A top leaf's count only says that it is a leaf: the streams take the largest there is as single walks do."""
+    P = prep.prepare(many_units())
+    P.nodes = P.nodes.copy()
+    nodes = P.nodes.reshape(-1, 8)
+    top, n = int(P.params[70]), int(P.params[71])
+    leaves = top + np.flatnonzero(nodes[top:top + 2 * n - 1, 7] != 0)
+    assert len(leaves) == n
+    nodes[leaves[::2], 7] = 0xFFFFFFFF
+    same(gpu.upload(P), sized(P, w, h), 1, 0, N.TRT_RENDER_COUNT)
