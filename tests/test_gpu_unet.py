@@ -198,3 +198,19 @@ def test_a_withheld_copy_ends_the_forward_with_an_error_and_the_network_stays_us
         assert np.array_equal(got, want)
     finally:
         n.close()
+
+
+@pytest.mark.parametrize("h,w", [(64, 64), (32, 256), (128, 128)])
+def test_one_withheld_copy_ends_one_block_alone(h, w):
+    """The layers after the one that waits in vain have started early, but the bounds of their own waits have not: they
+    run to their end on what it left, and one block is all that gave up."""
+    from threert_b200 import RenderError
+    n = unet.UNet(0, max_batch=1, max_h=h, max_w=w)
+    try:
+        n.set_params(unet.init_params(3))
+        f = np.random.default_rng(9).normal(0, 1, (1, h, w, unet.N_FEAT)).astype(np.float32)
+        n.hold_next_load()
+        with pytest.raises(RenderError, match="gave up in 1 block$"):
+            n.forward(f)
+    finally:
+        n.close()

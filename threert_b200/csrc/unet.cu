@@ -141,15 +141,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t a, uint32_t parity) {
         : "memory");
     return ok != 0u;
 }
-// A bounded wait: about 2^31 cycles (a second at the B200's clock), then the error word and the CTA's abort word,
-// which ends every other wait of the CTA at once.
+// A bounded wait: about 2^31 cycles (a second at the B200's clock), then the CTA's abort word, which ends every other wait
+// of the CTA at once, and a count of one more CTA that gave up in the error word.
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, uint32_t* err, volatile uint32_t* abort_flag) {
     long long t0 = clock64();
     while (!mbar_try_wait(a, parity)) {
         if (*abort_flag) return false;
         if (clock64() - t0 > (1ll << 31)) {
-            atomicOr(err, 1u);
-            *abort_flag = 1u;
+            if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0u) atomicAdd(err, 1u);
             return false;
         }
     }
@@ -418,6 +417,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
             const uint32_t idesc = umma_idesc(128u, n_mma);
             uint32_t it = 0, ti = 0;
             bool ok = !a.resident || mbar_wait_warp(wfull, 0u, a.err, abort_flag);
+            // (the stages' waits are of this CTA's own copies: their bound starts when the layer before has ended, not
+            // while it runs, or one layer that gives up would take the next with it)
+            pdl_wait();
             for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++ti) {
                 const uint32_t acc = ti & 1u;
                 if (ti >= 2u && !(ok = mbar_wait_warp(acc_empty(acc), ((ti / 2u) - 1u) & 1u, a.err, abort_flag))) break;
@@ -1042,7 +1044,7 @@ struct Net {
     cudaStream_t aux = nullptr;
     bool early = true;            // the layers start while the one before drains (launch_pdl)
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
-    uint32_t* dev_err = nullptr;  // set by a convolution whose pipeline wait gave up
+    uint32_t* dev_err = nullptr;  // the CTAs of convolutions and weight gradients whose pipeline wait gave up
     bool hold_next = false;       // the next convolution launched outside a graph withholds one copy (a test)
     uint32_t sms = 148;           // the device's SMs (the persistent convolution's grid)
     float* wpart = nullptr;       // the weight gradient's CTA partials (128 x 128 f32 each)
@@ -1426,7 +1428,8 @@ int finish(Net* n, const char* what) {
     if (rc) return rc;
     if (e) {
         cudaMemset(n->dev_err, 0, 4);
-        n->err = std::string(what) + ": a convolution's pipeline wait gave up";
+        n->err = std::string(what) + ": a convolution's pipeline wait gave up in " + std::to_string(e) +
+                 (e == 1u ? " block" : " blocks");
         return TRT_ECUDA;
     }
     return TRT_OK;
