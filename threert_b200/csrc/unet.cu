@@ -98,6 +98,7 @@ struct Conv {
 // stage's waits are paid once for them, TS stages (99 KB of shared memory: two CTAs an SM). Five stages of one block took
 // 185 us for the 264 x 136 forward and 487 for a training step on 16 crops of 64 x 64; two of three, 161 and 455.
 constexpr uint32_t TS = 2u, KB = 3u;
+static_assert(9u % KB == 0u, "a layer's K blocks fill its stages");
 constexpr uint32_t A_BOX = 128u * 32u * 2u, B_BOX = 128u * 32u * 2u, A_STAGE = KB * A_BOX, B_STAGE = KB * B_BOX;
 constexpr uint32_t CONV_SMEM = TS * (A_STAGE + B_STAGE) + 256u + 1024u;  // + room to align the stages to 1 KB
 // The halo variant (a row tile of 128 pixels read once with its halo, the taps as shifted descriptors): a stage is a
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t sraw = smem_addr(smem_raw), sbase = (sraw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (sbase - sraw);
-    const uint32_t kc = a.cin / 32u, nb = 9u * kc, nk = HALO ? kc : (nb + KB - 1u) / KB;  // (nk: a tile's stages)
+    const uint32_t kc = a.cin / 32u, nk = HALO ? kc : 9u / KB * kc;  // (nk: a tile's stages)
     const uint32_t A_OFF = HALO && a.resident ? halo_weights(kc, a.nt) : 0u, B_OFF = HALO ? 0u : TS * A_STAGE;
     const uint32_t BAR_OFF = HALO ? A_OFF + NS * A_BYTES : TS * (A_STAGE + B_STAGE);
     const uint32_t sA = sbase + A_OFF, sB = sbase + B_OFF, sBar = sbase + BAR_OFF;
@@ -391,9 +392,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                                 tma_load_3d(leader, sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
                                             (int)n0, (int)tap, full(s));
                     } else {
-                        const uint32_t here = min(KB, nb - k * KB);
-                        mbar_expect_tx(leader, full(s), here * (A_BOX + (a.resident ? 0u : a.nt * 64u)));
-                        for (uint32_t i = 0; i < here; ++i) {
+                        mbar_expect_tx(leader, full(s), KB * (A_BOX + (a.resident ? 0u : a.nt * 64u)));
+                        for (uint32_t i = 0; i < KB; ++i) {
                             const uint32_t tap = (k * KB + i) / kc, c0 = (k * KB + i) % kc * 32u;
                             const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
                             if (!withhold || i != 0u)
@@ -450,7 +450,6 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
                         const uint32_t b_box = a.resident ? a.nt * 4u : B_BOX / 16u;  // (in the descriptors' 16-byte units)
 #pragma unroll
                         for (uint32_t i = 0; i < KB; ++i) {
-                            if (i != 0u && k * KB + i >= nb) break;
                             umma_f16(leader, d, ad + i * (A_BOX / 16u), bd + i * b_box, idesc, (k | i) != 0u ? 1u : 0u);
                             if (!HALF_K)
                                 umma_f16(leader, d, ad + i * (A_BOX / 16u) + 2u, bd + i * b_box + 2u, idesc, 1u);
