@@ -358,110 +358,106 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
     };
 
     if (warp == 0) {
-        {
-            const uint32_t leader = elect_one();
-            // the loader: the resident weights (the nine taps' boxes, one after another), then the stages of every tile
-            // of this CTA, in order
-            // (halo: every 32-channel block's nine boxes, block-major)
-            if (a.resident) {
-                const uint32_t blocks = HALO ? kc : 1u;
-                mbar_expect_tx(leader, wfull, 9u * blocks * a.nt * 64u);
-                for (uint32_t k = 0; k < blocks; ++k)
-                    for (uint32_t tap = 0; tap < 9u; ++tap)
-                        tma_load_3d(leader, sB + (k * 9u + tap) * a.nt * 64u, &wmap, (int)(k * 32u), 0, (int)tap, wfull);
-            }
-            pdl_wait();
-            uint32_t it = 0;
-            bool ok = true;
-            for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                uint32_t b, n0;
-                int x0, y0;
-                tile_of(t, b, x0, y0, n0);
-                for (uint32_t k = 0; k < nk; ++k, ++it) {
-                    const uint32_t s = it % NS;
-                    if (it >= NS && !(ok = mbar_wait_warp(empty(s), ((it / NS) - 1u) & 1u, a.err, abort_flag))) break;
-                    const bool withhold = a.hold && blockIdx.x == 0 && it == 0;
-                    if constexpr (HALO) {
-                        // the tile's rows y0 - 1 .. y0 + 1, pixels x0 - 1 .. x0 + 128
-                        mbar_expect_tx(leader, full(s), HALO_BYTES + (a.resident ? 0u : 9u * a.nt * 64u));
-                        if (!withhold)
-                            tma_load_4d(leader, sA + s * A_BYTES, &xmap, (int)(a.x_off + k * 32u), x0 - 1, y0 - 1, (int)b,
-                                        full(s));
+        const uint32_t leader = elect_one();
+        // the loader: the resident weights (the nine taps' boxes, one after another), then the stages of every tile
+        // of this CTA, in order
+        // (halo: every 32-channel block's nine boxes, block-major)
+        if (a.resident) {
+            const uint32_t blocks = HALO ? kc : 1u;
+            mbar_expect_tx(leader, wfull, 9u * blocks * a.nt * 64u);
+            for (uint32_t k = 0; k < blocks; ++k)
+                for (uint32_t tap = 0; tap < 9u; ++tap)
+                    tma_load_3d(leader, sB + (k * 9u + tap) * a.nt * 64u, &wmap, (int)(k * 32u), 0, (int)tap, wfull);
+        }
+        pdl_wait();
+        uint32_t it = 0;
+        bool ok = true;
+        for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            uint32_t b, n0;
+            int x0, y0;
+            tile_of(t, b, x0, y0, n0);
+            for (uint32_t k = 0; k < nk; ++k, ++it) {
+                const uint32_t s = it % NS;
+                if (it >= NS && !(ok = mbar_wait_warp(empty(s), ((it / NS) - 1u) & 1u, a.err, abort_flag))) break;
+                const bool withhold = a.hold && blockIdx.x == 0 && it == 0;
+                if constexpr (HALO) {
+                    // the tile's rows y0 - 1 .. y0 + 1, pixels x0 - 1 .. x0 + 128
+                    mbar_expect_tx(leader, full(s), HALO_BYTES + (a.resident ? 0u : 9u * a.nt * 64u));
+                    if (!withhold)
+                        tma_load_4d(leader, sA + s * A_BYTES, &xmap, (int)(a.x_off + k * 32u), x0 - 1, y0 - 1, (int)b,
+                                    full(s));
+                    if (!a.resident)
+                        for (uint32_t tap = 0; tap < 9u; ++tap)
+                            tma_load_3d(leader, sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
+                                        (int)n0, (int)tap, full(s));
+                } else {
+                    mbar_expect_tx(leader, full(s), KB * (A_BOX + (a.resident ? 0u : a.nt * 64u)));
+                    for (uint32_t i = 0; i < KB; ++i) {
+                        const uint32_t tap = (k * KB + i) / kc, c0 = (k * KB + i) % kc * 32u;
+                        const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
+                        if (!withhold || i != 0u)
+                            tma_load_4d(leader, sA + s * A_STAGE + i * A_BOX, &xmap, (int)(a.x_off + c0), x0 + dx,
+                                        y0 + dy, (int)b, full(s));
                         if (!a.resident)
-                            for (uint32_t tap = 0; tap < 9u; ++tap)
-                                tma_load_3d(leader, sA + s * A_BYTES + HALO_STAGE + tap * a.nt * 64u, &wmap, (int)(k * 32u),
-                                            (int)n0, (int)tap, full(s));
-                    } else {
-                        mbar_expect_tx(leader, full(s), KB * (A_BOX + (a.resident ? 0u : a.nt * 64u)));
-                        for (uint32_t i = 0; i < KB; ++i) {
-                            const uint32_t tap = (k * KB + i) / kc, c0 = (k * KB + i) % kc * 32u;
-                            const int dy = (int)(tap / 3u) - 1, dx = (int)(tap % 3u) - 1;
-                            if (!withhold || i != 0u)
-                                tma_load_4d(leader, sA + s * A_STAGE + i * A_BOX, &xmap, (int)(a.x_off + c0), x0 + dx,
-                                            y0 + dy, (int)b, full(s));
-                            if (!a.resident)
-                                tma_load_3d(leader, sB + s * B_STAGE + i * B_BOX, &wmap, (int)c0, (int)n0, (int)tap, full(s));
-                        }
+                            tma_load_3d(leader, sB + s * B_STAGE + i * B_BOX, &wmap, (int)c0, (int)n0, (int)tap, full(s));
                     }
                 }
             }
-            if (lane == 0) counts[0] = it;
         }
+        if (lane == 0) counts[0] = it;
     } else if (warp == 1) {
-        {
-            const uint32_t leader = elect_one();
-            // the MMA issuer: a tile's stages into accumulator (tile count % 2), then that accumulator to the epilogue
-            // (at most 16 outputs: the MMAs' N covers 16 of the tile's rows of weights; the epilogue reads no column
-            // past the outputs)
-            const uint32_t n_mma = a.cout <= 16u ? 16u : a.nt;
-            const uint32_t idesc = umma_idesc(128u, n_mma);
-            uint32_t it = 0, ti = 0;
-            bool ok = !a.resident || mbar_wait_warp(wfull, 0u, a.err, abort_flag);
-            // (the stages' waits are of this CTA's own copies: their bound starts when the layer before has ended, not
-            // while it runs, or one layer that gives up would take the next with it)
-            pdl_wait();
-            for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++ti) {
-                const uint32_t acc = ti & 1u;
-                if (ti >= 2u && !(ok = mbar_wait_warp(acc_empty(acc), ((ti / 2u) - 1u) & 1u, a.err, abort_flag))) break;
+        const uint32_t leader = elect_one();
+        // the MMA issuer: a tile's stages into accumulator (tile count % 2), then that accumulator to the epilogue
+        // (at most 16 outputs: the MMAs' N covers 16 of the tile's rows of weights; the epilogue reads no column
+        // past the outputs)
+        const uint32_t n_mma = a.cout <= 16u ? 16u : a.nt;
+        const uint32_t idesc = umma_idesc(128u, n_mma);
+        uint32_t it = 0, ti = 0;
+        bool ok = !a.resident || mbar_wait_warp(wfull, 0u, a.err, abort_flag);
+        // (the stages' waits are of this CTA's own copies: their bound starts when the layer before has ended, not
+        // while it runs, or one layer that gives up would take the next with it)
+        pdl_wait();
+        for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++ti) {
+            const uint32_t acc = ti & 1u;
+            if (ti >= 2u && !(ok = mbar_wait_warp(acc_empty(acc), ((ti / 2u) - 1u) & 1u, a.err, abort_flag))) break;
+            tc_fence_after();
+            const uint32_t d = tmem + acc * a.nt;
+            for (uint32_t k = 0; k < nk; ++k, ++it) {
+                const uint32_t s = it % NS;
+                if (!(ok = mbar_wait_warp(full(s), (it / NS) & 1u, a.err, abort_flag))) break;
                 tc_fence_after();
-                const uint32_t d = tmem + acc * a.nt;
-                for (uint32_t k = 0; k < nk; ++k, ++it) {
-                    const uint32_t s = it % NS;
-                    if (!(ok = mbar_wait_warp(full(s), (it / NS) & 1u, a.err, abort_flag))) break;
-                    tc_fence_after();
-                    if constexpr (HALO) {
-                        // tap (dy, dx): 128 rows of 64 bytes from row (dy + 1) x 130 + dx + 1 (the swizzle goes by
-                        // the address, so a start inside its 8-row pattern reads what the copy wrote)
-                        const uint64_t ad0 = umma_desc_sw64(sA + s * A_BYTES, 512u);
-                        const uint64_t bd0 = umma_desc_sw64(
-                            a.resident ? sB + k * 9u * a.nt * 64u : sA + s * A_BYTES + HALO_STAGE, 512u);
-                        const uint32_t b_tap = a.nt * 4u;  // a tap's weights, in the descriptors' 16-byte units
+                if constexpr (HALO) {
+                    // tap (dy, dx): 128 rows of 64 bytes from row (dy + 1) x 130 + dx + 1 (the swizzle goes by
+                    // the address, so a start inside its 8-row pattern reads what the copy wrote)
+                    const uint64_t ad0 = umma_desc_sw64(sA + s * A_BYTES, 512u);
+                    const uint64_t bd0 = umma_desc_sw64(
+                        a.resident ? sB + k * 9u * a.nt * 64u : sA + s * A_BYTES + HALO_STAGE, 512u);
+                    const uint32_t b_tap = a.nt * 4u;  // a tap's weights, in the descriptors' 16-byte units
 #pragma unroll
-                        for (uint32_t tap = 0; tap < 9u; ++tap) {
-                            const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
-                            umma_f16(leader, d, ad0 + row * 4u, bd0 + tap * b_tap, idesc, (k | tap) != 0u ? 1u : 0u);
-                            if (!HALF_K)
-                                umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
-                        }
-                    } else {
-                        // (resident weights: one box a tap, kc = 1)
-                        const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
-                        const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * KB * a.nt * 64u : sB + s * B_STAGE, 512u);
-                        const uint32_t b_box = a.resident ? a.nt * 4u : B_BOX / 16u;  // (in the descriptors' 16-byte units)
-#pragma unroll
-                        for (uint32_t i = 0; i < KB; ++i) {
-                            umma_f16(leader, d, ad + i * (A_BOX / 16u), bd + i * b_box, idesc, (k | i) != 0u ? 1u : 0u);
-                            if (!HALF_K)
-                                umma_f16(leader, d, ad + i * (A_BOX / 16u) + 2u, bd + i * b_box + 2u, idesc, 1u);
-                        }
+                    for (uint32_t tap = 0; tap < 9u; ++tap) {
+                        const uint32_t row = (tap / 3u) * HALO_W + tap % 3u;
+                        umma_f16(leader, d, ad0 + row * 4u, bd0 + tap * b_tap, idesc, (k | tap) != 0u ? 1u : 0u);
+                        if (!HALF_K)
+                            umma_f16(leader, d, ad0 + row * 4u + 2u, bd0 + tap * b_tap + 2u, idesc, 1u);
                     }
-                    umma_commit(leader, empty(s));
+                } else {
+                    // (resident weights: one box a tap, kc = 1)
+                    const uint64_t ad = umma_desc_sw64(sA + s * A_STAGE, 512u);
+                    const uint64_t bd = umma_desc_sw64(a.resident ? sB + k * KB * a.nt * 64u : sB + s * B_STAGE, 512u);
+                    const uint32_t b_box = a.resident ? a.nt * 4u : B_BOX / 16u;  // (in the descriptors' 16-byte units)
+#pragma unroll
+                    for (uint32_t i = 0; i < KB; ++i) {
+                        umma_f16(leader, d, ad + i * (A_BOX / 16u), bd + i * b_box, idesc, (k | i) != 0u ? 1u : 0u);
+                        if (!HALF_K)
+                            umma_f16(leader, d, ad + i * (A_BOX / 16u) + 2u, bd + i * b_box + 2u, idesc, 1u);
+                    }
                 }
-                if (ok) umma_commit(leader, acc_full(acc));
+                umma_commit(leader, empty(s));
             }
-            if (lane == 0) counts[1] = it;
-            umma_commit(leader, mma_done);  // every MMA issued is done (after a wait that gave up too)
+            if (ok) umma_commit(leader, acc_full(acc));
         }
+        if (lane == 0) counts[1] = it;
+        umma_commit(leader, mma_done);  // every MMA issued is done (after a wait that gave up too)
     } else {
         // the epilogue, eight warps, two a tensor-memory lane quarter: warp w reads lanes 32 (w % 4) ... (its rows:
         // pixels of the tile) and half of the tile's columns, (w - 2) / 4 which
@@ -525,12 +521,12 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) k_conv(const __grid_constant_
 // 32-row slots of a 128-row accumulator (M), four a group, and one more slot holds all ones, so that its rows are the
 // bias gradient; N is the layer's output channels (32 to 128). A CTA takes one group of slots (blockIdx.y) over a run
 // of 128-pixel tiles (blockIdx.x):
-//  - one thread loads a tile's stage: per slot a TMA box of 32 channels x bw x bh pixels of x, shifted by the slot's
-//    tap (zeros outside the image), and the output gradient's boxes of 32 channels x the same pixels, unshifted; a
-//    box lands as 128 rows (pixels) of 64 bytes with the 64-byte swizzle, which is the canonical MN-major layout
+//  - a warp loads a tile's stage by one elected lane: per slot a TMA box of 32 channels x bw x bh pixels of x, shifted
+//    by the slot's tap (zeros outside the image), and the output gradient's boxes of 32 channels x the same pixels,
+//    unshifted; a box lands as 128 rows (pixels) of 64 bytes with the 64-byte swizzle, which is the canonical MN-major layout
 //    (32-element blocks of M or N one box = 8 KB apart, 8-pixel groups of K 512 bytes apart);
-//  - one thread issues eight tcgen05.mma (M 128, N, K 16, both operands MN-major, f32 accumulate in tensor memory)
-//    a stage and hands the stage back to the loader through an mbarrier;
+//  - a warp issues, by one elected lane, eight tcgen05.mma (M 128, N, K 16, both operands MN-major, f32 accumulate in
+//    tensor memory) a stage and hands the stage back to the loader through an mbarrier;
 //  - after the run the four epilogue warps read the accumulator (warp w: slot w % 4, its lanes the slot's 32 input
 //    channels) and store it as the CTA's f32 partial; k_wgrad_sum adds the partials of a group's runs, in run order,
 //    into dw (and the ones slot's first row into db), so that the sums do not depend on the CTAs' timing.
@@ -609,49 +605,45 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ CU
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
-        {
-            const uint32_t leader = elect_one();
-            // the loader: a stage a tile
-            uint32_t it = 0;
-            for (uint32_t t = k0; t < k1; ++t, ++it) {
-                const uint32_t s = it % a.ts;
-                if (it >= a.ts && !mbar_wait_warp(empty(s), ((it / a.ts) - 1u) & 1u, a.err, abort_flag)) break;
-                mbar_expect_tx(leader, full(s), (loaded + a.nb) * WG_BOX);
-                const uint32_t b = t / per_img, r = t % per_img;
-                const int x0 = (int)((r % a.tiles_x) * a.bw), y0 = (int)((r / a.tiles_x) * a.bh);
-                const uint32_t base = sbase + s * stage;
-                for (uint32_t j = 0; j < loaded; ++j) {
-                    const uint32_t pr = slot0 + j, tap = pr / a.kc, cb = pr % a.kc;
-                    tma_load_4d(leader, base + j * WG_BOX, &xmap, (int)(a.x_off + cb * 32u), x0 + (int)(tap % 3u) - 1,
-                                y0 + (int)(tap / 3u) - 1, (int)b, full(s));
-                }
-                for (uint32_t i = 0; i < a.nb; ++i)
-                    tma_load_4d(leader, base + (4u + i) * WG_BOX, &dymap, (int)(i * 32u), x0, y0, (int)b, full(s));
+        const uint32_t leader = elect_one();
+        // the loader: a stage a tile
+        uint32_t it = 0;
+        for (uint32_t t = k0; t < k1; ++t, ++it) {
+            const uint32_t s = it % a.ts;
+            if (it >= a.ts && !mbar_wait_warp(empty(s), ((it / a.ts) - 1u) & 1u, a.err, abort_flag)) break;
+            mbar_expect_tx(leader, full(s), (loaded + a.nb) * WG_BOX);
+            const uint32_t b = t / per_img, r = t % per_img;
+            const int x0 = (int)((r % a.tiles_x) * a.bw), y0 = (int)((r / a.tiles_x) * a.bh);
+            const uint32_t base = sbase + s * stage;
+            for (uint32_t j = 0; j < loaded; ++j) {
+                const uint32_t pr = slot0 + j, tap = pr / a.kc, cb = pr % a.kc;
+                tma_load_4d(leader, base + j * WG_BOX, &xmap, (int)(a.x_off + cb * 32u), x0 + (int)(tap % 3u) - 1,
+                            y0 + (int)(tap / 3u) - 1, (int)b, full(s));
             }
-            if (lane == 0) counts[0] = it;
+            for (uint32_t i = 0; i < a.nb; ++i)
+                tma_load_4d(leader, base + (4u + i) * WG_BOX, &dymap, (int)(i * 32u), x0, y0, (int)b, full(s));
         }
+        if (lane == 0) counts[0] = it;
     } else if (warp == 1) {
-        {
-            const uint32_t leader = elect_one();
-            // the MMA issuer: eight K-16 steps a stage into the one accumulator
-            const uint32_t idesc = umma_idesc(128u, n_cols) | (1u << 15) | (1u << 16);  // A and B MN-major
-            uint32_t it = 0;
-            for (uint32_t t = k0; t < k1; ++t, ++it) {
-                const uint32_t s = it % a.ts;
-                if (!mbar_wait_warp(full(s), (it / a.ts) & 1u, a.err, abort_flag)) break;
-                tc_fence_after();
-                const uint32_t base = sbase + s * stage;
+        const uint32_t leader = elect_one();
+        // the MMA issuer: eight K-16 steps a stage into the one accumulator
+        const uint32_t idesc = umma_idesc(128u, n_cols) | (1u << 15) | (1u << 16);  // A and B MN-major
+        uint32_t it = 0;
+        for (uint32_t t = k0; t < k1; ++t, ++it) {
+            const uint32_t s = it % a.ts;
+            if (!mbar_wait_warp(full(s), (it / a.ts) & 1u, a.err, abort_flag)) break;
+            tc_fence_after();
+            const uint32_t base = sbase + s * stage;
 #pragma unroll
-                for (uint32_t j = 0; j < 8u; ++j) {
-                    const uint64_t ad = umma_desc_mn64(base + j * 1024u, WG_BOX);
-                    const uint64_t bd = umma_desc_mn64(base + 4u * WG_BOX + j * 1024u, WG_BOX);
-                    umma_f16(leader, tmem, ad, bd, idesc, (it | j) != 0u ? 1u : 0u);
-                }
-                umma_commit(leader, empty(s));
+            for (uint32_t j = 0; j < 8u; ++j) {
+                const uint64_t ad = umma_desc_mn64(base + j * 1024u, WG_BOX);
+                const uint64_t bd = umma_desc_mn64(base + 4u * WG_BOX + j * 1024u, WG_BOX);
+                umma_f16(leader, tmem, ad, bd, idesc, (it | j) != 0u ? 1u : 0u);
             }
-            if (lane == 0) counts[1] = it;
-            umma_commit(leader, acc_full);  // every MMA issued is done (after a wait that gave up too)
+            umma_commit(leader, empty(s));
         }
+        if (lane == 0) counts[1] = it;
+        umma_commit(leader, acc_full);  // every MMA issued is done (after a wait that gave up too)
     } else {
         // the epilogue: warp w reads tensor-memory lanes 32 (w % 4) ..., the rows of slot w % 4
         const uint32_t quarter = warp & 3u, slot = slot0 + quarter;
@@ -895,10 +887,10 @@ __global__ void k_adam_weights(float* w, const float* __restrict__ g, float* m, 
 
 constexpr int N_FEAT = 11;  // input channels a pixel
 
-// The image's mean luminance and mean first-hit distance (over pixels that hit): sums into acc[0..2].
 // The image's mean luminance and mean first-hit distance (over pixels that hit), in a fixed order so that a denoise
 // is the same bit for bit however it is scheduled: each of FEAT_BLOCKS blocks sums its stride of pixels, and the last
-// block to finish sums the blocks' partials in block order (acc[3] counts the finished blocks, zero between calls).
+// block to finish sums the blocks' partials in block order into acc[0..2] (acc[3] counts the finished blocks, zero
+// between calls).
 constexpr uint32_t FEAT_BLOCKS = 256, FEAT_THREADS = 256;
 __global__ void k_feat_sums(const float4* __restrict__ accum, uint64_t n, float* partial, float* acc) {
     __shared__ float sh[3][FEAT_THREADS];
@@ -1000,7 +992,7 @@ __global__ void k_feat_host(const float* __restrict__ f, uint64_t n, bf16* x) {
 
 // ---- the network ----------------------------------------------------------------------------------------------------
 
-struct Layer { uint32_t cin, cout; int relu; };  // cin: padded to 32 (the input's 10 channels: 32)
+struct Layer { uint32_t cin, cout; int relu; };  // cin: padded to 32 (the input's 11 channels: 32)
 constexpr int N_LAYERS = 15;
 constexpr Layer LAYERS[N_LAYERS] = {
     {32, 32, 1},  {32, 32, 1},  {32, 64, 1},  {64, 64, 1},  {64, 96, 1},  {96, 96, 1},  {96, 128, 1}, {128, 128, 1},
