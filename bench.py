@@ -426,7 +426,7 @@ def run_serve(args, rank, world, local):
     name, sms = gpu.device_info()
     S = [gpu.upload(P) for P in Ps]
     bases = [P.params for P in Ps]
-    # The autotuner: wave size and the material sort, on a short burst of the mix (spp 1 and 16).
+    # The autotuner: wave size and the hit sort, on a short burst of the mix (spp 1 and 16).
     tune_reqs = SV.mix_requests(bases, 24, seed=100 + rank, spps=[1, 16])
     best, trials = SV.autotune(gpu, S, tune_reqs)
     log(f"autotune: {trials} -> {best}")
@@ -745,7 +745,7 @@ def main():
                     help="the reference's binary trees (fastest measured here) or the 8-wide quantised BVH")
     ap.add_argument("--sort", default="hits",
                     help="coherence sorts on the device: 'none', or a comma list of rays, hits, shadows "
-                         "(hits by material is the pass's default; the other two measured slower here)")
+                         "(hits by instance and section is the pass's default; the other two measured slower here)")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline")
     ap.add_argument("--no-extras", action="store_true",
                     help="city: skip the image-quality and serving figures (ΔE against 4096 spp, the learned "

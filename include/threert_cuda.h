@@ -82,7 +82,7 @@ typedef struct { float t; uint32_t tri; float u; float v; uint32_t inst; uint32_
 #define TRT_RENDER_COUNT      2u /* also count node visits, triangle tests and unit entries (a slower walk) */
 #define TRT_RENDER_WIDE       4u /* walk the 8-wide quantised BVH instead of the reference's binary trees */
 /* Coherence sorts on the device, per depth; the image does not depend on them, bit for bit. trt_render sorts hits by
- * instance and section (so by material) before shading when the scene has more than TRT_SORT_HITS_MIN_MATERIALS
+ * instance and section (so mostly by material) before shading when the scene has more than TRT_SORT_HITS_MIN_MATERIALS
  * materials (measured: the city's 4,201 and the crowd's 217 gain 3-10 %, the Cornell box's 4 loses 14 %) and the wave
  * at least TRT_SORT_HITS_MIN_PATHS paths, unless this flag is given; a server sorts the hits of every step of that size
  * unless its options' flags hold it: */

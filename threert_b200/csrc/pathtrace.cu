@@ -779,11 +779,13 @@ __global__ void __launch_bounds__(PATHS_BLOCK, TRT_BLOCKS_PATHS) k_paths(const J
 // it, since a path's state, hit and random numbers belong to the path, not to its queue position.
 //   SORT_RAYS: the extend queue by (queue chunk, direction octant): a warp's rays start near one another (the chunk)
 //     and point the same way, so they walk the same nodes in the same order.
-//   SORT_HITS (on unless TRT_RENDER_UNSORTED_HITS, in waves of TRT_SORT_HITS_MIN_PATHS): the shade queue by instance
-//     and section, misses first: a warp then reads one material record and takes one set of branches, and the next
-//     depth's queue, appended in this order, starts its rays from one mesh. The key is made of the hit record alone:
-//     the material row it stands for lay behind three dependent loads (the job, the instance, its row), which bounded
-//     the count (latency; 720p city frame 36 us a launch of 460,800 items under ncu). The frame 4.36 -> 4.32 ms.
+//   SORT_HITS (on unless TRT_RENDER_UNSORTED_HITS, in waves of TRT_SORT_HITS_MIN_PATHS): the shade queue by (instance
+//     number + section) modulo the bins, misses first: a warp then mostly reads one material record and takes one set of
+//     branches, and the next depth's queue, appended in this order, mostly starts its rays from one mesh. It stands for
+//     the material without being it: a unit's section shares a bin with the next unit's section before, with numbers
+//     4,095 on and, in a server's step, with other scenes' units. The key is made of the hit record alone: the material
+//     row lay behind three dependent loads (the job, the instance, its row), which bounded the count (latency; 720p city
+//     frame 36 us a launch of 460,800 items under ncu). The frame 4.36 -> 4.32 ms.
 //   SORT_SHADOWS: the shadow rays by (position chunk, direction octant) in each light class.
 // Blocks of 1,024 threads with two items each: the keys' loads and the atomics behind them are latency, which more
 // warps hide, while a block's clearing of the bins and its atomic a key it meets want many items a block. The 720p city
@@ -1257,11 +1259,11 @@ void launch_sort(trt_scene* s, Wave& W, const uint32_t* in, uint32_t* out, uint3
     s->launches += 2;
 }
 
-// A wave's launches on a stream pair (st, aux): ray generation, then each depth's walks, sorts, shading and resolve,
-// then the accumulation.
 // What the walks run from as streams of rays (the reasons and figures: launch_wave).
 constexpr uint32_t STREAM_MIN_UNITS = 256u, STREAM_MIN_SHADOW = 131072u, STREAM_MIN_EXTEND = 262144u;
 struct WalkGrids { int extend, shadow, extend_stream, shadow_stream; };  // (the persistent walks')
+// A wave's launches on a stream pair (st, aux): ray generation, then each depth's walks, sorts, shading and resolve,
+// then the accumulation.
 template <bool COUNT, bool WIDE>
 void launch_wave(trt_scene* s, Wave& W, const Job& job, uint32_t n, uint32_t last, uint32_t flags_eff,
                  cudaStream_t st, cudaStream_t aux, cudaEvent_t fork_ev, cudaEvent_t join_ev, const WalkGrids& grids) {
