@@ -10,6 +10,8 @@ CASE`): each case prepares its input, runs the kernels of interest a few times a
            scene (the sky kernels, the environment's texels and CDF)
   emitters the city's emitters re-weighed three times (the emitter-weight kernels)
   cornell  three frames of the Cornell box, 256 x 256, 16 spp
+  small    three small waves of each kind: the Cornell box at 64 x 64, 1 spp, and a city of 302 units at 128 x 128, 4 spp
+           (k_paths, k_accumulate)
 """
 from __future__ import annotations
 
@@ -33,12 +35,15 @@ def city(flags: int = 0):
 
 def unet_case():
     from threert_b200 import unet
-    net = unet.UNet(0, max_batch=16, max_h=720, max_w=1280)
+    net = unet.UNet(0, max_batch=1, max_h=720, max_w=1280)
     net.set_params(unet.init_params(0))
     rng = np.random.default_rng(0)
     f = rng.normal(0, 1, (1, 720, 1280, unet.N_FEAT)).astype(np.float32)
     for _ in range(3):
         net.forward(f)
+    net.close()
+    net = unet.UNet(0, max_batch=16, max_h=64, max_w=64)
+    net.set_params(unet.init_params(0))
     fb = rng.normal(0, 1, (16, 64, 64, unet.N_FEAT)).astype(np.float32)
     tb = rng.normal(0, 1, (16, 64, 64, 3)).astype(np.float32)
     net.step(fb, tb)
@@ -104,6 +109,20 @@ def cornell_case():
     g.close()
 
 
+def small_case():
+    from threert_b200 import Gpu, prep, scenes
+    town = scenes.city(n_objects=300, width=128, height=128, seed=5, extent=100.0, n_emitters=60, box_segments=2,
+                       sphere_slices=12, sphere_stacks=10, sky_size=(256, 128))
+    g = Gpu(0)
+    for P, spp in ((prep.prepare(scenes.cornell(64, 64)), 1), (prep.prepare(town), 4)):
+        S = g.upload(P)
+        for k in range(3):
+            S.render_raw(prep.params_with(P.params, seed=k + 1), spp, read=False, stats=False)
+        g.synchronize()
+        S.close()
+    g.close()
+
+
 if __name__ == "__main__":
     case = sys.argv[1] if len(sys.argv) > 1 else "city"
     if case == "city":
@@ -121,5 +140,7 @@ if __name__ == "__main__":
         emitters_case()
     elif case == "cornell":
         cornell_case()
+    elif case == "small":
+        small_case()
     else:
         raise SystemExit(f"unknown case {case}")
